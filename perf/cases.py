@@ -166,11 +166,9 @@ FRICT = dict(density=3000.0, young=1e7, ktDivKn=0.2, tanPhi=0.5, surfEnergy=0.0)
 HERTZ = [dict(density=1000.0, young=5e7, ktDivKn=0.2, tanPhi=t, surfEnergy=0.01) for t in (0.3, 0.6)]
 
 
-def _random_quaternions(g, n):
-    u = _uniform(g, (n, 3), 0, 1)
-    a, b, t = (1 - u[:, 0]).sqrt(), u[:, 0].sqrt(), 2 * math.pi
-    return torch.stack([b * torch.cos(t * u[:, 2]), a * torch.sin(t * u[:, 1]), a * torch.cos(t * u[:, 1]),
-                        b * torch.sin(t * u[:, 2])], dim=1)
+def _axes():
+    """Semi-axes of the ellipsoids over the largest one."""
+    return torch.tensor([1.0, 0.7, 0.5], device=LOCAL, dtype=torch.float64)
 
 
 def _scene(case, seed):
@@ -223,14 +221,15 @@ def _scene(case, seed):
             mats = [dict(m, young=1e8, density=1000.0) for m in mats]
         elif kind == "ell":
             r = _uniform(g, (n,), 3e-3, 6e-3)
-            phi, rounds = 0.50, 100
+            phi, rounds = 0.52, 100
             mats = [dict(FRICT, density=1000.0, young=1e7, tanPhi=0.4)]
         else:
             r = torch.full((n,), 5e-3, device=LOCAL, dtype=torch.float64) if law == "frict" else _uniform(g, (n,), 2e-3, 6e-3)
             phi, rounds = (0.3, 40) if kind == "cloud" else (0.52, 100)
-        thick = 0.95 if kind == "ell" else 1.0
-        pos, r, box = _packing(g, thick * r, phi, kind == "peri", rounds)
-        r = r / thick
+        pos, r, box = _packing(g, r, phi, kind == "peri", rounds)
+        if kind == "ell":
+            # parallel ellipsoids: the packing of spheres stretched along the axes
+            pos, box = pos * _axes(), box * _axes()
         if kind == "cloud":
             pos[:, 2] += 0.5 * float(box[2])  # above the floor of a box half as high again
             box[2] *= 1.5
@@ -252,12 +251,13 @@ def _scene(case, seed):
     k = len(r)
     rho = torch.tensor([m["density"] for m in mats], device=LOCAL, dtype=torch.float64)[mat]
     if kind == "ell":
-        semi = r[:, None] * torch.tensor([1.0, 0.7, 0.5], device=LOCAL, dtype=torch.float64)
+        semi = r[:, None] * _axes()
         mass = (4.0 / 3.0 * math.pi) * semi.prod(1) * rho
         q = semi.square()
         inertia = mass[:, None] / 5.0 * (q.sum(1, keepdim=True) - q)
         S["semi"] = semi.cpu().numpy()
-        ori = _random_quaternions(g, k)
+        tilt = torch.randn((k, 3), generator=g, device=LOCAL, dtype=torch.float64) * 0.01  # about a degree
+        ori = _unit(torch.cat([torch.ones(k, 1, device=LOCAL, dtype=torch.float64), tilt], dim=1))
     else:
         mass = (4.0 / 3.0 * math.pi) * r ** 3 * rho
         inertia = (0.4 * mass * r * r)[:, None].expand(k, 3)
@@ -376,7 +376,7 @@ def work(case):
     bodies = n if case["kind"] != "batch" else 5286.0 * n  # the mean of 500 .. 20000 over the logarithm
     # per step and body: position, velocity, spin and orientation read and written; per contact: the two bodies'
     # gathered state is theirs already, its own history (frame, contact point, force, stiffnesses) read and written
-    per_body = {"cloud": 0.02, "bed": 2.4, "peri": 2.8, "batch": 2.2, "ell": 0.8, "hopper": 2.4}[case["kind"]]
+    per_body = {"cloud": 0.02, "bed": 2.4, "peri": 2.8, "batch": 2.2, "ell": 2.0, "hopper": 2.4}[case["kind"]]
     flops = 1200.0 if case["kind"] == "ell" else 400.0
     return {"bytes": steps * bodies * (208.0 + 224.0 * per_body) + 104.0 * bodies * (2 if case["kind"] == "cloud" else 1),
             "flops": steps * bodies * (40.0 + flops * per_body)}
