@@ -76,6 +76,36 @@ __device__ __forceinline__ void cp2(const StepParams& P, int matA, int matB, dou
   }
 }
 
+// a * 0.5 where the product stands alone: on the integer pipe in the exact variant; the contracted one takes it
+// into the FMA of the sum that follows
+#ifdef WDEM_FMA
+#define HALF(x) (0.5 * (x))
+#else
+#define HALF(x) halfOf(x)
+#endif
+
+// HertzPhys.alpha = mean of the materials' alpha (Hertz.cpp:52) is 0: the noAttraction clamp applies.  When no
+// material of the table has an alpha (StepParams.alphaZero) nothing is read.
+__device__ __forceinline__ bool hertzAlphaZero(const StepParams& P, const Particles& p, int a, int b) {
+  if (P.alphaZero) return true;
+  WDEM_REAL_BRANCH();
+  const double alphaC = .5 * (c_mats[p.meta[a].y].alpha + c_mats[p.meta[b].y].alpha);
+  return zeroBits(alphaC);
+}
+
+// m times an integer vector of periods, rows summed left to right as mvec does: periods of 0 and +-1 make each
+// product a signed zero or a signed copy, formed on the integer pipe, and a sum with a zero is a copy (addZ)
+__device__ __forceinline__ double mulPeriod(double a, int c) {
+  if (finiteBits(a) && c >= -1 && c <= 1) return c == 0 ? signedZero(a, 0.0) : (c > 0 ? a : flipSign(a));
+  WDEM_REAL_BRANCH();
+  return a * (double)c;
+}
+__device__ __forceinline__ d3 cellShift(const double* m, const int4& cd) {
+  return mk(addZ(addZ(mulPeriod(m[0], cd.x), mulPeriod(m[1], cd.y)), mulPeriod(m[2], cd.z)),
+            addZ(addZ(mulPeriod(m[3], cd.x), mulPeriod(m[4], cd.y)), mulPeriod(m[5], cd.z)),
+            addZ(addZ(mulPeriod(m[6], cd.x), mulPeriod(m[7], cd.y)), mulPeriod(m[8], cd.z)));
+}
+
 // warp-aggregated add of per-thread counters (one atomic per warp)
 __device__ __forceinline__ void warpAdd(unsigned long long* dst, unsigned v) {
   const unsigned mask = __activemask();
@@ -558,7 +588,7 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
   const double4_32a A4 = p.posr[a], B4 = p.posr[b];
   d3 pos1 = xyz(A4);
   d3 shift2 = mk(0, 0, 0);
-  if (PERI) shift2 = mvec(P.hS, mk((double)cd.x, (double)cd.y, (double)cd.z));
+  if (PERI) shift2 = cellShift(P.hS, cd);
   const d3 pos2 = PERI ? xyz(B4) + shift2 : xyz(B4);
   double r1, r2, uN;
   d3 normal, contPt;
@@ -579,14 +609,15 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
     // Cg2_Sphere_Sphere_L6Geom::go
     r1 = A4.w; r2 = B4.w;
     d3 relPos = pos2 - pos1;
-    double t = fabs(P.distFactor) * (r1 + r2);
     const double relSq = sqnormExact(relPos);
-    double unDistSq = __dsub_rn(relSq, __dmul_rn(t, t));
-    if (positiveBits(unDistSq) && !real) return;
+    if (!real) {
+      const double t = fabs(P.distFactor) * (r1 + r2);
+      if (positiveBits(__dsub_rn(relSq, __dmul_rn(t, t)))) return;
+    }
     double dist = sqrt(relSq);
     uN = dist - (r1 + r2);
     normal = relPos / dist;
-    contPt = pos1 + (r1 + 0.5 * uN) * normal;
+    contPt = pos1 + (r1 + HALF(uN)) * normal;
   } else {
     // Cg2_Wall_Sphere_L6Geom::go (pA is the wall)
     const int wa = p.meta[a].x;
@@ -647,14 +678,14 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
     const int am = P.approxMask;
     const d3 currNormal = normal;
     d3 normRotVec = cross(prevNormal, currNormal);
-    d3 midNormal = (am & 1) ? prevNormal : 0.5 * (prevNormal + currNormal);
+    d3 midNormal = (am & 1) ? prevNormal : halfOf(prevNormal + currNormal);
     if (zeroBits(sqnorm(midNormal))) midNormal = currNormal;
     else if (!(am & 2) && !(am & 1)) midNormal = normalized(midNormal);
-    d3 normTwistVec = midNormal * dt * 0.5 * dot(midNormal, angVel1 + angVel2);
+    d3 normTwistVec = halfOf(midNormal * dt) * dot(midNormal, angVel1 + angVel2);
     d3 rt = normRotVec + normTwistVec;
     d3 mid0, mid1;
     if (am & 4) { mid0 = prevNormal; mid1 = prevT1; }
-    else { mid0 = midNormal; mid1 = prevT1 - cross(prevT1, rt) * 0.5; }
+    else { mid0 = midNormal; mid1 = prevT1 - HALF(cross(prevT1, rt)); }
     d3 mid2 = cross(mid0, mid1);
     cur0 = currNormal;
     cur1 = prevT1 - cross(mid1, rt);
@@ -666,12 +697,13 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
     d3 midContPt, midPos1, midPos2;
     // periodic: velocity of the pB image, Cell::intrShiftVel = gradV * pprevHsize * cellDist
     d3 shiftVel2 = mk(0, 0, 0);
-    if (PERI) shiftVel2 = mvec(P.shv, mk((double)cd.x, (double)cd.y, (double)cd.z));
+    if (PERI) shiftVel2 = cellShift(P.shv, cd);
     if (am & 8) { midContPt = contPt; midPos1 = pos1; midPos2 = pos2; }
     else {
-      midContPt = 0.5 * (prevContPt + contPt);
-      midPos1 = pos1 - (dt * 0.5) * vel1;
-      midPos2 = PERI ? pos2 - (dt * 0.5) * (vel2 + shiftVel2) : pos2 - (dt * 0.5) * vel2;
+      midContPt = HALF(prevContPt + contPt);
+      const double hdt = halfOf(dt);
+      midPos1 = pos1 - hdt * vel1;
+      midPos2 = PERI ? pos2 - hdt * (vel2 + shiftVel2) : pos2 - hdt * vel2;
     }
     d3 c1x = (P.noRatch && positiveBits(r1)) ? r1 * midNormal : midContPt - midPos1;
     d3 c2x = (P.noRatch && positiveBits(r2)) ? (-r2) * midNormal : midContPt - midPos2;
@@ -759,35 +791,21 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
   } else {
     const double velN = gvel.x;
     const double kn0 = hz[0];
-#ifdef WDEM_FMA
-    // one square root of the overlap for kn, Fne and kt, and its square root for the viscous coefficient
-    const double sq = sqrt(dmax(-uN, 0.));
-    kn = (3 / 2.) * kn0 * sq;
-#else
-    kn = (3 / 2.) * kn0 * sqrt(-uN);
-#endif
     if (positiveBits(uN)) keep = false;
     else {
-#ifdef WDEM_FMA
+      // one square root of the overlap for kn, Fne and kt, and its square root for the viscous coefficient (the
+      // reference's sqrt(-uN), sqrt(max(-uN, 0)) and sqrt(uN < 0 ? -uN : 0) are the same number for uN < 0, and
+      // differ for uN = 0 only in the last one's +0)
+      const double sq = sqrt(-uN);
+      kn = (3 / 2.) * kn0 * sq;
       double Fne = -kn0 * pown3(sq);
       double Fna = hz[3];
       double eta = (positiveBits(hz[2]) ? hz[2] * sqrt(sq) : 0.);
-#else
-      double Fne = -kn0 * pown3(sqrt(-uN));
-      double Fna = hz[3];
-      double eta = (positiveBits(hz[2]) ? hz[2] * sqrt(sqrt(dmax(-uN, 0.))) : 0.);
-#endif
       double Fnv = eta * velN;
-      // HertzPhys.alpha = mean of the materials' alpha (Hertz.cpp:52); the clamp applies when it is 0
-      const double alphaC = .5 * (c_mats[p.meta[a].y].alpha + c_mats[p.meta[b].y].alpha);
-      if (zeroBits(alphaC) && P.noAttraction && positiveBits(Fne + Fnv)) Fnv = -Fne;
+      if (P.noAttraction && hertzAlphaZero(P, p, a, b) && positiveBits(Fne + Fnv)) Fnv = -Fne;
       fx = Fne + Fna + Fnv;
       if (P.trackEnergy) eVN = Fnv * velN * dt;
-#ifdef WDEM_FMA
-      kt = hz[1] * sq;
-#else
-      kt = hz[1] * sqrt(negativeBits(uN) ? -uN : 0);
-#endif
+      kt = hz[1] * (negativeBits(uN) ? sq : 0.);
       double sc = dt * kt;
       fy = fy + sc * gvel.y;
       fz = fz + sc * gvel.z;
@@ -840,12 +858,18 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
   const qd ori = quatFromCols(cur0, cur1, cur2);
   const d3 F = qrot(ori, mk(fx, fy, fz));
   const d3 tq = mk(tqx, tqy, tqz);
-  const d3 T = isZeroBits(tq) ? mk(0, 0, 0) : qrot(ori, tq);
   const d3 xcA = contPt - pos1;
   const d3 xcB = contPt - pos2;
-  const d3 TA = cross(xcA, F) + T;
-  const d3 FB = F * -1.0;
-  const d3 TB = cross(xcB, FB) + T * -1.0;
+  const d3 FB = flipSign(F);
+  d3 TA = cross(xcA, F), TB = cross(xcB, FB);
+  if (isZeroBits(tq)) {
+    TA = plusZero(TA);  // + T = +0; to TB, -T = -0 adds nothing
+  } else {
+    WDEM_REAL_BRANCH();
+    const d3 T = qrot(ori, tq);
+    TA = TA + T;
+    TB = TB - T;
+  }
   // each particle's share at its CSR entry, stamped with this pass; a facet (pA) takes none
   // (ContactLoop::applyForceUninodal skips shapes with more than one node, ContactLoop.cpp:270-276)
   const int2 sl = c.slot[i];
@@ -897,36 +921,26 @@ struct dwq {
   dwf w, x, y, z;
 };
 // Quaternion(Matrix3) of the frame with columns c0, c1, c2 (the branches of quatFromCols)
+__device__ __forceinline__ dwf dwPick(bool c, dwf a, dwf b) { return {c ? a.h : b.h, c ? a.l : b.l}; }
 __device__ __forceinline__ dwq dwQuatFromCols(dw3 c0, dw3 c1, dw3 c2) {
   const dwf m00 = c0.x, m10 = c0.y, m20 = c0.z, m01 = c1.x, m11 = c1.y, m21 = c1.z, m02 = c2.x, m12 = c2.y, m22 = c2.z;
-  dwq q;
   const dwf tr = dwAdd(dwAdd(m00, m11), m22);
-  if (dwPos(tr)) {
-    dwf t = dwSqrt(dwAddF(tr, 1.f));
-    q.w = dwScale(t, 0.5f);
-    t = dwScale(dwRecip(t), 0.5f);
-    q.x = dwMul(dwSub(m21, m12), t);
-    q.y = dwMul(dwSub(m02, m20), t);
-    q.z = dwMul(dwSub(m10, m01), t);
-  } else {
-    int i = 0;
-    if (dwGt(m11, m00)) i = 1;
-    if (dwGt(m22, i == 0 ? m00 : m11)) i = 2;
-    if (i == 0) {
-      dwf t = dwSqrt(dwAddF(dwSub(dwSub(m00, m11), m22), 1.f));
-      q.x = dwScale(t, 0.5f); t = dwScale(dwRecip(t), 0.5f);
-      q.w = dwMul(dwSub(m21, m12), t); q.y = dwMul(dwAdd(m10, m01), t); q.z = dwMul(dwAdd(m20, m02), t);
-    } else if (i == 1) {
-      dwf t = dwSqrt(dwAddF(dwSub(dwSub(m11, m22), m00), 1.f));
-      q.y = dwScale(t, 0.5f); t = dwScale(dwRecip(t), 0.5f);
-      q.w = dwMul(dwSub(m02, m20), t); q.z = dwMul(dwAdd(m21, m12), t); q.x = dwMul(dwAdd(m01, m10), t);
-    } else {
-      dwf t = dwSqrt(dwAddF(dwSub(dwSub(m22, m00), m11), 1.f));
-      q.z = dwScale(t, 0.5f); t = dwScale(dwRecip(t), 0.5f);
-      q.w = dwMul(dwSub(m10, m01), t); q.x = dwMul(dwAdd(m02, m20), t); q.y = dwMul(dwAdd(m12, m21), t);
-    }
-  }
-  return q;
+  const bool pos = dwPos(tr);
+  const bool b1 = dwGt(m11, m00);
+  const bool i2 = dwGt(m22, dwPick(b1, m11, m00));
+  const bool i1 = b1 && !i2, i0 = !b1 && !i2;
+  const dwf mi = dwPick(i0, m00, dwPick(i1, m11, m22)), mj = dwPick(i0, m11, dwPick(i1, m22, m00)),
+            mk_ = dwPick(i0, m22, dwPick(i1, m00, m11));
+  const dwf u = dwPick(pos, tr, dwSub(dwSub(mi, mj), mk_));
+  dwf t = dwSqrt(dwAddF(u, 1.f));
+  const dwf d = dwScale(t, 0.5f);
+  t = dwScale(dwRecip(t), 0.5f);
+  const bool p0 = pos || i0, p2 = pos || i2;
+  const dwf e1 = dwMul(dwSub(dwPick(p0, m21, dwPick(i1, m02, m10)), dwPick(p0, m12, dwPick(i1, m20, m01))), t);
+  const dwf e2 = dwMul(dwAdd(dwPick(p2, m02, m10), dwPick(p2, dwPick(pos, dwNeg(m20), m20), m01)), t);
+  const dwf e3 = dwMul(dwAdd(dwPick(pos, m10, dwPick(i0, m20, m21)), dwPick(pos, dwNeg(m01), dwPick(i0, m02, m12))), t);
+  return {dwPick(pos, d, e1), dwPick(pos, e1, dwPick(i0, d, e2)), dwPick(pos, e2, dwPick(i1, d, dwPick(i0, e2, e3))),
+          dwPick(pos || !i2, e3, d)};
 }
 // v rotated by q: uv = q.vec x v, uv += uv, v + w uv + q.vec x uv (as qrot)
 __device__ __forceinline__ dw3 dwQrot(dwq q, dw3 v) {
@@ -949,7 +963,7 @@ __device__ __forceinline__ void contactBodyDW(const StepParams& P, const Particl
   const double4_32a A4 = p.posr[a], B4 = p.posr[b];
   const d3 pos1 = xyz(A4);
   d3 shift2 = mk(0, 0, 0);
-  if (PERI) shift2 = mvec(P.hS, mk((double)cd.x, (double)cd.y, (double)cd.z));
+  if (PERI) shift2 = cellShift(P.hS, cd);
   const d3 pos2 = PERI ? xyz(B4) + shift2 : xyz(B4);
   double r1, r2, uN;
   dw3 normal, d1, d2;  // d1, d2: the contact point's offsets from pA's and pB's node (the branch vectors)
@@ -1012,7 +1026,7 @@ __device__ __forceinline__ void contactBodyDW(const StepParams& P, const Particl
   // branch vectors midContPt - midPos = (contPt - pos) + (prevContPt - contPt) / 2 + dt/2 vel: the offsets
   // d1, d2 and the FP64 difference of the two contact points, which are close together
   d3 shiftVel2 = mk(0, 0, 0);
-  if (PERI) shiftVel2 = mvec(P.shv, mk((double)cd.x, (double)cd.y, (double)cd.z));
+  if (PERI) shiftVel2 = cellShift(P.shv, cd);
   const d3 vel1d = xyz(V1), vel2d = PERI ? xyz(V2) + shiftVel2 : xyz(V2);
   const dw3 halfPrev = dw3Scale(dw3Of(prevContPt - contPt), 0.5f);
   const dw3 c1x = (P.noRatch && positiveBits(r1)) ? dw3Mul(midNormal, dwFrom(r1))
@@ -1060,8 +1074,7 @@ __device__ __forceinline__ void contactBodyDW(const StepParams& P, const Particl
       const double hz2 = c.hist[HIST_E2][i];
       const double etaD = positiveBits(hz2) ? hz2 * sqrt(sq) : 0.;
       double Fnv = etaD * velN;
-      const double alphaC = .5 * (c_mats[p.meta[a].y].alpha + c_mats[p.meta[b].y].alpha);
-      if (zeroBits(alphaC) && P.noAttraction && positiveBits(Fne + Fnv)) Fnv = -Fne;
+      if (P.noAttraction && hertzAlphaZero(P, p, a, b) && positiveBits(Fne + Fnv)) Fnv = -Fne;
       fx = dwFrom(Fne + Fna + Fnv);
       const dwf eta = dwFrom(etaD);
       ktD = c.hist[HIST_E1][i] * sq;

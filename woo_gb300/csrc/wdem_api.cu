@@ -564,6 +564,9 @@ void fillStepParams(wdem_handle* h) {
   P.trackEnergy = r.trackEnergy;
   P.lfEnergy = r.trackEnergy;
   P.nMaterials = (int)h->mats.size();
+  P.alphaZero = 1;
+  for (const wdem_material& m : h->mats)
+    if (m.alpha != 0.) P.alphaZero = 0;
   P.periodic = h->periodic ? 1 : 0;
   P.matDt = h->useMatDt ? h->dMatDt : nullptr;
   P.hasEll = h->hasEll ? 1 : 0;

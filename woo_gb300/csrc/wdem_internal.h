@@ -132,6 +132,7 @@ struct StepParams {
   int trackEnergy;
   int lfEnergy;       // Leapfrog's reallyTrackEnergy: trackEnergy, off in step 0 of a cell with gradV != I
   int nMaterials;
+  int alphaZero;      // every material's alpha is 0
   // periodic cell (Cell, homoDeform GRADV2), row-major 3x3
   int periodic;
   int hasShear;

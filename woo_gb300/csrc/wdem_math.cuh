@@ -144,48 +144,78 @@ __device__ __forceinline__ d3 mvec(const double* m, d3 v) {
 
 struct qd { double w, x, y, z; };
 
+// x * 0.5 and x + x on the integer pipe (the exponent moved by one: exact while the result is normal);
+// subnormal results, overflows, infinities and NaN take the FP64 operation.  An FP64 instruction holds the
+// pipe for 16 cycles a warp on GB300, these few integer ones for about 2.
+__device__ __forceinline__ double halfOf(double x) {
+  const Halves h = halvesOf(x);
+  const unsigned e = h.hi & 0x7ff00000u;
+  if (e >= 0x00200000u && e != 0x7ff00000u) return fromHalves(h.lo, h.hi - 0x00100000u);
+  if (((h.hi << 1) | h.lo) == 0) return x;
+  WDEM_REAL_BRANCH();
+  return 0.5 * x;
+}
+__device__ __forceinline__ double twice(double x) {
+  const Halves h = halvesOf(x);
+  const unsigned e = h.hi & 0x7ff00000u;
+  if (e >= 0x00100000u && e < 0x7fe00000u) return fromHalves(h.lo, h.hi + 0x00100000u);
+  if (((h.hi << 1) | h.lo) == 0) return x;
+  WDEM_REAL_BRANCH();
+  return x + x;
+}
+__device__ __forceinline__ d3 halfOf(d3 a) { return mk(halfOf(a.x), halfOf(a.y), halfOf(a.z)); }
+__device__ __forceinline__ d3 twice(d3 a) { return mk(twice(a.x), twice(a.y), twice(a.z)); }
+// -x: the sign bit (x * -1.0 but for a NaN's sign)
+__device__ __forceinline__ double flipSign(double x) { const Halves h = halvesOf(x); return fromHalves(h.lo, h.hi ^ 0x80000000u); }
+__device__ __forceinline__ d3 flipSign(d3 a) { return mk(flipSign(a.x), flipSign(a.y), flipSign(a.z)); }
+// x + 0.0: x, except that -0 becomes +0
+__device__ __forceinline__ double plusZero(double x) { return negZero(x) ? 0.0 : x; }
+__device__ __forceinline__ d3 plusZero(d3 a) { return mk(plusZero(a.x), plusZero(a.y), plusZero(a.z)); }
+// c ? a : b without an FP64 instruction
+__device__ __forceinline__ double pick(bool c, double a, double b) {
+  const Halves x = halvesOf(a), y = halvesOf(b);
+  return fromHalves(c ? x.lo : y.lo, c ? x.hi : y.hi);
+}
+
 // Rotation matrix given by columns c0, c1, c2 -> unit quaternion (Shoemake: trace branch, else the
 // largest diagonal element).  m(r,k) = column k, row r.
+// The four cases differ only in which entries are added or subtracted: the operands and signs are selected
+// on the integer pipe and one square root, one division and three sums run for all lanes.  Contact frames
+// point anywhere, so the lanes of a warp fall into all four cases and separate branches would issue the
+// square root and the division up to four times.  Same IEEE operations per case (a - b is a + (-b)).
 __device__ __forceinline__ qd quatFromCols(d3 c0, d3 c1, d3 c2) {
   const double m00 = c0.x, m10 = c0.y, m20 = c0.z;
   const double m01 = c1.x, m11 = c1.y, m21 = c1.z;
   const double m02 = c2.x, m12 = c2.y, m22 = c2.z;
+  const double tr = m00 + m11 + m22;
+  const bool pos = tr > 0;
+  // largest diagonal element i, j = i+1, k = j+1 (mod 3)
+  const bool b1 = m11 > m00;
+  const bool i2 = m22 > pick(b1, m11, m00);
+  const bool i1 = b1 && !i2, i0 = !b1 && !i2;
+  const double mi = pick(i0, m00, pick(i1, m11, m22)), mj = pick(i0, m11, pick(i1, m22, m00)),
+               mk_ = pick(i0, m22, pick(i1, m00, m11));
+  const double u = pick(pos, tr, mi - mj - mk_);
+  double t = sqrt(u + 1.0);
+  const double d = halfOf(t);
+  t = 0.5 / t;
+  const bool p0 = pos || i0;
+  const double e1 = (pick(p0, m21, pick(i1, m02, m10)) - pick(p0, m12, pick(i1, m20, m01))) * t;
+  const bool p2 = pos || i2;
+  const double e2 = (pick(p2, m02, m10) + pick(p2, pick(pos, flipSign(m20), m20), m01)) * t;
+  const double e3 = (pick(pos, m10, pick(i0, m20, m21)) + pick(pos, flipSign(m01), pick(i0, m02, m12))) * t;
   qd q;
-  double t = m00 + m11 + m22;
-  if (t > 0) {
-    t = sqrt(t + 1.0);
-    q.w = 0.5 * t;
-    t = 0.5 / t;
-    q.x = (m21 - m12) * t;
-    q.y = (m02 - m20) * t;
-    q.z = (m10 - m01) * t;
-  } else {
-    // largest diagonal element i, j = i+1, k = j+1 (mod 3), written out per case
-    int i = 0;
-    if (m11 > m00) i = 1;
-    if (m22 > (i == 0 ? m00 : m11)) i = 2;
-    if (i == 0) {         // j=1, k=2
-      t = sqrt(m00 - m11 - m22 + 1.0);
-      q.x = 0.5 * t; t = 0.5 / t;
-      q.w = (m21 - m12) * t; q.y = (m10 + m01) * t; q.z = (m20 + m02) * t;
-    } else if (i == 1) {  // j=2, k=0
-      t = sqrt(m11 - m22 - m00 + 1.0);
-      q.y = 0.5 * t; t = 0.5 / t;
-      q.w = (m02 - m20) * t; q.z = (m21 + m12) * t; q.x = (m01 + m10) * t;
-    } else {              // j=0, k=1
-      t = sqrt(m22 - m00 - m11 + 1.0);
-      q.z = 0.5 * t; t = 0.5 / t;
-      q.w = (m10 - m01) * t; q.x = (m02 + m20) * t; q.y = (m12 + m21) * t;
-    }
-  }
+  q.w = pick(pos, d, e1);
+  q.x = pick(pos, e1, pick(i0, d, e2));
+  q.y = pick(pos, e2, pick(i1, d, pick(i0, e2, e3)));
+  q.z = pick(pos || !i2, e3, d);
   return q;
 }
 
 // v rotated by unit quaternion q: uv = q.vec x v; uv += uv; v + w uv + q.vec x uv
 __device__ __forceinline__ d3 qrot(qd q, d3 v) {
   d3 qv = mk(q.x, q.y, q.z);
-  d3 uv = cross(qv, v);
-  uv = uv + uv;
+  const d3 uv = twice(cross(qv, v));
   return v + q.w * uv + cross(qv, uv);
 }
 
