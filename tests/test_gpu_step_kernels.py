@@ -43,3 +43,18 @@ def test_hertz_materials_with_alpha(wdem_lib):
     spec.materials[1].alpha = 0.4
     h, _ = _run_both(spec, (1, 60))
     assert h.status().nReal > 50
+
+
+@pytest.mark.parametrize("m", [63, 64, 65, 96, 97, 200])
+def test_wall_force_over_long_rows(wdem_lib, m):
+    """The force on a wall from m spheres touching it, and as many hovering above: rows at and beyond the length
+    where a warp takes them from the single thread, with stamped and unstamped records mixed."""
+    r = 0.005
+    k = np.arange(2 * m)
+    side = int(np.ceil(np.sqrt(2 * m)))
+    centers = np.stack([0.02 + 2.2 * r * (k % side), 0.02 + 2.2 * r * (k // side), np.where(k % 2, 1.02 * r, 0.98 * r)], axis=1)
+    mats = [dict(kind=abi.MAT_FRICT, density=2500.0, young=1e7, ktDivKn=0.2, tanPhi=0.5)]
+    pa = scenes.assemble(centers, np.full(2 * m, r), 0, [(2, 1, 0.0, 0)], mats, vel=np.random.default_rng(m).normal(0, 0.2, (2 * m, 3)))
+    spec = scenes.SceneSpec(scenes.default_params(scenes.materials_array(mats), dt=1e-5, gravity=(0, 0, -9.81)), None, pa)
+    h, _ = _run_both(spec, (1, 3))
+    assert h.status().nReal >= m

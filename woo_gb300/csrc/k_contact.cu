@@ -877,11 +877,11 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
   if (PERI || !(sb & CS_FACET)) {
     double4_32a* oa = c.out + OUT_RECORDS * (long long)sl.x;
     oa[OUT_F] = make_double4_32a(F.x, F.y, F.z, stamp);
-    oa[OUT_T] = make_double4_32a(TA.x, TA.y, TA.z, 0.0);
+    oa[OUT_T] = make_double4_32a(TA.x, TA.y, TA.z, stamp);
   }
   double4_32a* ob = c.out + OUT_RECORDS * (long long)sl.y;
   ob[OUT_F] = make_double4_32a(FB.x, FB.y, FB.z, stamp);
-  ob[OUT_T] = make_double4_32a(TB.x, TB.y, TB.z, 0.0);
+  ob[OUT_T] = make_double4_32a(TB.x, TB.y, TB.z, stamp);
   // the row positions this pass stamped, for the integrator's gather
   if (p.rowMask) {
     const uchar2 rb = c.rowBit[i];
@@ -1120,11 +1120,11 @@ __device__ __forceinline__ void contactBodyDW(const StepParams& P, const Particl
   if (PERI || !(sb & CS_FACET)) {
     double4_32a* oa = c.out + OUT_RECORDS * (long long)sl.x;
     oa[OUT_F] = make_double4_32a(Fd.x, Fd.y, Fd.z, stamp);
-    oa[OUT_T] = make_double4_32a(TA.x, TA.y, TA.z, 0.0);
+    oa[OUT_T] = make_double4_32a(TA.x, TA.y, TA.z, stamp);
   }
   double4_32a* ob = c.out + OUT_RECORDS * (long long)sl.y;
   ob[OUT_F] = make_double4_32a(-Fd.x, -Fd.y, -Fd.z, stamp);
-  ob[OUT_T] = make_double4_32a(TB.x, TB.y, TB.z, 0.0);
+  ob[OUT_T] = make_double4_32a(TB.x, TB.y, TB.z, stamp);
   if (p.rowMask) {
     const uchar2 rb = c.rowBit[i];
     if (PERI || !(sb & CS_FACET)) atomicOr(&p.rowMask[a], 1u << rb.x);

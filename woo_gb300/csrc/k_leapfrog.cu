@@ -30,47 +30,60 @@ __device__ __forceinline__ void gatherRow(long long want, int i, const Contacts&
   }
 }
 
-// The same sum over the entries of the row that the contact pass marked in the particle's row mask, in the
-// row's order: an entry outside the mask was not stamped by that pass; a stale bit (from a pass before a
-// rebuild) fails the stamp test as in gatherRow.
-__device__ __forceinline__ void gatherRowMasked(long long want, int i, unsigned mask, const Contacts& c, const Csr& csr,
-                                                d3& F, d3& T) {
-  const int e0 = csr.rowptr[i], e1 = csr.rowptr[i + 1];
+// The same sum over the entries of the row [e0, e1) that the contact pass marked in the particle's row mask, in
+// the row's order: an entry outside the mask was not stamped by that pass; a stale bit (from a pass before a
+// rebuild) fails the stamp test as in gatherRow.  WHAT selects the force and the torque records: the integrator's
+// list pass sums them in two threads of different warps (both records carry the stamp).  Up to four records are
+// loaded before the first is added: the sum is one chain of FP64 additions, and a load per link would put an L2
+// round trip into each.
+enum { SUM_F = 1, SUM_T = 2 };
+template <int WHAT>
+__device__ __forceinline__ void gatherRowMasked(long long want, int e0, int e1, unsigned mask, const Contacts& c, d3& F,
+                                                d3& T) {
+  constexpr int B = WHAT == (SUM_F | SUM_T) ? 2 : 4;
+  constexpr int rec = WHAT == SUM_T ? OUT_T : OUT_F;
   unsigned lo = mask & 0x7fffffffu;
   while (lo) {
-    const int e = e0 + __ffs(lo) - 1;
-    lo &= lo - 1;
-    if (e >= e1) break;
-    const double4_32a* o = c.out + OUT_RECORDS * (long long)e;
-    const double4_32a f4 = o[OUT_F];
-    if (__double_as_longlong(f4.w) != want) continue;
-    F = F + xyz(f4);
-    T = T + xyz(o[OUT_T]);
+    double4_32a f[B], t[B];
+    bool on[B];
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      const int e = e0 + __ffs(lo) - 1;  // lo = 0: e0 - 1, not loaded
+      on[k] = lo != 0 && e < e1;
+      lo &= lo - 1;
+      if (on[k]) {
+        f[k] = c.out[OUT_RECORDS * (long long)e + rec];
+        if (WHAT == (SUM_F | SUM_T)) t[k] = c.out[OUT_RECORDS * (long long)e + OUT_T];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      if (!on[k] || __double_as_longlong(f[k].w) != want) continue;
+      if (WHAT == SUM_T) T = T + xyz(f[k]);
+      else F = F + xyz(f[k]);
+      if (WHAT == (SUM_F | SUM_T)) T = T + xyz(t[k]);
+    }
   }
   if (mask & 0x80000000u) {
     for (int e = e0 + 31; e < e1; e++) {
       const double4_32a* o = c.out + OUT_RECORDS * (long long)e;
-      const double4_32a f4 = o[OUT_F];
-      if (__double_as_longlong(f4.w) != want) continue;
-      F = F + xyz(f4);
-      T = T + xyz(o[OUT_T]);
+      const double4_32a r = o[rec];
+      if (__double_as_longlong(r.w) != want) continue;
+      if (WHAT == SUM_T) T = T + xyz(r);
+      else F = F + xyz(r);
+      if (WHAT == (SUM_F | SUM_T)) T = T + xyz(o[OUT_T]);
     }
   }
 }
 
-__device__ __forceinline__ void gatherForce(const StepParams& P, long long want, int i, double mass, unsigned flags,
-                                            const Contacts& c, const Csr& csr, d3& F, d3& T) {
-  const bool grav = P.hasGravity && !(flags & WDEM_GRAVITY_SKIP);
-  if (grav) {
-    // mass * g; a component of g that is exactly zero gives a zero of the sign of the (finite) mass,
-    // set without the multiply (g is uniform over the scene, so the branch does not diverge)
-    const bool mf = finiteBits(mass);
-    F.x = (zeroBits(P.gravity[0]) && mf) ? signedZero(mass, P.gravity[0]) : mass * P.gravity[0];
-    F.y = (zeroBits(P.gravity[1]) && mf) ? signedZero(mass, P.gravity[1]) : mass * P.gravity[1];
-    F.z = (zeroBits(P.gravity[2]) && mf) ? signedZero(mass, P.gravity[2]) : mass * P.gravity[2];
-  } else F = mk(0, 0, 0);
-  T = mk(0, 0, 0);
-  gatherRow(want, i, c, csr, F, T);
+// m g of a node (zero without gravity); a component of g that is exactly zero gives a zero of the sign of the
+// (finite) mass, set without the multiply (g is uniform over the scene, so the branch does not diverge)
+__device__ __forceinline__ d3 gravityForce(const StepParams& P, double mass, unsigned flags) {
+  if (!P.hasGravity || (flags & WDEM_GRAVITY_SKIP)) return mk(0, 0, 0);
+  const bool mf = finiteBits(mass);
+  return mk((zeroBits(P.gravity[0]) && mf) ? signedZero(mass, P.gravity[0]) : mass * P.gravity[0],
+            (zeroBits(P.gravity[1]) && mf) ? signedZero(mass, P.gravity[1]) : mass * P.gravity[1],
+            (zeroBits(P.gravity[2]) && mf) ? signedZero(mass, P.gravity[2]) : mass * P.gravity[2]);
 }
 
 // Raises the collider trigger.  All particles of a free-falling cloud cross the verlet distance in the
@@ -160,7 +173,10 @@ __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   const long long step = stepOf(P, st);
   if (i >= n || haltedIntegrator(st, step)) return;
-  if (p.rowMask) p.rowMask[i] = 0;  // this path gathers whole rows; the marks of the last pass are consumed
+  // the marks of the last contact pass are consumed here
+  const unsigned marks = p.rowMask[i];
+  p.rowMask[i] = 0;
+  const int row0 = csr.rowptr[i], row1 = csr.rowptr[i + 1];
   const int4 meta = p.meta[i];
   const unsigned flags = (unsigned)meta.w;
   const bool asph = ELL && (meta.x & META_ASPH);
@@ -173,7 +189,9 @@ __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int
     F = xyz(p.force[i]);
     T = xyz(p.torque[i]);
   } else if (!blockedAll) {
-    gatherForce(P, seqOf(P, st) - 1, i, mass, flags, c, csr, F, T);
+    F = gravityForce(P, mass, flags);
+    T = mk(0, 0, 0);
+    gatherRowMasked<SUM_F | SUM_T>(seqOf(P, st) - 1, row0, row1, marks, c, F, T);
   } else {
     // the force on a fully blocked node changes nothing in its motion; it is materialised only
     // when downloaded (k_reduce_forces)
@@ -361,8 +379,8 @@ __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int
 // ulp) need neither |w| nor the axis: the vector part sin(h) w/|w| = w dt/2 (1 - h^2/6 (1 - h^2/20))
 // with h^2 = |w|^2 dt^2/4.  The normalisation 1/sqrt(z) of a product of unit quaternions (|z - 1| a
 // few ulp) is its Taylor polynomial 1 - e/2 + 3e^2/8, e = z - 1 (error 5e^3/16, far below an ulp).
-__device__ __forceinline__ void rotateSphere(const StepParams& P, const Particles& p, unsigned i, d3 angVel, int mat) {
-  const double4_32a o4 = p.ori[i];
+__device__ __forceinline__ void rotateSphere(const StepParams& P, const Particles& p, unsigned i, const double4_32a o4,
+                                             d3 angVel, int mat) {
   qd ori; ori.w = o4.x; ori.x = o4.y; ori.y = o4.z; ori.z = o4.w;
   const double dt = dtOf(P, mat);
   const double w2 = sqnorm(angVel);
@@ -431,39 +449,31 @@ __device__ __forceinline__ FastRec loadFast(const Particles& p, int i) {
   return r;
 }
 
+// Translation: force, damping, velocity, position, the FP32 shadow and the verlet trigger.  SPLIT: called by the
+// list pass, where another thread turns the particle.
 template <bool PERI>
-__device__ __forceinline__ void integrateFast(const StepParams& P, const Particles& p, const int i, const int n, const Contacts& c,
-                                              const Csr& csr, DeviceStatus* st, const bool touchedNow, const FastRec& rec,
-                                              const unsigned rowMask) {
+__device__ __forceinline__ void translateFast(const StepParams& P, const Particles& p, const int i, DeviceStatus* st,
+                                              const bool touchedNow, const FastRec& rec, const d3& contactF) {
   const int4 meta = rec.meta;
   const unsigned flags = (unsigned)meta.w;
   const double4_32a vm = rec.vm;
   const double mass = vm.w;
   const bool blockedAll = (flags & 63u) == 63u;
   const bool blockedNone = (flags & 63u) == 0u;
-  d3 F, T;
   const bool grav = P.hasGravity && !(flags & WDEM_GRAVITY_SKIP);
   const bool damp = (P.dampOn && !(flags & WDEM_DAMPING_SKIP));
   // the gravity-only path takes its acceleration from the cache; without damping nothing reads m g
   // along the gravity axis then
   const int skipAxis = (blockedNone && grav && !touchedNow && P.gravAxis >= 0 && !damp) ? P.gravAxis : -1;
-  if (!blockedAll) {
-    if (grav) {
-      const bool mf = finiteBits(mass);
-      F = mk(gravForce(mass, mf, P.gravity[0], skipAxis == 0), gravForce(mass, mf, P.gravity[1], skipAxis == 1),
-             gravForce(mass, mf, P.gravity[2], skipAxis == 2));
-    } else F = mk(0, 0, 0);
-    T = mk(0, 0, 0);
-    if (touchedNow) gatherRowMasked(seqOf(P, st) - 1, i, rowMask, c, csr, F, T);
-  } else {
-    F = mk(0, 0, 0); T = mk(0, 0, 0);
+  d3 F = mk(0, 0, 0);
+  if (touchedNow) F = contactF;
+  else if (!blockedAll && grav) {
+    const bool mf = finiteBits(mass);
+    F = mk(gravForce(mass, mf, P.gravity[0], skipAxis == 0), gravForce(mass, mf, P.gravity[1], skipAxis == 1),
+           gravForce(mass, mf, P.gravity[2], skipAxis == 2));
   }
   const double dt = dtOf(P, meta.y);
   d3 vel = xyz(vm);
-  const double4_32a w4 = rec.w4;
-  const double4_32a& w4c = w4;
-  d3 angVel = xyz(w4);
-  bool angChanged = false;
   const double4_32a pr = rec.pr;
   d3 pos = xyz(pr);
   if (!blockedAll) {
@@ -472,7 +482,7 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
       // F = m g exactly: the acceleration along the gravity axis is the cached qdiv(m g, m); the other
       // components are qdiv of signed zeros, i.e. the zeros themselves
       lin = F;
-      if (P.gravAxis == 0) lin.x = w4c.w; else if (P.gravAxis == 1) lin.y = w4c.w; else lin.z = w4c.w;
+      if (P.gravAxis == 0) lin.x = rec.w4.w; else if (P.gravAxis == 1) lin.y = rec.w4.w; else lin.z = rec.w4.w;
     } else if (blockedNone) lin = divBy(F, mass);
     else {
       lin = mk(0, 0, 0);
@@ -508,62 +518,6 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
       vel.y = addScaled(vel.y, dt, lin.y);
       vel.z = addScaled(vel.z, dt, lin.z);
     }
-    if (!isZeroBits(T)) {
-      WDEM_REAL_BRANCH();
-      const d3 inertia = xyz(p.inert[i]);
-      if (!isZeroBits(inertia)) {
-        d3 ang;
-        if (blockedNone) ang = divByEach(T, inertia);
-        else {
-          ang = mk(0, 0, 0);
-          if (!(flags & 8u)) ang.x = ang.x + qdiv(T.x, inertia.x);
-          if (!(flags & 16u)) ang.y = ang.y + qdiv(T.y, inertia.y);
-          if (!(flags & 32u)) ang.z = ang.z + qdiv(T.z, inertia.z);
-        }
-        if (damp) {
-          const double hd = 0.5 * dt;
-          // periodic: the fluctuation spin angVel - spinVec (Cell::pprevFluctAngVel)
-          const d3 w0 = PERI ? mk(addZ(angVel.x, negD(P.spinVec[0])), addZ(angVel.y, negD(P.spinVec[1])),
-                                  addZ(angVel.z, negD(P.spinVec[2])))
-                             : angVel;
-          if (!zeroBits(T.x)) { const int sg = signProd(T.x, w0.x + hd * ang.x); if (sg) ang.x = ang.x * (sg > 0 ? P.dampM : P.dampP); }
-          if (!zeroBits(T.y)) { const int sg = signProd(T.y, w0.y + hd * ang.y); if (sg) ang.y = ang.y * (sg > 0 ? P.dampM : P.dampP); }
-          if (!zeroBits(T.z)) { const int sg = signProd(T.z, w0.z + hd * ang.z); if (sg) ang.z = ang.z * (sg > 0 ? P.dampM : P.dampP); }
-        }
-        angVel.x = addScaled(angVel.x, dt, ang.x);
-        angVel.y = addScaled(angVel.y, dt, ang.y);
-        angVel.z = addScaled(angVel.z, dt, ang.z);
-        angChanged = true;
-      }
-    } else {
-      // a zero torque still divides by the inertia and adds to angVel: that changes angVel only when an
-      // inertia component is not positive (0/0, 0/negative) or angVel holds a -0
-      if (!(meta.x & META_IPOS) || hasNegZero(angVel)) {
-        WDEM_REAL_BRANCH();
-        const d3 inertia = xyz(p.inert[i]);
-        if (!isZeroBits(inertia)) {
-          d3 ang;
-          if (blockedNone) ang = divByEach(T, inertia);
-          else {
-            ang = mk(0, 0, 0);
-            if (!(flags & 8u)) ang.x = ang.x + qdiv(T.x, inertia.x);
-            if (!(flags & 16u)) ang.y = ang.y + qdiv(T.y, inertia.y);
-            if (!(flags & 32u)) ang.z = ang.z + qdiv(T.z, inertia.z);
-          }
-          angVel = angVel + dt * ang;
-          angChanged = true;
-        }
-      }
-    }
-    // periodic spin correction angVel -= deltaSpinVec (Leapfrog.cpp:192-197), for nodes with inertia;
-    // subtracting +0 leaves every value unchanged
-    if (PERI && !P.dSpinZero) {
-      const double4_32a in4 = p.inert[i];
-      if (!isZeroBits(xyz(in4))) {
-        angVel = mk(addZ(angVel.x, negD(P.dSpin[0])), addZ(angVel.y, negD(P.dSpin[1])), addZ(angVel.z, negD(P.dSpin[2])));
-        angChanged = true;
-      }
-    }
   } else if (PERI) {
     // fixed node with GRADV2: velocity correction without acceleration (Leapfrog.cpp:207-211)
     const d3 a = mvecC(P.LmL, P.clsLmL, pos);
@@ -573,47 +527,12 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
   pos.x = addScaledR(pos.x, vel.x, dt);
   pos.y = addScaledR(pos.y, vel.y, dt);
   pos.z = addScaledR(pos.z, vel.z, dt);
-  // leapfrogSphericalRotate; an unrotated, already-normalised orientation is left alone
-  int mx = meta.x;
-  bool rotate = false;
-  if (!isZeroBits(angVel)) {
-    // untouched spheres: rotated from the rotation list in the second pass (spinning spheres are
-    // scattered over most warps, whose FP64 pipe would wait for their few spinning lanes); the second
-    // pass's own (touched) particles rotate here
-    rotate = true;
-    mx &= ~META_ORI_FIXED;
-  } else if (!(mx & META_ORI_FIXED)) {
-    const double4_32a o4 = p.ori[i];
-    qd ori; ori.w = o4.x; ori.x = o4.y; ori.y = o4.z; ori.z = o4.w;
-    const double z2 = ori.x * ori.x + ori.y * ori.y + ori.z * ori.z + ori.w * ori.w;
-    if (isOneBits(z2)) mx |= META_ORI_FIXED;  // normalisation is the identity from now on
-    else {
-      ori = qnormalized(ori);
-      p.ori[i] = make_double4_32a(ori.w, ori.x, ori.y, ori.z);
-    }
-  }
-  if (mx != meta.x) reinterpret_cast<int*>(&p.meta[i])[0] = mx;
   p.posr[i] = make_double4_32a(pos.x, pos.y, pos.z, pr.w);
   const float4 pf = make_float4(truncF(pos.x), truncF(pos.y), truncF(pos.z), truncF(pr.w));
   p.posf[i] = pf;
   p.velm[i] = make_double4_32a(vel.x, vel.y, vel.z, mass);
-  if (angChanged) p.angw[i] = make_double4_32a(angVel.x, angVel.y, angVel.z, w4.w);
   if (!finiteBits(pos.x) || !finiteBits(pos.y) || !finiteBits(pos.z)) {
     if (atomicCAS(&st->code, 0, WDEM_ERR_NAN) == 0) st->detail = i;
-  }
-  if (touchedNow) {
-    if (rotate) rotateSphere(P, p, (unsigned)i, angVel, meta.y);
-  } else {
-    const unsigned am = __activemask();
-    const unsigned b = __ballot_sync(am, rotate);
-    if (b) {
-      const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
-      unsigned base = 0;
-      if (lane == leader) base = atomicAdd(&st->rotCount, (unsigned)__popc(b));
-      base = __shfl_sync(am, base, leader);
-      const unsigned slot = base + __popc(b & ((1u << lane) - 1));
-      if (rotate && slot < (unsigned)n) p.rotList[slot] = (unsigned)i;
-    }
   }
   // aabbIsDirty (moved^2 > verletDist^2): FP32 distance of the shadows with a bound on its error
   // (truncation < 2^-23 relative per coordinate, FP32 arithmetic a few 2^-24 of the distance)
@@ -630,6 +549,104 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
     dirty = sqnorm(dd) > P.maxD2;
   }
   raiseDirty(st, dirty, stepOf(P, st));
+}
+
+// Rotation: angular velocity from the torque T of the contacts, and whether the orientation turns; returns that
+// (the caller turns it: rotateSphere).  inertia4: Particles.inert of the node where the caller has loaded it
+// (touched nodes read it in any case), else null.
+template <bool PERI>
+__device__ __forceinline__ bool spinFast(const StepParams& P, const Particles& p, const int i, const int4 meta,
+                                         const double4_32a w4, const d3 T, const double4_32a* inertia4, d3& angVel) {
+  const unsigned flags = (unsigned)meta.w;
+  const bool blockedAll = (flags & 63u) == 63u;
+  const bool blockedNone = (flags & 63u) == 0u;
+  const bool damp = (P.dampOn && !(flags & WDEM_DAMPING_SKIP));
+  angVel = xyz(w4);
+  bool angChanged = false;
+  if (!blockedAll) {
+    const double dt = dtOf(P, meta.y);
+    // a zero torque still divides by the inertia and adds to angVel: that changes angVel only when an
+    // inertia component is not positive (0/0, 0/negative) or angVel holds a -0
+    const bool torque = !isZeroBits(T);
+    if (torque || !(meta.x & META_IPOS) || hasNegZero(angVel)) {
+      WDEM_REAL_BRANCH();
+      const d3 inertia = xyz(inertia4 ? *inertia4 : p.inert[i]);
+      if (!isZeroBits(inertia)) {
+        d3 ang;
+        if (blockedNone) ang = divByEach(T, inertia);
+        else {
+          ang = mk(0, 0, 0);
+          if (!(flags & 8u)) ang.x = ang.x + qdiv(T.x, inertia.x);
+          if (!(flags & 16u)) ang.y = ang.y + qdiv(T.y, inertia.y);
+          if (!(flags & 32u)) ang.z = ang.z + qdiv(T.z, inertia.z);
+        }
+        if (torque) {
+          if (damp) {
+            const double hd = 0.5 * dt;
+            // periodic: the fluctuation spin angVel - spinVec (Cell::pprevFluctAngVel)
+            const d3 w0 = PERI ? mk(addZ(angVel.x, negD(P.spinVec[0])), addZ(angVel.y, negD(P.spinVec[1])),
+                                    addZ(angVel.z, negD(P.spinVec[2])))
+                               : angVel;
+            if (!zeroBits(T.x)) { const int sg = signProd(T.x, w0.x + hd * ang.x); if (sg) ang.x = ang.x * (sg > 0 ? P.dampM : P.dampP); }
+            if (!zeroBits(T.y)) { const int sg = signProd(T.y, w0.y + hd * ang.y); if (sg) ang.y = ang.y * (sg > 0 ? P.dampM : P.dampP); }
+            if (!zeroBits(T.z)) { const int sg = signProd(T.z, w0.z + hd * ang.z); if (sg) ang.z = ang.z * (sg > 0 ? P.dampM : P.dampP); }
+          }
+          angVel.x = addScaled(angVel.x, dt, ang.x);
+          angVel.y = addScaled(angVel.y, dt, ang.y);
+          angVel.z = addScaled(angVel.z, dt, ang.z);
+        } else angVel = angVel + dt * ang;
+        angChanged = true;
+      }
+    }
+    // periodic spin correction angVel -= deltaSpinVec (Leapfrog.cpp:192-197), for nodes with inertia;
+    // subtracting +0 leaves every value unchanged
+    if (PERI && !P.dSpinZero) {
+      const double4_32a in4 = inertia4 ? *inertia4 : p.inert[i];
+      if (!isZeroBits(xyz(in4))) {
+        angVel = mk(addZ(angVel.x, negD(P.dSpin[0])), addZ(angVel.y, negD(P.dSpin[1])), addZ(angVel.z, negD(P.dSpin[2])));
+        angChanged = true;
+      }
+    }
+  }
+  if (angChanged) p.angw[i] = make_double4_32a(angVel.x, angVel.y, angVel.z, w4.w);
+  // leapfrogSphericalRotate; an unrotated, already-normalised orientation is left alone
+  int mx = meta.x;
+  bool rotate = false;
+  if (!isZeroBits(angVel)) {
+    rotate = true;
+    mx &= ~META_ORI_FIXED;
+  } else if (!(mx & META_ORI_FIXED)) {
+    const double4_32a o4 = p.ori[i];
+    qd ori; ori.w = o4.x; ori.x = o4.y; ori.y = o4.z; ori.z = o4.w;
+    const double z2 = ori.x * ori.x + ori.y * ori.y + ori.z * ori.z + ori.w * ori.w;
+    if (isOneBits(z2)) mx |= META_ORI_FIXED;  // normalisation is the identity from now on
+    else {
+      ori = qnormalized(ori);
+      p.ori[i] = make_double4_32a(ori.w, ori.x, ori.y, ori.z);
+    }
+  }
+  if (mx != meta.x) reinterpret_cast<int*>(&p.meta[i])[0] = mx;
+  return rotate;
+}
+
+// A node without contact forces, in the first pass: untouched spinning spheres go to the rotation list of the
+// second pass (they are scattered over most warps, whose FP64 pipe would wait for their few spinning lanes).
+template <bool PERI>
+__device__ __forceinline__ void integrateFast(const StepParams& P, const Particles& p, const int i, const int n,
+                                              DeviceStatus* st, const FastRec& rec) {
+  d3 angVel;
+  const bool rotate = spinFast<PERI>(P, p, i, rec.meta, rec.w4, mk(0, 0, 0), nullptr, angVel);
+  const unsigned am = __activemask();
+  const unsigned b = __ballot_sync(am, rotate);
+  if (b) {
+    const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
+    unsigned base = 0;
+    if (lane == leader) base = atomicAdd(&st->rotCount, (unsigned)__popc(b));
+    base = __shfl_sync(am, base, leader);
+    const unsigned slot = base + __popc(b & ((1u << lane) - 1));
+    if (rotate && slot < (unsigned)n) p.rotList[slot] = (unsigned)i;
+  }
+  translateFast<PERI>(P, p, i, st, false, rec, mk(0, 0, 0));
 }
 
 // First pass: particles without contact forces this step.  Those that a real contact touched are
@@ -659,7 +676,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_leapfrog_fast(StepParams P, P
       if (listed && slot < (unsigned)n) p.touchList[slot] = (unsigned)i;
     }
     if (listed) return;
-    integrateFast<PERI>(P, p, i, n, c, csr, st, false, rec, 0u);
+    integrateFast<PERI>(P, p, i, n, st, rec);
   } else {
     constexpr int NW = BS / 32;
     __shared__ unsigned sCnt[2][NW];
@@ -711,29 +728,55 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_leapfrog_fast(StepParams P, P
       if (mine && j != i) rec = loadFast(p, j);  // the block loaded it a moment ago
     }
     if (!mine) return;
-    integrateFast<PERI>(P, p, j, n, c, csr, st, false, rec, 0u);
+    integrateFast<PERI>(P, p, j, n, st, rec);
   }
 }
 
-// Second pass, over two lists: the touched particles (CSR force gather, full integration, rotation
-// inline), then the rotation list of the first pass.
+// Second pass, over two lists: the touched particles (CSR force gather, full integration), then the rotation list
+// of the first pass.  A touched particle takes two threads, in different warps: one gathers the forces and moves
+// it, the other gathers the torques and turns it (neither reads what the other computes); each has all its loads
+// in flight at once.  The pass is bound by these dependent chains (list entry, row, records, FP64) more than by
+// bytes or FP64 issue, so two shorter chains side by side beat one.
+static const int LIST_T = 256, LIST_ITEMS = LIST_T / 2;
 template <bool PERI>
-__global__ void __launch_bounds__(256) k_leapfrog_lists(StepParams P, Particles p, int n, Contacts c, Csr csr,
-                                                         DeviceStatus* st) {
+__global__ void __launch_bounds__(LIST_T) k_leapfrog_lists(StepParams P, Particles p, int n, Contacts c, Csr csr,
+                                                            DeviceStatus* st) {
   if (haltedIntegrator(st, stepOf(P, st))) return;
   const unsigned nt = st->touchCount < (unsigned)n ? st->touchCount : (unsigned)n;
   const unsigned nr = st->rotCount < (unsigned)n ? st->rotCount : (unsigned)n;
-  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nt + nr; k += gridDim.x * blockDim.x) {
-    if (k < nt) {
-      const int i = (int)p.touchList[k];
-      p.touched[i] = 0;
-      const unsigned m = p.rowMask[i];
-      p.rowMask[i] = 0;
-      integrateFast<PERI>(P, p, i, n, c, csr, st, true, loadFast(p, i), m);
-    } else {
-      const unsigned i = p.rotList[k - nt];
-      rotateSphere(P, p, i, xyz(p.angw[i]), p.meta[i].y);
+  const long long want = seqOf(P, st) - 1;
+  const bool turns = threadIdx.x >= LIST_ITEMS;
+  const unsigned lane = threadIdx.x & (LIST_ITEMS - 1);
+  for (unsigned base = blockIdx.x * LIST_ITEMS; base < nt; base += gridDim.x * LIST_ITEMS) {
+    const unsigned k = base + lane;
+    const bool live = k < nt;
+    const int i = live ? (int)p.touchList[k] : 0;
+    unsigned mask = 0;
+    if (live) mask = p.rowMask[i];
+    __syncthreads();  // both threads of a particle have its mask
+    if (live) {
+      if (!turns) {
+        const int e0 = csr.rowptr[i], e1 = csr.rowptr[i + 1];
+        const FastRec rec = loadFast(p, i);
+        d3 F = gravityForce(P, rec.vm.w, (unsigned)rec.meta.w), T;
+        gatherRowMasked<SUM_F>(want, e0, e1, mask, c, F, T);
+        p.touched[i] = 0;
+        p.rowMask[i] = 0;
+        translateFast<PERI>(P, p, i, st, true, rec, F);
+      } else {
+        const int e0 = csr.rowptr[i], e1 = csr.rowptr[i + 1];
+        const int4 meta = p.meta[i];
+        const double4_32a w4 = p.angw[i], in4 = p.inert[i], o4 = p.ori[i];
+        d3 F, T = mk(0, 0, 0), angVel;
+        gatherRowMasked<SUM_T>(want, e0, e1, mask, c, F, T);
+        if (spinFast<PERI>(P, p, i, meta, w4, T, &in4, angVel)) rotateSphere(P, p, (unsigned)i, o4, angVel, meta.y);
+      }
     }
+  }
+  for (unsigned k = blockIdx.x * LIST_T + threadIdx.x; k < nr; k += gridDim.x * LIST_T) {
+    const unsigned i = p.rotList[k];
+    const double4_32a o4 = p.ori[i];
+    rotateSphere(P, p, i, o4, xyz(p.angw[i]), p.meta[i].y);
   }
 }
 
@@ -743,7 +786,7 @@ template <bool PERI>
 static unsigned listGrid(const StepParams& P) {
   static int per = 0;
   if (per == 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_leapfrog_lists<PERI>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_leapfrog_lists<PERI>, LIST_T, 0);
     per = std::max(1, per);
   }
   const int sms = P.numSMs > 0 ? P.numSMs : 152;
@@ -772,17 +815,18 @@ void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, in
                      DeviceStatus* st) {
   if (n <= 0) return;
   unsigned blocks = (n + 255) / 256;
+  const unsigned listBlocks = (unsigned)((n + LIST_ITEMS - 1) / LIST_ITEMS);
   if (!fromArrays && !P.hasEll && !P.lfEnergy && p.touched && p.rotList) {
     // st->rotCount and st->touchCount are zero here: k_contacts_cull clears them for the next step (and
     // the handle starts at zero)
     if (P.periodic) {
-      const unsigned rb = std::min(blocks, listGrid<true>(P));
+      const unsigned rb = std::min(listBlocks, listGrid<true>(P));
       launchFast<true>(s, P, p, n, c, csr, st);
-      (k_leapfrog_lists<true><<<rb, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+      (k_leapfrog_lists<true><<<rb, LIST_T, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
     } else {
-      const unsigned rb = std::min(blocks, listGrid<false>(P));
+      const unsigned rb = std::min(listBlocks, listGrid<false>(P));
       launchFast<false>(s, P, p, n, c, csr, st);
-      (k_leapfrog_lists<false><<<rb, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+      (k_leapfrog_lists<false><<<rb, LIST_T, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
     }
     return;
   }
@@ -850,20 +894,66 @@ void launch_dyndt(cudaStream_t s, const StepParams& P, Particles p, int n, Conta
   (k_dyndt<<<(n + 127) / 128, 128, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
 }
 
-// DemData.force/torque as Woo holds them after ContactLoop (reset to m*g by Leapfrog, then contacts)
-__global__ void k_reduce_forces(StepParams P, Particles p, int n, Contacts c, Csr csr) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int4 meta = p.meta[i];
-  d3 F, T;
-  gatherForce(P, P.seq - 1, i, p.velm[i].w, (unsigned)meta.w, c, csr, F, T);
-  p.force[i] = make_double4_32a(F.x, F.y, F.z, 0);
-  p.torque[i] = make_double4_32a(T.x, T.y, T.z, 0);
+// DemData.force/torque as Woo holds them after ContactLoop (reset to m*g by Leapfrog, then contacts).
+// Rows up to REDUCE_ROW entries are summed by one thread.  A wall's row has an entry for every body near it, and
+// one thread walking it was the whole kernel (1167 us for the beds of 120k spheres, whose walls have 2,500
+// entries): such a row is taken by a warp, which loads 32 records at a time, packs the stamped ones into shared
+// memory in row order, and adds them with one lane per component, so the six sums keep the row's order.
+static const int REDUCE_T = 128, REDUCE_ROW = 64;
+__global__ void __launch_bounds__(REDUCE_T) k_reduce_forces(StepParams P, Particles p, int n, Contacts c, Csr csr) {
+  __shared__ int longRow[REDUCE_T];
+  __shared__ int nLong;
+  __shared__ double packed[REDUCE_T / 32][32][6];
+  const int i = blockIdx.x * REDUCE_T + threadIdx.x;
+  if (threadIdx.x == 0) nLong = 0;
+  __syncthreads();
+  const long long want = P.seq - 1;
+  if (i < n) {
+    if (csr.rowptr[i + 1] - csr.rowptr[i] > REDUCE_ROW) longRow[atomicAdd(&nLong, 1)] = i;
+    else {
+      d3 F = gravityForce(P, p.velm[i].w, (unsigned)p.meta[i].w), T = mk(0, 0, 0);
+      gatherRow(want, i, c, csr, F, T);
+      p.force[i] = make_double4_32a(F.x, F.y, F.z, 0);
+      p.torque[i] = make_double4_32a(T.x, T.y, T.z, 0);
+    }
+  }
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int q = w; q < nLong; q += REDUCE_T / 32) {
+    const int r = longRow[q];
+    const int e0 = csr.rowptr[r], e1 = csr.rowptr[r + 1];
+    double acc = 0.;  // lanes 0-2: force, 3-5: torque
+    const d3 g = gravityForce(P, p.velm[r].w, (unsigned)p.meta[r].w);
+    if (lane < 3) acc = comp(g, lane);
+    double4_32a f, t;
+    auto load = [&](int e) {
+      f.w = 0.;  // stamp 0: no pass
+      if (e < e1) { f = c.out[OUT_RECORDS * (long long)e + OUT_F]; t = c.out[OUT_RECORDS * (long long)e + OUT_T]; }
+    };
+    load(e0 + lane);
+    for (int e = e0; e < e1; e += 32) {
+      const bool on = e + lane < e1 && __double_as_longlong(f.w) == want;
+      const unsigned b = __ballot_sync(0xffffffffu, on);
+      if (on) {
+        double* o = packed[w][__popc(b & ((1u << lane) - 1u))];
+        o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = t.x; o[4] = t.y; o[5] = t.z;
+      }
+      load(e + 32 + lane);  // the next 32 records arrive during the additions
+      __syncwarp();
+      const int m = __popc(b);
+      if (lane < 6)
+        for (int k = 0; k < m; k++) acc = acc + packed[w][k][lane];
+      __syncwarp();
+    }
+    if (lane < 6) (lane < 3 ? reinterpret_cast<double*>(&p.force[r]) : reinterpret_cast<double*>(&p.torque[r]) - 3)[lane] = acc;
+    if (lane == 6) p.force[r].w = 0.;
+    if (lane == 7) p.torque[r].w = 0.;
+  }
 }
 
 void launch_reduce_forces(cudaStream_t s, const StepParams& P, Particles p, int n, Contacts c, Csr csr) {
   if (n <= 0) return;
-  (k_reduce_forces<<<(n + 127) / 128, 128, 0, s>>>(P, p, n, c, csr), ++::wdem::g_kernel_launches);
+  (k_reduce_forces<<<(n + REDUCE_T - 1) / REDUCE_T, REDUCE_T, 0, s>>>(P, p, n, c, csr), ++::wdem::g_kernel_launches);
 }
 
 WDEM_VARIANT_END

@@ -22,7 +22,7 @@
 //     tanPhi  double
 //     slot    int2     the contact's two entries in the CSR (pA's, pB's)
 //     out     2 double4_32a records per CSR entry (one 32-byte sector each), written by the contact pass at
-//             the entry's position: (force on the entry's particle, pass stamp), (torque, unused); a particle's
+//             the entry's position: (force on the entry's particle, pass stamp), (torque, pass stamp); a particle's
 //             records are contiguous, so the integrator's gather reads its CSR row as one run
 //   CSR over particles: rowptr[N+1], entries[2C] = contact index | (isB << 31), rows sorted
 //   by the partner's id key so that sums run in the order of the sorted contact keys.
@@ -85,7 +85,8 @@ enum { HIST_T0X = 0, HIST_T0Y, HIST_T0Z, HIST_T1X, HIST_T1Y, HIST_T1Z, HIST_CX, 
        HIST_COUNT };
 enum { HIST_FRICT = HIST_E0 };  // FrictPhys contacts carry the first 14 history arrays
 // records of one CSR entry in Contacts.out: the force with the stamp of the contact pass that wrote it in w
-// (its StepParams.seq; a record whose stamp is not the previous pass's is stale and skipped), the torque
+// (its StepParams.seq; a record whose stamp is not the previous pass's is stale and skipped), the torque with the
+// same stamp
 enum { OUT_F = 0, OUT_T = 1, OUT_RECORDS = 2 };
 enum { MAX_MATERIALS = 1024 };  // 1024 x 56 B fits the 64 KB constant bank
 
