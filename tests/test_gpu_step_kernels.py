@@ -58,3 +58,28 @@ def test_wall_force_over_long_rows(wdem_lib, m):
     spec = scenes.SceneSpec(scenes.default_params(scenes.materials_array(mats), dt=1e-5, gravity=(0, 0, -9.81)), None, pa)
     h, _ = _run_both(spec, (1, 3))
     assert h.status().nReal >= m
+
+
+@pytest.mark.parametrize("n", [1017, 1018, 1019, 2042, 4500])
+def test_rows_of_walls_at_range_edges(wdem_lib, n):
+    """Bodies (with 6 walls) around multiples of 1024, where a wall's row gets another range of partner ids: the
+    force sums need every row in the order of the partner ids, the carry finds old contacts in it."""
+    side = 0.011 * np.ceil(n ** (1.0 / 3.0))
+    spec = scenes.random_cloud(n, n, box=(side, side, side), rmin=0.004, rmax=0.005, dense=0.93)
+    assert spec.particles.n == n + 6
+    h, o = _run_both(spec, (1, 4, 40))
+    assert h.status().nFullRuns == o.n_full_runs() > 1
+
+
+@pytest.mark.parametrize("n", [1, 2, 4095, 4096, 4097, 12289, 135000])
+def test_pairs_at_scan_tile_edges(wdem_lib, n):
+    """Box pairs for counts at the edges of the scan's tiles (4096 values) and, last, beyond the 32 tiles that one
+    look-back reads at a time; the pair set is known: boxes on a line, each meeting the next two."""
+    k = np.random.default_rng(n).permutation(n)
+    lo = np.stack([k * 1.0, np.zeros(n), np.zeros(n)], axis=1)
+    h = abi.Handle(n)
+    got = h.collide_boxes(lo, lo + np.array([2.5, 1.0, 1.0]), np.full(n, 5, np.uint32), 2)
+    at = np.argsort(k)
+    want = np.concatenate([np.stack([at[:-d], at[d:]], axis=1) for d in (1, 2) if n > d] + [np.zeros((0, 2), int)])
+    want = np.sort(want, axis=1)
+    assert np.array_equal(got, want[np.lexsort((want[:, 1], want[:, 0]))])

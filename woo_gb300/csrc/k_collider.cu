@@ -21,6 +21,7 @@
 #include "wdem_math.cuh"
 #include "wdem_peri.cuh"
 #include "../../include/wdem.h"
+#include <algorithm>
 #include <cstdio>
 
 namespace wdem {
@@ -269,67 +270,122 @@ __global__ void k_make_keys(Particles p, const int* small, int nSmall, const Gri
 
 
 // ------------------------------------------------------------------------------------ scan
-// Exclusive scan of a[0..n) in place, a[n] <- total.  Block-wise scan, recursive on block sums.
-static const int SCAN_T = 256, SCAN_I = 4, SCAN_TILE = SCAN_T * SCAN_I;
+// Exclusive scan of a[0..n) in place, a[n] <- total, in one kernel (decoupled look-back, Merrill & Garland 2016).
+// A block takes its tile in the order of a ticket, so every earlier tile is running or done; it publishes the
+// tile's sum, its first warp looks back over 32 earlier tiles at a time up to the nearest published prefix, and it
+// publishes its own prefix.  A published word carries the number of the scan, so nothing is cleared between scans,
+// and the ticket counts on from where the last scan left it.  A rebuild's scans were 3 to 5 launches each before
+// (tile scans, the scan of their sums, the sums added back), of 3 us for 15k bodies.
+static const int SCAN_T = 256, SCAN_I = 16, SCAN_TILE = SCAN_T * SCAN_I;
+static const unsigned SCAN_AGG = 1u, SCAN_PRE = 2u, SCAN_EPOCHS = 1u << 30;
+static const long long SCAN_SPIN = 1ll << 22;
 
-__global__ void k_scan_tiles(unsigned* a, long long n, unsigned* sums) {
-  __shared__ unsigned s[SCAN_T];
-  long long base = (long long)blockIdx.x * SCAN_TILE;
-  unsigned v[SCAN_I];
-  unsigned tsum = 0;
-  for (int k = 0; k < SCAN_I; k++) {
-    long long idx = base + threadIdx.x * SCAN_I + k;
-    v[k] = idx < n ? a[idx] : 0;
-    tsum += v[k];
-  }
-  s[threadIdx.x] = tsum;
+__global__ void __launch_bounds__(SCAN_T) k_scan(unsigned* a, long long n, unsigned long long* status, unsigned* ticket,
+                                                 unsigned ticket0, unsigned epoch, DeviceStatus* st) {
+  __shared__ unsigned tileS, prefixS;
+  __shared__ unsigned warpSum[SCAN_T / 32];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t == 0) tileS = atomicAdd(ticket, 1u) - ticket0;
   __syncthreads();
-  for (int off = 1; off < SCAN_T; off <<= 1) {
-    unsigned t = threadIdx.x >= off ? s[threadIdx.x - off] : 0;
-    __syncthreads();
-    s[threadIdx.x] += t;
-    __syncthreads();
+  const long long tile = tileS;
+  const long long first = tile * SCAN_TILE + (long long)t * SCAN_I;
+  unsigned v[SCAN_I];
+  unsigned sum = 0;
+#pragma unroll
+  for (int k = 0; k < SCAN_I; k += 4) {
+    uint4 q = make_uint4(0, 0, 0, 0);
+    if (first + k + 4 <= n) q = *reinterpret_cast<const uint4*>(a + first + k);
+    else {
+      if (first + k < n) q.x = a[first + k];
+      if (first + k + 1 < n) q.y = a[first + k + 1];
+      if (first + k + 2 < n) q.z = a[first + k + 2];
+    }
+    v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
+    sum += q.x + q.y + q.z + q.w;
   }
-  unsigned run = s[threadIdx.x] - tsum;  // exclusive prefix of this thread
-  for (int k = 0; k < SCAN_I; k++) {
-    long long idx = base + threadIdx.x * SCAN_I + k;
-    if (idx < n) a[idx] = run;
-    run += v[k];
+  unsigned inc = sum;  // inclusive scan of the threads' sums within the warp
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += u;
   }
-  if (threadIdx.x == SCAN_T - 1) sums[blockIdx.x] = s[SCAN_T - 1];
+  if (lane == 31) warpSum[warp] = inc;
+  __syncthreads();
+  unsigned before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < SCAN_T / 32; w++) {
+    if (w < warp) before += warpSum[w];
+    total += warpSum[w];
+  }
+  if (warp == 0) {
+    const unsigned long long tag = (unsigned long long)epoch << 34;
+    unsigned prefix = 0;
+    if (tile > 0) {
+      if (lane == 0) *(volatile unsigned long long*)(status + tile) = tag | ((unsigned long long)SCAN_AGG << 32) | total;
+      for (long long j = tile - 1; j >= 0; j -= 32) {
+        const long long q = j - lane;
+        unsigned long long w = tag | ((unsigned long long)SCAN_PRE << 32);  // before the first tile: prefix 0
+        if (q >= 0) {
+          w = *(volatile unsigned long long*)(status + q);
+          long long it = 0;
+          while ((w >> 34) != epoch || ((w >> 32) & 3u) == 0) {
+            if (++it > SCAN_SPIN) {
+              atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT);
+              w = tag | ((unsigned long long)SCAN_PRE << 32);
+              break;
+            }
+            __nanosleep(20);
+            w = *(volatile unsigned long long*)(status + q);
+          }
+        }
+        const unsigned pre = __ballot_sync(0xffffffffu, ((w >> 32) & 3u) == SCAN_PRE);
+        const int stop = pre ? __ffs(pre) - 1 : 31;  // the nearest tile whose prefix is known
+        prefix += __reduce_add_sync(0xffffffffu, lane <= stop ? (unsigned)w : 0u);
+        if (pre) break;
+      }
+    }
+    if (lane == 0) {
+      *(volatile unsigned long long*)(status + tile) = tag | ((unsigned long long)SCAN_PRE << 32) | (prefix + total);
+      prefixS = prefix;
+    }
+  }
+  __syncthreads();
+  unsigned run = prefixS + before + (inc - sum);
+#pragma unroll
+  for (int k = 0; k < SCAN_I; k += 4) {
+    uint4 q;
+    q.x = run; run += v[k];
+    q.y = run; run += v[k + 1];
+    q.z = run; run += v[k + 2];
+    q.w = run; run += v[k + 3];
+    if (first + k + 4 <= n) *reinterpret_cast<uint4*>(a + first + k) = q;
+    else {
+      if (first + k < n) a[first + k] = q.x;
+      if (first + k + 1 < n) a[first + k + 1] = q.y;
+      if (first + k + 2 < n) a[first + k + 2] = q.z;
+    }
+  }
+  // the thread after the last value (of the last tile, also when n fills it) holds the total
+  if ((tile + 1) * SCAN_TILE >= n && t == SCAN_T - 1) a[n] = prefixS + total;
 }
 
+// 32-bit words of scan scratch (ticket, then one 64-bit status word per tile) for scans of n values
+long long scan_scratch_words(long long n) { return 64 + 2 * ((n + SCAN_TILE - 1) / SCAN_TILE + 1); }
 
-
-// Exclusive scan of a[0..n) in place with the total written to a[n]: tile scans, the tile sums scanned by
-// the same routine (which leaves their total at sums[nb]), then the sums added back; with one tile the
-// tile kernel writes the total itself.
-__global__ void k_scan_add(unsigned* a, long long n, const unsigned* sums, long long nb) {
-  long long base = (long long)blockIdx.x * SCAN_TILE;
-  unsigned add = sums[blockIdx.x];
-  for (int k = 0; k < SCAN_I; k++) {
-    long long idx = base + threadIdx.x * SCAN_I + k;
-    if (idx < n) a[idx] += add;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) a[n] = sums[nb];
-}
-
-static void scan_rec(cudaStream_t s, unsigned* a, long long n, unsigned* scratch) {
-  long long nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-  if (nb == 0) {
+void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs) {
+  if (n <= 0) {
     cudaMemsetAsync(a, 0, sizeof(unsigned), s);  // empty: total 0
     return;
   }
-  unsigned* sums = scratch;  // nb + 1 entries
-  (k_scan_tiles<<<(unsigned)nb, SCAN_T, 0, s>>>(a, n, nb == 1 ? a + n : sums), ++::wdem::g_kernel_launches);
-  if (nb > 1) {
-    scan_rec(s, sums, nb, scratch + ((nb + 1 + 63) & ~63ll));
-    (k_scan_add<<<(unsigned)nb, SCAN_T, 0, s>>>(a, n, sums, nb), ++::wdem::g_kernel_launches);
+  if (++cs.scanEpoch >= SCAN_EPOCHS) {  // the numbers start again: no word of the old ones may be left
+    cudaMemsetAsync(cs.scanScratch, 0, cs.scanCap * sizeof(unsigned), s);
+    cs.scanEpoch = 1;
+    cs.scanTickets = 0;
   }
-}
-
-void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs) {
-  scan_rec(s, a, n, cs.blockSums + 64);
+  const unsigned nt = (unsigned)((n + SCAN_TILE - 1) / SCAN_TILE);
+  (k_scan<<<nt, SCAN_T, 0, s>>>(a, n, reinterpret_cast<unsigned long long*>(cs.scanScratch + 64), cs.scanScratch,
+                                cs.scanTickets, cs.scanEpoch, cs.st),
+   ++::wdem::g_kernel_launches);
+  cs.scanTickets += nt;
 }
 
 // ------------------------------------------------------------------------------------ radix sort
@@ -725,19 +781,53 @@ __global__ void k_retain_write(Contacts old, long long nOld, const unsigned* fla
 
 // ------------------------------------------------------------------------------------ old-contact lookup
 // The contact of the pair (a, b) in the container whose CSR is `csr` (built at the last rebuild or upload):
-// binary search of the partner in the row of the lower id, whose keys are sorted by partner; -1 if none.
+// binary search of the partner in the row of the lower id, which is sorted by partner; -1 if none.
 __device__ __forceinline__ long long csrFind(const Csr& csr, int a, int b) {
   const int lo = min(a, b), hi = max(a, b);
   if (lo < 0 || hi >= csr.n) return -1;  // ids the rows do not cover (appended since) had no contact
-  const unsigned long long key = ((unsigned long long)(unsigned)lo << csr.idBits) | (unsigned)hi;
   int l = csr.rowptr[lo], r = csr.rowptr[lo + 1];
+  const int end = r;
   while (l < r) {
     const int m = (l + r) >> 1;
-    if (csr.keys[m] < key) l = m + 1; else r = m;
+    if (csr.partner[m] < (unsigned)hi) l = m + 1; else r = m;
   }
-  if (l < csr.rowptr[lo + 1] && csr.keys[l] == key) return (long long)(csr.ent[l] & 0x7fffffffu);
+  if (l < end && csr.partner[l] == (unsigned)hi) return (long long)(csr.ent[l] & 0x7fffffffu);
   return -1;
 }
+
+// ------------------------------------------------------------------------------------ CSR rows
+// The CSR is built by counting: every entry takes a place in its row (one atomic per entry), a scan of the rows'
+// counts gives their starts, the entries go to their places, and each entry's rank among its row's partners is its
+// final position.  Rows hold ten or twenty entries, so the ranks are a few loads from L1; the order does not depend
+// on the atomics.  The radix sort of 2 C keys of up to 46 bits this replaces took 6 passes over 12 bytes an entry
+// (9 sorting launches a rebuild with 500k bodies and 2 M pairs, 730 us of 2 rebuilds; this: see k_csr_rank).
+// A wall's or facet's row can hold every body: it is divided into V ranges of S partner ids, counted apart (so the
+// atomics spread as well), and an entry is ranked within its range.
+struct RowCount {
+  unsigned* cnt;        // rowptr as counts, then starts
+  unsigned* sub;        // nLarge x V counts of the large bodies' ranges, then starts within their rows
+  const int* largeIdx;  // index of a body in the large list, -1 for the others
+  int V, S;
+};
+// V ranges for each of nLarge bodies of n: about n ranges in all, none of fewer than 1024 ids
+static void largeRanges(int n, int nLarge, int& V, int& S) {
+  V = 1;
+  if (nLarge > 0) V = std::max(1, std::min(n / 1024 + 1, n / nLarge));
+  S = (n + V - 1) / V;
+  if (S < 1) S = 1;
+}
+// index of the range that partner's entry in a large body's row falls into, -1 for the other rows
+__device__ __forceinline__ int rangeOf(const RowCount& R, int row, int partner, bool maybeLarge) {
+  if (!maybeLarge) return -1;
+  const int l = R.largeIdx[row];
+  return l < 0 ? -1 : l * R.V + partner / R.S;
+}
+__device__ __forceinline__ int takePlace(const RowCount& R, int row, int partner, bool maybeLarge) {
+  const int k = rangeOf(R, row, partner, maybeLarge);
+  return (int)atomicAdd(k < 0 ? &R.cnt[row] : &R.sub[k], 1u);
+}
+// pairs with a wall or a facet carry one of these bits (and so do pairs without a functor)
+__device__ __forceinline__ bool maybeLarge(uint8_t state) { return (state & (CS_WALL_A | CS_WALL_B | CS_FACET)) != 0; }
 
 // ------------------------------------------------------------------------------------ carry-over
 // History of pairs already in the container is copied; new pairs start as potential contacts
@@ -766,7 +856,8 @@ __global__ void k_part_flag(Contacts neu, long long nNew, Contacts old, Csr oldC
   flag[c] = f;
 }
 __global__ void k_carry_compact(Particles p, Contacts neu, long long nNew, Contacts old, const unsigned long long* tmpIds,
-                                const unsigned* tmpJ, const unsigned* scan, const int4* tmpDist, long long step, int nHist) {
+                                const unsigned* tmpJ, const unsigned* scan, const int4* tmpDist, long long step, int nHist,
+                                RowCount R) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nNew) return;
   const unsigned before = scan[c];
@@ -782,14 +873,18 @@ __global__ void k_carry_compact(Particles p, Contacts neu, long long nNew, Conta
     neu.state[d] = CS_POTENTIAL | sb;
     neu.step0[d] = (int)step;
     if (neu.lam) neu.lam[d] = __longlong_as_double(0x7ff8000000000000ll);
+    neu.slot[d] = make_int2(takePlace(R, id.x, id.y, maybeLarge(sb)), takePlace(R, id.y, id.x, maybeLarge(sb)));
     return;
   }
   const long long j = jj;
   if (neu.lam && old.lam) neu.lam[d] = old.lam[j];
   else if (neu.lam) neu.lam[d] = __longlong_as_double(0x7ff8000000000000ll);
-  neu.ids[d] = old.ids[j];  // keep the stored orientation (and, periodic, the stored cellDist)
+  const uint8_t sh = old.state[j] & CS_SHAPES;
+  const int2 oid = old.ids[j];
+  neu.ids[d] = oid;  // keep the stored orientation (and, periodic, the stored cellDist)
+  neu.slot[d] = make_int2(takePlace(R, oid.x, oid.y, maybeLarge(sh)), takePlace(R, oid.y, oid.x, maybeLarge(sh)));
   if (neu.cdist) neu.cdist[d] = old.cdist ? old.cdist[j] : tmpDist[c];
-  neu.state[d] = (wasReal ? CS_REAL : CS_POTENTIAL) | (old.state[j] & CS_SHAPES);
+  neu.state[d] = (wasReal ? CS_REAL : CS_POTENTIAL) | sh;
   neu.step0[d] = old.step0[j];
   if (wasReal) {
     for (int h = 0; h < nHist; h++) neu.hist[h][d] = old.hist[h][j];
@@ -798,40 +893,78 @@ __global__ void k_carry_compact(Particles p, Contacts neu, long long nNew, Conta
 }
 
 // ------------------------------------------------------------------------------------ CSR
-__global__ void k_csr_entries(Contacts c, long long nc, int idBits, unsigned long long* keys, unsigned* vals) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// places in the rows of an uploaded container's contacts (a rebuild takes them in k_carry_compact)
+__global__ void k_csr_places(Contacts c, long long nc, RowCount R) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nc) return;
-  int2 id = c.ids[e];
-  keys[2 * e] = ((unsigned long long)(unsigned)id.x << idBits) | (unsigned)id.y;
-  vals[2 * e] = (unsigned)e;
-  keys[2 * e + 1] = ((unsigned long long)(unsigned)id.y << idBits) | (unsigned)id.x;
-  vals[2 * e + 1] = (unsigned)e | 0x80000000u;
+  const int2 id = c.ids[e];
+  const bool big = maybeLarge(c.state[e]);
+  c.slot[e] = make_int2(takePlace(R, id.x, id.y, big), takePlace(R, id.y, id.x, big));
 }
-// the sorted entries, and each contact's two entry positions (where the contact pass writes its shares)
-// with their positions in the rows (which bit of the row's mask the contact pass sets)
-__global__ void k_csr_ent_slots(const unsigned* vals, const unsigned long long* keys, int idBits, const int* rowptr,
-                                long long ne, unsigned* ent, int2* slot, uchar2* rowBit) {
+// the ranges of one large body: counts to starts within its row (one block a body); the row's length to cnt
+__global__ void __launch_bounds__(256) k_csr_large(const int* large, RowCount R) {
+  __shared__ unsigned warpSum[8];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  unsigned* sub = R.sub + (long long)blockIdx.x * R.V;
+  unsigned carry = 0;
+  for (int base = 0; base < R.V; base += 256) {
+    const unsigned v = base + t < R.V ? sub[base + t] : 0;
+    unsigned inc = v;
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += u;
+    }
+    if (lane == 31) warpSum[warp] = inc;
+    __syncthreads();
+    unsigned before = 0, total = 0;
+    for (int w = 0; w < 8; w++) {
+      if (w < warp) before += warpSum[w];
+      total += warpSum[w];
+    }
+    if (base + t < R.V) sub[base + t] = carry + before + inc - v;
+    carry += total;
+    __syncthreads();
+  }
+  if (t == 0) R.cnt[large[blockIdx.x]] = carry;
+}
+// the entries at their places: (partner, contact | isB << 31)
+__global__ void k_csr_fill(Contacts c, long long nc, RowCount R, unsigned long long* tmp) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nc) return;
+  const int2 id = c.ids[e], place = c.slot[e];
+  const bool big = maybeLarge(c.state[e]);
+  const int kA = rangeOf(R, id.x, id.y, big), kB = rangeOf(R, id.y, id.x, big);
+  tmp[R.cnt[id.x] + (kA < 0 ? 0u : R.sub[kA]) + place.x] = ((unsigned long long)(unsigned)id.y << 32) | (unsigned)e;
+  tmp[R.cnt[id.y] + (kB < 0 ? 0u : R.sub[kB]) + place.y] = ((unsigned long long)(unsigned)id.x << 32) | ((unsigned)e | 0x80000000u);
+}
+// Each entry's final position: the start of its row (or range) plus the number of smaller entries in it.  Writes
+// the row's contacts and partners in order, the contact's two entry positions (where the contact pass writes its
+// shares) and their positions in the rows (which bit of the row's mask it sets).  Threads follow the entries of tmp,
+// so the threads of a warp read the same few rows from L1.
+__global__ void k_csr_rank(Contacts c, long long ne, RowCount R, const unsigned long long* tmp, unsigned* ent,
+                           unsigned* partner) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
-  const unsigned v = vals[e];
-  ent[e] = v;
-  const unsigned ci = v & 0x7fffffffu;
-  const long long k = e - rowptr[keys[e] >> idBits];
-  const unsigned char bit = (unsigned char)(k < 31 ? k : 31);
-  if (v >> 31) { slot[ci].y = (int)e; rowBit[ci].y = bit; }
-  else { slot[ci].x = (int)e; rowBit[ci].x = bit; }
-}
-__global__ void k_csr_rows(const unsigned long long* keys, long long ne, int idBits, int n, int* rowptr) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) {
-    if (ne == 0 && e <= n) rowptr[e] = 0;
-    return;
+  const unsigned long long v = tmp[e];
+  const unsigned val = (unsigned)v, ci = val & 0x7fffffffu;
+  const bool isB = (val >> 31) != 0;
+  const int2 id = c.ids[ci];
+  const int row = isB ? id.y : id.x, other = isB ? id.x : id.y;
+  const unsigned row0 = R.cnt[row], row1 = R.cnt[row + 1];
+  unsigned beg = row0, end = row1;
+  const int k = rangeOf(R, row, other, maybeLarge(c.state[ci]));
+  if (k >= 0) {
+    beg = row0 + R.sub[k];
+    if ((k + 1) % R.V != 0) end = row0 + R.sub[k + 1];
   }
-  long long r = (long long)(keys[e] >> idBits);
-  long long rp = e > 0 ? (long long)(keys[e - 1] >> idBits) : -1;
-  for (long long k = rp + 1; k <= r; k++) rowptr[k] = (int)e;
-  if (e == ne - 1)
-    for (long long k = r + 1; k <= n; k++) rowptr[k] = (int)ne;
+  unsigned pos = beg;
+  for (unsigned q = beg; q < end; q++) pos += tmp[q] < v ? 1u : 0u;
+  ent[pos] = val;
+  partner[pos] = (unsigned)other;
+  const unsigned in = pos - row0;
+  const unsigned char bit = (unsigned char)(in < 31 ? in : 31);
+  if (isB) { c.slot[ci].y = (int)pos; c.rowBit[ci].y = bit; }
+  else { c.slot[ci].x = (int)pos; c.rowBit[ci].x = bit; }
 }
 
 // ------------------------------------------------------------------------------------ periodic grid
@@ -1145,9 +1278,28 @@ void launch_stress(cudaStream_t s, const StepParams& P, Particles p, Contacts c,
   for (int q = 0; q < 9; q++) energy_accumulate(s, scratch9 + (long long)q * nc, nc, partials, out9 + q, true);
 }
 
-long long col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew, Contacts old, Csr oldCsr,
-                            long long step, int nHist, ColliderScratch& cs) {
-  if (nNew <= 0) return 0;
+static RowCount rowCount(int n, const Csr& csr, const ColliderScratch& cs) {
+  RowCount R;
+  R.cnt = reinterpret_cast<unsigned*>(csr.rowptr);
+  R.sub = cs.rowSub;
+  R.largeIdx = cs.largeIdx;
+  largeRanges(n, cs.nLarge, R.V, R.S);
+  return R;
+}
+static void clearRows(cudaStream_t s, int n, const RowCount& R, const ColliderScratch& cs) {
+  cudaMemsetAsync(R.cnt, 0, (size_t)n * sizeof(unsigned), s);
+  if (cs.nLarge > 0) cudaMemsetAsync(R.sub, 0, (size_t)cs.nLarge * R.V * sizeof(unsigned), s);
+}
+
+void col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew, Contacts old, Csr csr, int nRowsOld,
+                       int n, long long step, int nHist, ColliderScratch& cs) {
+  Csr oldCsr = csr;
+  oldCsr.n = nRowsOld;
+  const RowCount R = rowCount(n, csr, cs);
+  if (nNew <= 0) {
+    clearRows(s, n, R, cs);
+    return;
+  }
   unsigned long long* tmpIds = cs.keys;
   unsigned* tmpJ = cs.vals;
   unsigned* flag = cs.valsAlt;
@@ -1155,24 +1307,25 @@ long long col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long
   const unsigned blocks = (unsigned)((nNew + 255) / 256);
   (k_part_flag<<<blocks, 256, 0, s>>>(neu, nNew, old, oldCsr, tmpIds, tmpJ, flag, tmpDist), ++::wdem::g_kernel_launches);
   exclusive_scan_u32(s, flag, nNew, cs);
-  (k_carry_compact<<<blocks, 256, 0, s>>>(p, neu, nNew, old, tmpIds, tmpJ, flag, tmpDist, step, nHist), ++::wdem::g_kernel_launches);
-  return nNew;
+  clearRows(s, n, R, cs);  // the old rows have been read
+  (k_carry_compact<<<blocks, 256, 0, s>>>(p, neu, nNew, old, tmpIds, tmpJ, flag, tmpDist, step, nHist, R), ++::wdem::g_kernel_launches);
 }
 
-void col_csr(cudaStream_t s, Contacts c, long long nc, int n, Csr& csr, ColliderScratch& cs) {
-  int idBits = bitsFor((unsigned long long)n + 1);
-  long long ne = 2 * nc;
-  if (nc > 0) (k_csr_entries<<<(unsigned)((nc + 255) / 256), 256, 0, s>>>(c, nc, idBits, cs.keys, cs.vals), ++::wdem::g_kernel_launches);
-  radix_sort(s, cs.keys, cs.vals, cs.keysAlt, cs.valsAlt, ne, 2 * idBits, cs);
-  // the sorted keys stay with the CSR for the next rebuild's carry (cs.keys is the sort's scratch)
-  if (ne > 0) cudaMemcpyAsync(csr.keys, cs.keys, (size_t)ne * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
-  csr.idBits = idBits;
+// The CSR of the container.  placed: its contacts have taken their places (k_carry_compact).
+void col_csr(cudaStream_t s, Contacts c, long long nc, int n, Csr& csr, ColliderScratch& cs, bool placed) {
+  const RowCount R = rowCount(n, csr, cs);
+  const unsigned blocks = (unsigned)((nc + 255) / 256);
+  if (!placed) {
+    clearRows(s, n, R, cs);
+    if (nc > 0) (k_csr_places<<<blocks, 256, 0, s>>>(c, nc, R), ++::wdem::g_kernel_launches);
+  }
   csr.n = n;
-  long long threads = ne > 0 ? ne : (long long)n + 1;
-  (k_csr_rows<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(cs.keys, ne, idBits, n, csr.rowptr), ++::wdem::g_kernel_launches);
-  if (ne > 0)
-    (k_csr_ent_slots<<<(unsigned)((ne + 255) / 256), 256, 0, s>>>(cs.vals, cs.keys, idBits, csr.rowptr, ne, csr.ent, c.slot, c.rowBit),
-     ++::wdem::g_kernel_launches);
+  if (cs.nLarge > 0) (k_csr_large<<<(unsigned)cs.nLarge, 256, 0, s>>>(cs.large, R), ++::wdem::g_kernel_launches);
+  exclusive_scan_u32(s, R.cnt, n, cs);
+  if (nc <= 0) return;
+  unsigned long long* tmp = cs.keysAlt;
+  (k_csr_fill<<<blocks, 256, 0, s>>>(c, nc, R, tmp), ++::wdem::g_kernel_launches);
+  (k_csr_rank<<<(unsigned)((2 * nc + 255) / 256), 256, 0, s>>>(c, 2 * nc, R, tmp, csr.ent, csr.partner), ++::wdem::g_kernel_launches);
 }
 
 }  // namespace wdem

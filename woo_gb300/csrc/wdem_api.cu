@@ -356,6 +356,19 @@ void collectTimes(wdem_handle* h) {
   h->evUsed = 0;
 }
 
+// scratch for scans of up to n values (cleared: no status word of an earlier scan)
+int ensureScan(wdem_handle* h, long long n) {
+  ColliderScratch& cs = h->cs;
+  if (scan_scratch_words(n) > cs.scanCap) {
+    const long long cap = scan_scratch_words(n + n / 2);
+    CK(dalloc(cs.scanScratch, cap));
+    CK(cudaMemsetAsync(cs.scanScratch, 0, cap * sizeof(unsigned), h->stream));
+    cs.scanCap = cap;
+    cs.scanEpoch = cs.scanTickets = 0;
+  }
+  return WDEM_OK;
+}
+
 // Scratch for the collider sized for nSmall particles and up to nc contacts.
 int ensureScratch(wdem_handle* h, long long nc) {
   ColliderScratch& cs = h->cs;
@@ -387,14 +400,7 @@ int ensureScratch(wdem_handle* h, long long nc) {
     CK(dalloc(cs.retainFlag, cap));
     cs.retainCap = cap;
   }
-  // scan scratch: level sums of the longest scan (histograms, pair counts, retain flags)
-  long long longest = std::max<long long>(std::max<long long>(cs.histCap, (long long)h->N + 2), cs.retainCap);
-  long long needSums = 64 + 2 * (longest / 1024 + 64) + 4096;
-  if (needSums > cs.blockSumsCap) {
-    CK(dalloc(cs.blockSums, needSums));
-    cs.blockSumsCap = needSums;
-  }
-  return WDEM_OK;
+  return ensureScan(h, std::max<long long>(std::max<long long>((long long)h->N + 2, cs.sortCap), cs.retainCap));
 }
 
 // periodic candidate buffers for n candidates (flags scanned in place: n + 1 entries), and the scan
@@ -406,19 +412,14 @@ int ensureCand(wdem_handle* h, long long n) {
     CK(dalloc(cs.cand, cap)); CK(dalloc(cs.candPer, cap)); CK(dalloc(cs.candFlag, cap + 1));
     cs.candCap = cap;
   }
-  long long needSums = 64 + 2 * ((n + 1) / 1024 + 64) + 4096;
-  if (needSums > cs.blockSumsCap) {
-    CK(dalloc(cs.blockSums, needSums));
-    cs.blockSumsCap = needSums;
-  }
-  return WDEM_OK;
+  return ensureScan(h, n + 1);
 }
 
 int ensureCsr(wdem_handle* h, long long nc) {
   if (2 * nc + 1 > h->csrCap) {
     long long cap = std::max<long long>(2 * nc + 1, h->csrCap * 3 / 2);
     CK(dalloc(h->csr.ent, cap));
-    CK(dalloc(h->csr.keys, cap));
+    CK(dalloc(h->csr.partner, cap));
     h->csrCap = cap;
   }
   return WDEM_OK;
@@ -505,15 +506,14 @@ int rebuild(wdem_handle* h) {
   col_retain_write(s, old.c, nOld, cs, neu.c.ids, total, neu.cap);
   if (h->periodic && old.c.cdist) col_retain_write_dist(s, old.c, nOld, cs, neu.c.cdist, total, neu.cap);
   const int side = 1 - h->cur;
-  // history carried over (each new pair found in the old container through the old CSR's sorted keys),
+  // history carried over (each new pair found in the old container through the old CSR's sorted rows),
   // contacts real before the rebuild compacted to the front (the sort scratch, sized for 2 nNew entries,
   // holds the temporaries); then the new container's CSR
   if ((rc = ensureScratch(h, nNew))) return rc;
-  Csr oldCsr = h->csr;
-  if (nOld <= 0) oldCsr.n = 0;
-  col_carry_compact(s, h->d, neu.c, nNew, old.c, oldCsr, h->step, (hertz && old.hertz) ? (int)HIST_COUNT : (int)HIST_FRICT, cs);
+  col_carry_compact(s, h->d, neu.c, nNew, old.c, h->csr, nOld > 0 ? h->csr.n : 0, n, h->step,
+                    (hertz && old.hertz) ? (int)HIST_COUNT : (int)HIST_FRICT, cs);
   if ((rc = ensureCsr(h, nNew))) return rc;
-  col_csr(s, neu.c, nNew, n, h->csr, cs);
+  col_csr(s, neu.c, nNew, n, h->csr, cs, true);
   h->cur = side;
   h->nContacts = nNew;
   h->nFullRuns++;
@@ -693,7 +693,8 @@ int wdem_create(int device, int32_t maxParticles, wdem_handle** out) {
   ok &= dalloc(h->cs.srec, 2 * (size_t)N + 2) == cudaSuccess;
   ok &= dalloc(h->cs.grid, 1) == cudaSuccess;
   ok &= dalloc(h->csr.rowptr, (size_t)N + 1) == cudaSuccess;
-  ok &= dalloc(h->csr.cursor, (size_t)N) == cudaSuccess;
+  ok &= dalloc(h->cs.largeIdx, (size_t)N) == cudaSuccess;
+  ok &= dalloc(h->cs.rowSub, 2 * (size_t)N + 1) == cudaSuccess;
   unsigned long long* tmp = nullptr;
   ok &= dalloc(tmp, 64) == cudaSuccess;
   h->cs.temp = tmp;
@@ -733,10 +734,10 @@ int wdem_destroy(wdem_handle* h) {
   cudaFree(h->dEnergy); cudaFree(h->ePartials); cudaFree(h->dStress); cudaFree(h->stressTerms);
   cudaFree(h->dSmall);
   freeContacts(h->buf[0]); freeContacts(h->buf[1]);
-  cudaFree(h->csr.rowptr); cudaFree(h->csr.ent); cudaFree(h->csr.cursor); cudaFree(h->csr.keys);
+  cudaFree(h->csr.rowptr); cudaFree(h->csr.ent); cudaFree(h->csr.partner);
   ColliderScratch& cs = h->cs;
   cudaFree(cs.keys); cudaFree(cs.keysAlt); cudaFree(cs.vals); cudaFree(cs.valsAlt); cudaFree(cs.hist);
-  cudaFree(cs.blockSums); cudaFree(cs.cellStart); cudaFree(cs.counts); cudaFree(cs.large); cudaFree(cs.grid); cudaFree(cs.srec);
+  cudaFree(cs.scanScratch); cudaFree(cs.largeIdx); cudaFree(cs.rowSub); cudaFree(cs.cellStart); cudaFree(cs.counts); cudaFree(cs.large); cudaFree(cs.grid); cudaFree(cs.srec);
   cudaFree(cs.retainFlag); cudaFree(cs.temp); cudaFree(cs.periC); cudaFree(cs.periH); cudaFree(cs.periCi); cudaFree(cs.periHi);
   cudaFree(cs.cand); cudaFree(cs.candPer); cudaFree(cs.candFlag); cudaFree(cs.sweepBuf);
   cudaFree(h->dst);
@@ -984,6 +985,12 @@ int wdem_upload_particles(wdem_handle* h, const wdem_particles* p) {
   if (!h->largeIds.empty())
     CK(cudaMemcpyAsync(h->cs.large, h->largeIds.data(), h->largeIds.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   h->cs.nLarge = (int)h->largeIds.size();
+  {
+    std::vector<int> largeIdx(h->N, -1);
+    for (size_t k = 0; k < h->largeIds.size(); k++) largeIdx[h->largeIds[k]] = (int)k;
+    CK(cudaMemcpyAsync(h->cs.largeIdx, largeIdx.data(), h->N * sizeof(int), cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));  // the host vector goes out of scope
+  }
   cudaFree(h->cs.sceneWall);
   h->cs.sceneWall = nullptr;
   h->cs.nScenes = nScenes;
@@ -1063,7 +1070,7 @@ int wdem_upload_contacts(wdem_handle* h, const wdem_contacts* c) {
   // the uploaded container's CSR: the next rebuild carries the history of its contacts through it
   if ((rc = ensureScratch(h, nc))) return rc;
   if ((rc = ensureCsr(h, nc))) return rc;
-  col_csr(s, b.c, nc, h->n, h->csr, h->cs);
+  col_csr(s, b.c, nc, h->n, h->csr, h->cs, false);
   CK(cudaStreamSynchronize(s));
   h->nContacts = nc;
   h->needRebuild = true;

@@ -212,10 +212,8 @@ struct Contacts {
 struct Csr {
   int* rowptr;    // N+1
   unsigned* ent;  // 2C
-  int* cursor;    // N (scratch for filling)
-  unsigned long long* keys;  // 2C: the entries' sort keys, row << idBits | partner (the next rebuild's carry
-                             // finds each old contact in them)
-  int idBits;     // bits of a particle id in keys
+  unsigned* partner;  // 2C: the entries' other body, ascending within a row (the next rebuild's carry finds each
+                      // old contact in them)
   int n;          // particles the rows cover (0: no rows)
 };
 
@@ -322,8 +320,11 @@ struct ColliderScratch {
   long long sortCap;                    // capacity of the four sort arrays
   unsigned* hist;                       // radix histograms (+1 for the scan total)
   long long histCap;
-  unsigned* blockSums;                  // scan scratch
-  long long blockSumsCap;
+  unsigned* scanScratch;                // ticket and tile status words of the scans (scan_scratch_words)
+  long long scanCap;
+  unsigned scanEpoch, scanTickets;      // number of the last scan, tickets its predecessors took
+  int* largeIdx;                        // N: index of a body in `large`, -1 for the others
+  unsigned* rowSub;                     // 2N: entry counts of the large bodies' partner ranges (k_csr_large)
   int* cellStart;                       // maxCols + 1
   float4* srec;                         // sweep records in sort order: 2 per particle (N capacity)
   int2* sweepBuf;                       // the counting sweep's first SWEEP_BUF pairs of each thread
@@ -391,11 +392,13 @@ void launch_stress(cudaStream_t s, const StepParams& P, Particles p, Contacts c,
 void col_retain_flags(cudaStream_t s, const StepParams& P, Particles p, Contacts old, long long nOld, ColliderScratch& cs);
 void col_retain_write(cudaStream_t s, Contacts old, long long nOld, ColliderScratch& cs, int2* out, long long base,
                       long long cap);
-void col_csr(cudaStream_t s, Contacts c, long long nc, int n, Csr& csr, ColliderScratch& cs);
-// history carry-over with compaction: contacts that were real before the rebuild first (in emission order),
-// then the others; uses the sort scratch (sized for 2 nNew) as temporary storage
-long long col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew, Contacts old, Csr oldCsr,
-                            long long step, int nHist, ColliderScratch& cs);
+void col_csr(cudaStream_t s, Contacts c, long long nc, int n, Csr& csr, ColliderScratch& cs, bool placed);
+long long scan_scratch_words(long long n);
+// history carry-over with compaction: contacts that were real before the rebuild first (in emission order), then
+// the others, each taking its two places in the new rows of csr (whose nRowsOld old rows are read before); uses the
+// sort scratch (sized for 2 nNew) as temporary storage
+void col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew, Contacts old, Csr csr, int nRowsOld,
+                       int n, long long step, int nHist, ColliderScratch& cs);
 // exclusive scan of a[0..n) in place; a[n] receives the total (the array holds n+1 entries)
 void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs);
 int sort_passes_for(int nSmallBits);
