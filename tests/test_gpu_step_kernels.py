@@ -64,8 +64,8 @@ def test_wall_force_over_long_rows(wdem_lib, m):
 def test_rows_of_walls_at_range_edges(wdem_lib, n):
     """Bodies (with 6 walls) around multiples of 1024, where a wall's row gets another range of partner ids: the
     force sums need every row in the order of the partner ids, the carry finds old contacts in it."""
-    side = 0.011 * np.ceil(n ** (1.0 / 3.0))
-    spec = scenes.random_cloud(n, n, box=(side, side, side), rmin=0.004, rmax=0.005, dense=0.93)
+    side = 0.0125 * np.ceil(n ** (1.0 / 3.0))  # room for the generator to place all n
+    spec = scenes.random_cloud(n, n, box=(side, side, side), rmin=0.004, rmax=0.005, dense=0.8)
     assert spec.particles.n == n + 6
     h, o = _run_both(spec, (1, 4, 40))
     assert h.status().nFullRuns == o.n_full_runs() > 1
@@ -83,3 +83,24 @@ def test_pairs_at_scan_tile_edges(wdem_lib, n):
     want = np.concatenate([np.stack([at[:-d], at[d:]], axis=1) for d in (1, 2) if n > d] + [np.zeros((0, 2), int)])
     want = np.sort(want, axis=1)
     assert np.array_equal(got, want[np.lexsort((want[:, 1], want[:, 0]))])
+
+
+@pytest.mark.parametrize("size, n", [((0.03, 0.06, 0.045), 60), ((0.045, 0.045, 0.045), 70), ((0.1, 0.034, 0.034), 80),
+                                     ((0.055, 0.04, 0.1), 150), ((0.1, 0.1, 0.1), 700)])
+def test_periodic_grids_of_few_cells(wdem_lib, size, n):
+    """Cells of the pair search from 1 to 8 per axis: with fewer than 3 along an axis both neighbours are the same
+    cell and all neighbouring cells are searched by id, otherwise the cells ahead only."""
+    spec = scenes.periodic_cloud(n, 5, size=size, shear=0.15)
+    h, o = _run_both(spec, (1, 15))
+    assert np.array_equal(h.download_contacts().cellDist, o.contacts().cellDist)
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+def test_more_pairs_than_the_sweep_keeps(wdem_lib, periodic):
+    """Large spheres among small ones: bodies with more partners than the counting walk keeps are walked again."""
+    kw = dict(rmin=0.0012, rmax=0.009, dense=0.95, verletDist=0.0015)
+    spec = scenes.periodic_cloud(900, 8, size=(0.07, 0.07, 0.07), **kw) if periodic else scenes.random_cloud(
+        900, 8, box=(0.07, 0.07, 0.07), **kw)
+    h, _ = _run_both(spec, (1, 20))
+    c = h.download_contacts()
+    assert np.bincount(np.concatenate([c.idA, c.idB])).max() > 40

@@ -8,7 +8,7 @@
 // (Collision.cpp:21-43), plus every real contact carried over from before (the reference never
 // removes real contacts in the collider).  Instead of an incremental insertion sort, the rebuild
 //   1. sorts small particles by (grid column in the two long axes, quantised box minimum along the
-//      shortest axis) with an LSD radix sort written here (one kernel per digit, decoupled look-back),
+//      shortest axis): counted into buckets of the key's upper bits, ranked within their buckets,
 //   2. sweeps each particle forward along the sweep axis in its own and the 8 neighbouring columns,
 //      testing the exact FP64 closed-interval overlap (grid cell >= widest box, so no pair is missed),
 //   3. tests walls, facets and other large boxes against every particle of their scene,
@@ -26,7 +26,7 @@
 
 namespace wdem {
 
-// columns of the sweep grid at most (keys of 20 column bits and 12 or more quantisation bits: 4 radix passes)
+// columns of the sweep grid at most (32-bit keys: 20 column bits and 12 quantisation bits)
 static const int SWEEP_MAX_COLS = (1 << 20) - 2;
 
 // ------------------------------------------------------------------------------------------ boxes
@@ -151,45 +151,20 @@ __device__ __forceinline__ double ordVal(unsigned long long k) {
 }
 
 // ext layout (ordered keys): [0..2] min centre, [3..5] max centre (stored as ~key for max via min),
-// [6..8] min box lower bound, [9..11] max box upper bound, [12..14] max box width
-struct ExtAcc { unsigned long long v[15]; };
+// [6..8] min box lower bound, [9..11] max box upper bound, [12..14] max box width; [15] the blocks done
+enum { EXT_WORDS = 16, EXT_VALUES = 15 };
 
-__global__ void k_extents_init(unsigned long long* ext) {
-  int t = threadIdx.x;
-  if (t < 15) ext[t] = ~0ull;  // all stored as "min" accumulators
-}
-
-__global__ void k_extents(Particles p, const int* small, int nSmall, unsigned long long* ext) {
-  __shared__ unsigned long long sh[15];
-  if (threadIdx.x < 15) sh[threadIdx.x] = ~0ull;
-  __syncthreads();
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nSmall) {
-    int i = small[k];
-    double4_32a pr = p.posr[i];
-    double4_32a mn = p.bbmin[i], mx = p.bbmax[i];
-    double c[3] = {pr.x, pr.y, pr.z};
-    double lo[3] = {mn.x, mn.y, mn.z};
-    double hi[3] = {mx.x, mx.y, mx.z};
-    for (int a = 0; a < 3; a++) {
-      atomicMin(&sh[a], ordKey(c[a]));
-      atomicMin(&sh[3 + a], ~ordKey(c[a]));
-      atomicMin(&sh[6 + a], ordKey(lo[a]));
-      atomicMin(&sh[9 + a], ~ordKey(hi[a]));
-      atomicMin(&sh[12 + a], ~ordKey(hi[a] - lo[a]));
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 15) atomicMin(&ext[threadIdx.x], sh[threadIdx.x]);
-}
-
-__global__ void k_grid_setup(const unsigned long long* ext, int nSmall, int maxCols, int qbits, GridParams* g) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ void gridSetup(const unsigned long long* ext, int nSmall, int maxCols, int maxBuckets, int qbits, GridParams* g) {
   GridParams G;
   G.nSmall = nSmall;
   G.qbits = qbits;
   G.qmax = (1u << qbits) - 1;
-  if (nSmall == 0) { G.ok = 0; G.sweepAxis = 0; G.ax1 = 1; G.ax2 = 2; G.ncx = G.ncy = 1; G.lo1 = G.lo2 = 0; G.cell = 1; G.invCell = 1; G.loS = 0; G.invQ = 0; *g = G; return; }
+  if (nSmall == 0) {
+    G.ok = 0; G.sweepAxis = 0; G.ax1 = 1; G.ax2 = 2; G.ncx = G.ncy = 1; G.lo1 = G.lo2 = 0; G.cell = 1; G.invCell = 1;
+    G.loS = 0; G.invQ = 0; G.kbits = 0;
+    *g = G;
+    return;
+  }
   double cmin[3], cmax[3], bmin[3], bmax[3], w[3];
   for (int a = 0; a < 3; a++) {
     cmin[a] = ordVal(ext[a]);
@@ -199,7 +174,7 @@ __global__ void k_grid_setup(const unsigned long long* ext, int nSmall, int maxC
     w[a] = ordVal(~ext[12 + a]);
   }
   // the sweep runs along the shortest extent of the box centres and the columns tile the two longest: the
-  // most columns for the cap, so the fewest boxes per column and the shortest binary searches into them
+  // most columns for the cap, so the fewest boxes per column and the shortest walks into them
   // (a row of batched scenes along one axis would otherwise put all scenes into the same few long columns)
   int ax = 0;
   for (int a = 1; a < 3; a++) if (cmax[a] - cmin[a] < cmax[ax] - cmin[ax]) ax = a;
@@ -225,6 +200,10 @@ __global__ void k_grid_setup(const unsigned long long* ext, int nSmall, int maxC
   G.lo1 = cmin[a1]; G.lo2 = cmin[a2];
   G.ncx = (int)(floor(e1 / cell) + 1);
   G.ncy = (int)(floor(e2 / cell) + 1);
+  // the buckets: each column divided by the upper kbits bits of the quantised lower bound, as many as fit
+  int kb = 0;
+  while (kb < qbits && ((long long)G.ncx * G.ncy) << (kb + 1) <= (long long)maxBuckets) kb++;
+  G.kbits = kb;
   G.loS = bmin[ax];
   double span = bmax[ax] - bmin[ax];
   G.invQ = (span > 0 && span < 1e300) ? (double)(G.qmax - 1) / span : 0.0;
@@ -232,6 +211,90 @@ __global__ void k_grid_setup(const unsigned long long* ext, int nSmall, int maxC
   if (!(G.loS == G.loS)) G.loS = 0.0;
   G.ok = 1;
   *g = G;
+}
+
+// Cells of the periodic box (unsheared coordinates), at least as wide as the widest box per axis, so
+// overlapping periodic images of two boxes lie in neighbouring cells (with wrap-around).  Axes with
+// fewer than 3 cells get one cell.  Candidates are then decided by the exact spatialOverlapPeri.
+struct PeriGrid {
+  int nc[3];
+  double cw[3], invCw[3], invL[3];
+  int ok;
+};
+
+__device__ void gridSetupPeri(const unsigned long long* ext, const StepParams& P, int maxCells, PeriGrid* g) {
+  PeriGrid G;
+  long long tot = 1;
+  for (int k = 0; k < 3; k++) {
+    double W = ordVal(~ext[12 + k]);
+    int n = (W > 0 && W < 1e300) ? (int)floor(P.csize[k] / (W * (1 + 1e-6))) : 1;
+    if (n < 3) n = 1;
+    if (n > 1024) n = 1024;
+    G.nc[k] = n;
+    tot *= n;
+  }
+  while (tot > maxCells) {
+    int kmax = 0;
+    for (int k = 1; k < 3; k++) if (G.nc[k] > G.nc[kmax]) kmax = k;
+    G.nc[kmax] = G.nc[kmax] * 3 / 4;
+    if (G.nc[kmax] < 3) G.nc[kmax] = 1;
+    tot = (long long)G.nc[0] * G.nc[1] * G.nc[2];
+  }
+  for (int k = 0; k < 3; k++) {
+    G.cw[k] = P.csize[k] / G.nc[k];
+    G.invCw[k] = 1.0 / G.cw[k];
+    G.invL[k] = 1.0 / P.csize[k];
+  }
+  G.ok = 1;
+  *g = G;
+}
+
+// Extents of the small bodies, and the grid from them: every thread keeps the minima of its bodies, a warp's are
+// combined by shuffles, the block's in shared memory; the last block to finish sets up the grid (the grid's single
+// thread was a launch of its own, 6 us, and the extents took 15 shared atomics a body).
+struct GridArgs {
+  int maxCols, maxBuckets, qbits;
+  GridParams* grid;  // null: periodic
+  PeriGrid* peri;
+};
+static const int EXT_T = 256;
+__global__ void __launch_bounds__(EXT_T) k_extents(StepParams P, Particles p, const int* small, int nSmall,
+                                                   unsigned long long* ext, GridArgs A) {
+  __shared__ unsigned long long sh[EXT_VALUES];
+  __shared__ bool last;
+  if (threadIdx.x < EXT_VALUES) sh[threadIdx.x] = ~0ull;
+  __syncthreads();
+  unsigned long long v[EXT_VALUES];
+#pragma unroll
+  for (int q = 0; q < EXT_VALUES; q++) v[q] = ~0ull;
+  auto lower = [](unsigned long long& a, unsigned long long b) { if (b < a) a = b; };
+  for (int k = blockIdx.x * EXT_T + threadIdx.x; k < nSmall; k += gridDim.x * EXT_T) {
+    const int i = small[k];
+    const double4_32a pr = p.posr[i], mn = p.bbmin[i], mx = p.bbmax[i];
+    lower(v[0], ordKey(pr.x)); lower(v[1], ordKey(pr.y)); lower(v[2], ordKey(pr.z));
+    lower(v[3], ~ordKey(pr.x)); lower(v[4], ~ordKey(pr.y)); lower(v[5], ~ordKey(pr.z));
+    lower(v[6], ordKey(mn.x)); lower(v[7], ordKey(mn.y)); lower(v[8], ordKey(mn.z));
+    lower(v[9], ~ordKey(mx.x)); lower(v[10], ~ordKey(mx.y)); lower(v[11], ~ordKey(mx.z));
+    lower(v[12], ~ordKey(mx.x - mn.x)); lower(v[13], ~ordKey(mx.y - mn.y)); lower(v[14], ~ordKey(mx.z - mn.z));
+  }
+#pragma unroll
+  for (int q = 0; q < EXT_VALUES; q++) {
+    for (int off = 16; off > 0; off >>= 1) lower(v[q], __shfl_xor_sync(0xffffffffu, v[q], off));
+    if ((threadIdx.x & 31) == 0) atomicMin(&sh[q], v[q]);
+  }
+  __syncthreads();
+  if (threadIdx.x < EXT_VALUES) atomicMin(&ext[threadIdx.x], sh[threadIdx.x]);
+  __threadfence();
+  __syncthreads();
+  // the counter starts at all ones, like the minima
+  if (threadIdx.x == 0) last = (unsigned)(atomicAdd(&ext[EXT_VALUES], 1ull) + 1ull) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  __threadfence();
+  unsigned long long e[EXT_VALUES];
+  for (int q = 0; q < EXT_VALUES; q++) e[q] = *(volatile unsigned long long*)(ext + q);
+  if (A.peri) gridSetupPeri(e, P, A.maxBuckets, A.peri);
+  else gridSetup(e, nSmall, A.maxCols, A.maxBuckets, A.qbits, A.grid);
 }
 
 __device__ __forceinline__ double cmp3(const double4_32a& v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
@@ -254,20 +317,20 @@ __device__ __forceinline__ void columnOf(const double4_32a& pr, const GridParams
   cy = (int)fmin(fmax(t2, 0.0), (double)(G.ncy - 1));
 }
 
-__global__ void k_make_keys(Particles p, const int* small, int nSmall, const GridParams* g,
-                            unsigned long long* keys, unsigned* vals) {
+// sweep key of each small body (column, quantised lower bound) and its place in its bucket
+__global__ void k_make_keys(Particles p, const int* small, int nSmall, const GridParams* g, unsigned* keys, unsigned* place,
+                            unsigned* count) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nSmall) return;
   GridParams G = *g;
   int i = small[k];
   int cx, cy;
   columnOf(p.posr[i], G, cx, cy);
-  unsigned long long col = (unsigned long long)cx + (unsigned long long)G.ncx * cy;
-  unsigned q = quant(cmp3(p.bbmin[i], G.sweepAxis), G);
-  keys[k] = (col << G.qbits) | q;
-  vals[k] = (unsigned)i;
+  const unsigned col = (unsigned)(cx + G.ncx * cy);
+  const unsigned key = (col << G.qbits) | quant(cmp3(p.bbmin[i], G.sweepAxis), G);
+  keys[k] = key;
+  place[k] = atomicAdd(&count[key >> (G.qbits - G.kbits)], 1u);
 }
-
 
 // ------------------------------------------------------------------------------------ scan
 // Exclusive scan of a[0..n) in place, a[n] <- total, in one kernel (decoupled look-back, Merrill & Garland 2016).
@@ -388,201 +451,45 @@ void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratc
   cs.scanTickets += nt;
 }
 
-// ------------------------------------------------------------------------------------ radix sort
-// LSD radix sort, 8-bit digits, keys u64 with u32 payload, one kernel per digit (Merrill & Garland's
-// single-pass prefix scan with decoupled look-back, applied per digit as in "Onesweep", Adinets & Merrill
-// 2022).  Before the passes, one kernel counts the digits of every pass over the whole input (the global
-// digit starts do not depend on the order) and one block scans them.  A pass kernel takes its tile in
-// acquisition order (atomic counter, so every earlier tile is running or done), counts the tile's digits,
-// publishes them (aggregate), looks back over earlier tiles for the digit's exclusive prefix (stopping at
-// the first inclusive prefix), publishes its own inclusive prefix, ranks the tile's keys stably (round,
-// warp, lane order) into shared memory and writes each digit's run contiguously.  Every look-back wait is
-// bounded; a wait that gives up sets WDEM_ERR_TIMEOUT.
-static const int RS_T = 256, RS_R = 8, RS_TILE = RS_T * RS_R;
-static const int RS_MAX_PASSES = 8;
-static const unsigned RS_AGG = 1u << 30, RS_PRE = 2u << 30, RS_VAL = (1u << 30) - 1;
-static const long long RS_SPIN = 1ll << 22;
-
-// global digit counts of all passes: gcount[p][d]
-__global__ void __launch_bounds__(RS_T) k_rs_count(const unsigned long long* keys, long long n, int passes, unsigned* gcount) {
-  __shared__ unsigned h[RS_MAX_PASSES][256];
-  for (int p = 0; p < passes; p++) h[p][threadIdx.x] = 0;
-  __syncthreads();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = keys[i];
-    for (int p = 0; p < passes; p++) atomicAdd(&h[p][(k >> (8 * p)) & 255], 1u);
-  }
-  __syncthreads();
-  for (int p = 0; p < passes; p++)
-    if (h[p][threadIdx.x]) atomicAdd(&gcount[p * 256 + threadIdx.x], h[p][threadIdx.x]);
+// ------------------------------------------------------------------------------------ bucket sort
+// Small bodies in the order of (key, id): each takes a place in the bucket of its key's upper bits (k_make_keys,
+// k_keys_peri), a scan of the buckets' counts gives their starts, the bodies go to their places and are ranked
+// within their buckets, which hold a body or two (sweep keys) or a cell's handful (periodic).  The start of any key
+// is then a table lookup for the sweep.  An LSD radix sort of the keys took 4 passes of 8 bits, each a
+// dependent launch of 10 us at 15k bodies and 25 us at 500k.
+__global__ void k_bucket_place(const int* small, int nSmall, const unsigned* keys, const unsigned* place,
+                               const unsigned* start, const GridParams* g, unsigned long long* tmp) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nSmall) return;
+  const unsigned key = keys[k];
+  const unsigned b = g ? key >> (g->qbits - g->kbits) : key;
+  tmp[start[b] + place[k]] = ((unsigned long long)key << 32) | (unsigned)small[k];
 }
-// exclusive scan of each pass's 256 counts (one block, thread = digit)
-__global__ void __launch_bounds__(RS_T) k_rs_starts(unsigned* gcount, int passes) {
-  __shared__ unsigned s[256];
-  for (int p = 0; p < passes; p++) {
-    const unsigned c = gcount[p * 256 + threadIdx.x];
-    s[threadIdx.x] = c;
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {
-      const unsigned t = threadIdx.x >= off ? s[threadIdx.x - off] : 0;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
-    }
-    gcount[p * 256 + threadIdx.x] = s[threadIdx.x] - c;
-    __syncthreads();
-  }
+__device__ __forceinline__ unsigned rankInBucket(const unsigned long long* tmp, unsigned long long v, unsigned beg, unsigned end) {
+  unsigned pos = beg;
+  for (unsigned q = beg; q < end; q++) pos += tmp[q] < v ? 1u : 0u;
+  return pos;
 }
-
-__global__ void __launch_bounds__(RS_T) k_rs_pass(const unsigned long long* kin, const unsigned* vin, unsigned long long* kout,
-                                                  unsigned* vout, long long n, int shift, const unsigned* digitStart,
-                                                  unsigned* status, unsigned* tileCounter, DeviceStatus* st) {
-  __shared__ unsigned tileS;
-  __shared__ unsigned cnt[256];      // the tile's digit counts
-  __shared__ unsigned lstart[256];   // exclusive prefix of cnt: the digit's run in the tile's staging
-  __shared__ unsigned goff[256];     // the digit's first position in the output
-  __shared__ unsigned runBase[256];
-  __shared__ unsigned wc[RS_T / 32][256];
-  __shared__ unsigned long long skey[RS_TILE];
-  __shared__ unsigned sval[RS_TILE];
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  if (t == 0) tileS = atomicAdd(tileCounter, 1u);
-  cnt[t] = 0;
-  runBase[t] = 0;
-  __syncthreads();
-  const long long tile = tileS;
-  const long long base = tile * RS_TILE;
-  unsigned long long k[RS_R];
-  unsigned v[RS_R];
-#pragma unroll
-  for (int r = 0; r < RS_R; r++) {
-    const long long idx = base + r * RS_T + t;
-    k[r] = idx < n ? kin[idx] : 0;
-    v[r] = idx < n ? vin[idx] : 0;
-    if (idx < n) atomicAdd(&cnt[(k[r] >> shift) & 255], 1u);
-  }
-  __syncthreads();
-  // thread t: digit t.  Aggregate first, then the look-back, then the inclusive prefix.
-  const unsigned c = cnt[t];
-  volatile unsigned* mine = status + tile * 256;
-  unsigned excl = 0;
-  if (tile == 0) {
-    mine[t] = RS_PRE | c;
-  } else {
-    mine[t] = RS_AGG | c;
-    for (long long j = tile - 1; j >= 0; j--) {
-      volatile unsigned* pr = status + j * 256;
-      unsigned w = pr[t];
-      long long it = 0;
-      while ((w & ~RS_VAL) == 0) {
-        if (++it > RS_SPIN) {
-          atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT);
-          w = RS_PRE;
-          break;
-        }
-        __nanosleep(32);
-        w = pr[t];
-      }
-      excl += w & RS_VAL;
-      if ((w & ~RS_VAL) == RS_PRE) break;
-    }
-    mine[t] = RS_PRE | (excl + c);
-  }
-  goff[t] = digitStart[t] + excl;
-  // exclusive scan of the tile's counts: where each digit's run starts in the staging arrays
-  {
-    unsigned* sc = &wc[0][0];  // free until the ranking rounds
-    sc[t] = c;
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {
-      const unsigned u = t >= off ? sc[t - off] : 0;
-      __syncthreads();
-      sc[t] += u;
-      __syncthreads();
-    }
-    lstart[t] = sc[t] - c;
-    __syncthreads();
-  }
-  // stable ranking into the staging arrays: round r, then warp, then lane
-  for (int r = 0; r < RS_R; r++) {
-    for (int w = 0; w < RS_T / 32; w++) wc[w][t] = 0;
-    __syncthreads();
-    const long long idx = base + r * RS_T + t;
-    const bool valid = idx < n;
-    const unsigned d = valid ? (unsigned)((k[r] >> shift) & 255) : 256u + lane;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const unsigned rankInWarp = __popc(peers & ((1u << lane) - 1));
-    if (valid && lane == __ffs(peers) - 1) wc[warp][d] = __popc(peers);
-    __syncthreads();
-    unsigned dsum = 0;
-    for (int w = 0; w < RS_T / 32; w++) { const unsigned cc = wc[w][t]; wc[w][t] = dsum; dsum += cc; }
-    __syncthreads();
-    if (valid) {
-      const unsigned pos = lstart[d] + runBase[d] + wc[warp][d] + rankInWarp;
-      skey[pos] = k[r];
-      sval[pos] = v[r];
-    }
-    __syncthreads();
-    runBase[t] += dsum;
-  }
-  __syncthreads();
-  // each digit's run written contiguously
-  const long long m = n - base < RS_TILE ? n - base : RS_TILE;
-  for (int j = t; j < m; j += RS_T) {
-    const unsigned long long kk = skey[j];
-    const unsigned d = (unsigned)((kk >> shift) & 255);
-    const unsigned pos = goff[d] + (unsigned)j - lstart[d];
-    kout[pos] = kk;
-    vout[pos] = sval[j];
-  }
+// Sweep order, with the sweep records, two float4 per body: the box in FP32 with the minimum rounded down and
+// the maximum rounded up (every pair of FP64 boxes that overlap overlaps in FP32 too, so a pair the FP32
+// test rejects needs no FP64 test), the mask (lo.w) and meta.x with shape and scene (hi.w).  The sweep
+// walks these contiguous records instead of gathering meta, bbmin and bbmax by particle id.
+__global__ void k_bucket_rank(Particles p, int nSmall, const unsigned long long* tmp, const unsigned* start,
+                              const GridParams* g, unsigned* keys, unsigned* vals, float4* rec) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nSmall) return;
+  const unsigned long long v = tmp[e];
+  const unsigned key = (unsigned)(v >> 32);
+  const int i = (int)(unsigned)v;
+  const double4_32a mn = p.bbmin[i], mx = p.bbmax[i];
+  const int4 m = p.meta[i];
+  const unsigned b = key >> (g->qbits - g->kbits);
+  const unsigned s = rankInBucket(tmp, v, start[b], start[b + 1]);
+  keys[s] = key;
+  vals[s] = (unsigned)i;
+  rec[2 * s] = make_float4(__double2float_rd(mn.x), __double2float_rd(mn.y), __double2float_rd(mn.z), __uint_as_float((unsigned)m.z));
+  rec[2 * s + 1] = make_float4(__double2float_ru(mx.x), __double2float_ru(mx.y), __double2float_ru(mx.z), __int_as_float(m.x));
 }
-
-// scratch of one sort: status words of every pass (passes x tiles x 256), then the per-pass tile counters
-// and global digit starts (passes x 256), cleared by one memset
-static void radix_sort(cudaStream_t s, unsigned long long*& keys, unsigned*& vals, unsigned long long*& keysAlt,
-                       unsigned*& valsAlt, long long n, int bits, ColliderScratch& cs) {
-  DeviceStatus* st = cs.st;
-  if (n <= 1) return;
-  const long long nTiles = (n + RS_TILE - 1) / RS_TILE;
-  const int passes = (bits + 7) / 8;
-  unsigned* status = cs.hist;
-  unsigned* starts = status + (size_t)passes * nTiles * 256;
-  unsigned* counters = starts + passes * 256;
-  cudaMemsetAsync(status, 0, ((size_t)passes * nTiles * 256 + passes * 256 + passes) * sizeof(unsigned), s);
-  const unsigned cb = (unsigned)std::min<long long>((n + RS_T - 1) / RS_T, 152 * 8);
-  (k_rs_count<<<cb, RS_T, 0, s>>>(keys, n, passes, starts), ++::wdem::g_kernel_launches);
-  (k_rs_starts<<<1, RS_T, 0, s>>>(starts, passes), ++::wdem::g_kernel_launches);
-  for (int p = 0; p < passes; p++) {
-    (k_rs_pass<<<(unsigned)nTiles, RS_T, 0, s>>>(keys, vals, keysAlt, valsAlt, n, 8 * p, starts + p * 256,
-                                                  status + (size_t)p * nTiles * 256, counters + p, st),
-     ++::wdem::g_kernel_launches);
-    unsigned long long* tk = keys; keys = keysAlt; keysAlt = tk;
-    unsigned* tv = vals; vals = valsAlt; valsAlt = tv;
-  }
-}
-// words of radix-sort scratch for n keys
-long long radix_scratch_words(long long n) {
-  const long long nTiles = (n + RS_TILE - 1) / RS_TILE;
-  return (long long)RS_MAX_PASSES * nTiles * 256 + RS_MAX_PASSES * 257 + 64;
-}
-
-// ------------------------------------------------------------------------------------ sort small
-__global__ void k_cell_start(const unsigned long long* keys, int nSmall, const GridParams* g, int* cellStart) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int ncols = g->ncx * g->ncy;
-  if (nSmall == 0) {
-    for (int k = s; k <= ncols; k += gridDim.x * blockDim.x) cellStart[k] = 0;
-    return;
-  }
-  if (s >= nSmall) return;
-  const int qb = g->qbits;
-  long long c = (long long)(keys[s] >> qb);
-  long long cp = s > 0 ? (long long)(keys[s - 1] >> qb) : -1;
-  for (long long k = cp + 1; k <= c; k++) cellStart[k] = s;
-  if (s == nSmall - 1)
-    for (long long k = c + 1; k <= ncols; k++) cellStart[k] = nSmall;
-}
-
 
 // ------------------------------------------------------------------------------------ sweep
 __device__ __forceinline__ bool overlap3(const double4_32a& mn1, const double4_32a& mx1, const double4_32a& mn2, const double4_32a& mx2) {
@@ -602,34 +509,22 @@ __device__ __forceinline__ int2 orient(int i, int j, int shi, int shj) {
   return make_int2(a, b);
 }
 
-// Sweep records, two float4 per particle in sort order: the box in FP32 with the minimum rounded down and
-// the maximum rounded up (every pair of FP64 boxes that overlap overlaps in FP32 too, so a pair the FP32
-// test rejects needs no FP64 test), the mask (lo.w) and meta.x with shape and scene (hi.w).  The sweep
-// walks these contiguous records instead of gathering meta, bbmin and bbmax by particle id.
-__global__ void k_sweep_records(Particles p, const unsigned* vals, int nSmall, float4* rec) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nSmall) return;
-  const int i = (int)vals[s];
-  const double4_32a mn = p.bbmin[i], mx = p.bbmax[i];
-  const int4 m = p.meta[i];
-  rec[2 * s] = make_float4(__double2float_rd(mn.x), __double2float_rd(mn.y), __double2float_rd(mn.z), __uint_as_float((unsigned)m.z));
-  rec[2 * s + 1] = make_float4(__double2float_ru(mx.x), __double2float_ru(mx.y), __double2float_ru(mx.z), __int_as_float(m.x));
-}
 __device__ __forceinline__ bool overlapF(const float4& mn1, const float4& mx1, const float4& mn2, const float4& mx2) {
   return (mn1.x <= mx2.x) && (mx1.x >= mn2.x) && (mn1.y <= mx2.y) && (mx1.y >= mn2.y) && (mn1.z <= mx2.z) && (mx1.z >= mn2.z);
 }
 
 struct SweepArgs {
   const float4* rec;
-  const unsigned long long* keys;
+  const unsigned* keys;
   const unsigned* vals;
-  const int* cellStart;
+  const unsigned* start;  // first sorted position of each bucket
   const int* large;
   int nLarge;
   int nSmall;
   unsigned loneMask;
   const int* sceneWall;  // per-scene ranges of the large list (null: one scene)
-  int2* buf;             // SWEEP_BUF pairs per thread, written by the counting pass (null: none kept)
+  unsigned* buf;         // SWEEP_BUF partners per thread (thread minor), written by the counting pass: the other
+                         //   body's id, bit 31 when it comes first in the pair (null: none kept)
 };
 
 // The sweep runs twice: counting (WRITE false) and writing at the scanned offsets (WRITE true).  With a
@@ -645,18 +540,24 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
   if (WRITE && A.buf) {
     const unsigned found = counts[s + 1] - counts[s];
     if (found <= (unsigned)SWEEP_BUF) {
-      const int2* b = A.buf + (long long)s * SWEEP_BUF;
-      for (unsigned k = 0; k < found; k++)
-        if (base + k < (unsigned long long)cap) out[base + k] = b[k];
+      const long long T = sweepThreads(A.nSmall, A.nLarge);
+      const int i = s < A.nSmall ? (int)A.vals[s] : A.nLarge > 0 ? A.large[s - A.nSmall] : 0;
+      for (unsigned k = 0; k < found; k++) {
+        const unsigned v = A.buf[k * T + s];
+        const int j = (int)(v & 0x7fffffffu);
+        if (base + k < (unsigned long long)cap) out[base + k] = (v >> 31) ? make_int2(j, i) : make_int2(i, j);
+      }
       return;
     }
   }
-  auto emit = [&](int2 pr) {
+  // the pair of the thread's body i with j, as orient() gives it
+  auto emit = [&](int i, int2 pr) {
     if (WRITE) {
       const unsigned long long o = base + cnt;
       if (o < (unsigned long long)cap) out[o] = pr;
     } else if (A.buf && cnt < (unsigned)SWEEP_BUF) {
-      A.buf[(long long)s * SWEEP_BUF + cnt] = pr;
+      const long long T = sweepThreads(A.nSmall, A.nLarge);
+      A.buf[(long long)cnt * T + s] = pr.x == i ? (unsigned)pr.y : (unsigned)pr.x | 0x80000000u;
     }
     cnt++;
   };
@@ -674,42 +575,45 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
         if (sceneOf(mi.x) != sceneOf(mj.x)) break;
         if (!mayCollide((unsigned)mi.z, (unsigned)mj.z, A.loneMask)) continue;
         if (!overlap3(mn, mx, p.bbmin[j], p.bbmax[j])) continue;
-        emit(orient(i, j, mi.x & 15, mj.x & 15));
+        emit(i, orient(i, j, mi.x & 15, mj.x & 15));
       }
     }
     if (!WRITE) counts[s] = cnt;
     return;
   }
   GridParams G = *g;
-  unsigned long long key = A.keys[s];
+  const unsigned key = A.keys[s];
   int i = (int)A.vals[s];
   int4 mi = p.meta[i];
   double4_32a mn = p.bbmin[i], mx = p.bbmax[i];
   const float4 fmn = A.rec[2 * s], fmx = A.rec[2 * s + 1];
-  unsigned qi = (unsigned)(key & G.qmax);
+  unsigned qi = key & G.qmax;
   unsigned qmax = quant(cmp3(mx, G.sweepAxis), G);
-  long long col = (long long)(key >> G.qbits);
-  int cx = (int)(col % G.ncx), cy = (int)(col / G.ncx);
+  const int col = (int)(key >> G.qbits);
+  const int cx = col % G.ncx, cy = col / G.ncx;
+  const int kshift = G.qbits - G.kbits;
   for (int dy = -1; dy <= 1; dy++) {
     int y = cy + dy;
     if (y < 0 || y >= G.ncy) continue;
     for (int dx = -1; dx <= 1; dx++) {
       int x = cx + dx;
       if (x < 0 || x >= G.ncx) continue;
-      long long c2 = (long long)x + (long long)G.ncx * y;
-      int beg = A.cellStart[c2], end = A.cellStart[c2 + 1];
+      const int c2 = x + G.ncx * y;
+      const int end = (int)A.start[(unsigned)(c2 + 1) << G.kbits];
       int q;
       if (c2 == col) q = s + 1;
       else {
-        unsigned long long target = ((unsigned long long)c2 << G.qbits) | qi;
-        int lo = beg, hi = end;
-        while (lo < hi) { int mid = (lo + hi) >> 1; if (A.keys[mid] < target) lo = mid + 1; else hi = mid; }
-        q = lo;
-        while (q < end && A.keys[q] == target && (int)A.vals[q] < i) q++;
+        // the first box of the column after (key, id): from its bucket's start
+        const unsigned target = ((unsigned)c2 << G.qbits) | qi;
+        q = (int)A.start[target >> kshift];
+        while (q < end) {
+          const unsigned kq = A.keys[q];
+          if (kq > target || (kq == target && (int)A.vals[q] >= i)) break;
+          q++;
+        }
       }
       for (; q < end; q++) {
-        unsigned long long kq = A.keys[q];
-        if ((unsigned)(kq & G.qmax) > qmax) break;
+        if ((A.keys[q] & G.qmax) > qmax) break;
         const float4 gmn = A.rec[2 * q], gmx = A.rec[2 * q + 1];
         const unsigned maskj = __float_as_uint(gmn.w);
         const int metaxj = __float_as_int(gmx.w);
@@ -718,7 +622,7 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
         if (!overlapF(fmn, fmx, gmn, gmx)) continue;
         int j = (int)A.vals[q];
         if (!overlap3(mn, mx, p.bbmin[j], p.bbmax[j])) continue;
-        emit(orient(i, j, mi.x & 15, metaxj & 15));
+        emit(i, orient(i, j, mi.x & 15, metaxj & 15));
       }
     }
   }
@@ -729,7 +633,7 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
     int4 mj = p.meta[j];
     if (!mayCollide((unsigned)mi.z, (unsigned)mj.z, A.loneMask)) continue;
     if (!overlap3(mn, mx, p.bbmin[j], p.bbmax[j])) continue;
-    emit(orient(i, j, mi.x & 15, mj.x & 15));
+    emit(i, orient(i, j, mi.x & 15, mj.x & 15));
   }
   if (!WRITE) counts[s] = cnt;
 }
@@ -747,7 +651,7 @@ __global__ void k_retain_flag(StepParams P, Particles p, Contacts old, long long
     bool ov;
     if (P.periodic) {
       // boxes that overlap on every axis by more than the FP32 margin (both narrow: no ambiguity) overlap
-      // in the exact test too (the FP32 copies of this rebuild, k_peri_sorted)
+      // in the exact test too (the FP32 copies of this rebuild, k_keys_peri)
       const float4 c1 = pci[id.x], h1 = phi[id.x], c2 = pci[id.y], h2 = phi[id.y];
       const float L0 = (float)P.csize[0], L1 = (float)P.csize[1], L2 = (float)P.csize[2];
       if (h1.w == 0.f && h2.w == 0.f && periNear(c1.x, h1.x, c2.x, h2.x, L0, 1.f / L0) &&
@@ -968,180 +872,197 @@ __global__ void k_csr_rank(Contacts c, long long ne, RowCount R, const unsigned 
 }
 
 // ------------------------------------------------------------------------------------ periodic grid
-// Cells of the periodic box (unsheared coordinates), at least as wide as the widest box per axis, so
-// overlapping periodic images of two boxes lie in neighbouring cells (with wrap-around).  Axes with
-// fewer than 3 cells get one cell.  Candidates are then decided by the exact spatialOverlapPeri.
-struct PeriGrid {
-  int nc[3];
-  double cw[3];
-  int ok;
-};
-
-__global__ void k_grid_peri(const unsigned long long* ext, StepParams P, int maxCells, PeriGrid* g) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  PeriGrid G;
-  long long tot = 1;
-  for (int k = 0; k < 3; k++) {
-    double W = ordVal(~ext[12 + k]);
-    int n = (W > 0 && W < 1e300) ? (int)floor(P.csize[k] / (W * (1 + 1e-6))) : 1;
-    if (n < 3) n = 1;
-    if (n > 1024) n = 1024;
-    G.nc[k] = n;
-    tot *= n;
-  }
-  while (tot > maxCells) {
-    int kmax = 0;
-    for (int k = 1; k < 3; k++) if (G.nc[k] > G.nc[kmax]) kmax = k;
-    G.nc[kmax] = G.nc[kmax] * 3 / 4;
-    if (G.nc[kmax] < 3) G.nc[kmax] = 1;
-    tot = (long long)G.nc[0] * G.nc[1] * G.nc[2];
-  }
-  for (int k = 0; k < 3; k++) G.cw[k] = P.csize[k] / G.nc[k];
-  G.ok = 1;
-  *g = G;
-}
-
-__device__ __forceinline__ void periCell(const double4_32a& mn, const double4_32a& mx, const StepParams& P,
-                                         const PeriGrid& G, int* c) {
-  const double ctr[3] = {.5 * (mn.x + mx.x), .5 * (mn.y + mx.y), .5 * (mn.z + mx.z)};
-  for (int k = 0; k < 3; k++) {
-    double w = ctr[k] - floor(ctr[k] / P.csize[k]) * P.csize[k];
-    double v = floor(w / G.cw[k]);
-    c[k] = (int)fmin(fmax(v, 0.0), (double)(G.nc[k] - 1));
-  }
-}
-
-__global__ void k_keys_peri(StepParams P, Particles p, const int* small, int nSmall, const PeriGrid* g,
-                            unsigned long long* keys, unsigned* vals) {
+// Each box's centre wrapped into the cell, in FP32 with its half-widths (pci, phi, by particle id), the number of
+// periods taken off per axis with the mask (wrap), its grid cell and its place in the cell's bucket.  The candidate
+// loop rejects with the FP32 copies the pairs whose minimum-image centre distance exceeds the sum of the
+// half-widths by more than the rounding of these copies on some axis: such boxes are disjoint on that axis for
+// every period shift, so spatialOverlapPeri rejects them too.  Boxes wider than a quarter of the cell skip
+// the filter (there the exact test may find an ambiguous contact, which is an error to report).
+__global__ void k_keys_peri(StepParams P, Particles p, const int* small, int nSmall, const PeriGrid* g, unsigned* keys,
+                            unsigned* place, unsigned* count, float4* pci, float4* phi, int4* wrap) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nSmall) return;
   const PeriGrid G = *g;
   const int i = small[k];
-  int c[3];
-  periCell(p.bbmin[i], p.bbmax[i], P, G, c);
-  keys[k] = ((unsigned long long)c[2] * G.nc[1] + c[1]) * G.nc[0] + c[0];
-  vals[k] = (unsigned)i;
-}
-
-// cellStart[c] = first sorted position of cell c, for the grid's own cells (nc0 nc1 nc2 + 1 entries)
-__global__ void k_cell_start_plain(const unsigned long long* keys, int nSmall, const PeriGrid* g, int* cellStart) {
-  const long long ncells = (long long)g->nc[0] * g->nc[1] * g->nc[2];
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nSmall == 0) {
-    for (long long k = s; k <= ncells; k += (long long)gridDim.x * blockDim.x) cellStart[k] = 0;
-    return;
-  }
-  if (s >= nSmall) return;
-  long long c = (long long)keys[s];
-  long long cp = s > 0 ? (long long)keys[s - 1] : -1;
-  for (long long k = cp + 1; k <= c; k++) cellStart[k] = s;
-  if (s == nSmall - 1)
-    for (long long k = c + 1; k <= ncells; k++) cellStart[k] = nSmall;
-}
-
-// FP32 copies, in cell order, of each box's centre wrapped into the cell and of its half-widths: the
-// candidate loop rejects with them the pairs whose minimum-image centre distance exceeds the sum of
-// the half-widths by more than the rounding of these copies on some axis.  Such boxes are disjoint on
-// that axis for every period shift, so spatialOverlapPeri rejects them too, and it is evaluated (in
-// FP64, as the reference does) only for the survivors.  Boxes wider than a quarter of the cell skip
-// the filter (there the exact test may find an ambiguous contact, which is an error to report).
-__global__ void k_peri_sorted(StepParams P, Particles p, const unsigned* vals, int nSmall, float4* pc, float4* ph,
-                              float4* pci, float4* phi) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nSmall) return;
-  const int i = (int)vals[q];
   const double4_32a mn = p.bbmin[i], mx = p.bbmax[i];
   const double lo[3] = {mn.x, mn.y, mn.z}, hi[3] = {mx.x, mx.y, mx.z};
   float c[3], h[3];
+  int f[3], cell[3];
   bool wide = false;
-  for (int k = 0; k < 3; k++) {
-    const double L = P.csize[k];
-    const double ctr = .5 * (lo[k] + hi[k]), half = .5 * (hi[k] - lo[k]);
-    const double w = ctr - floor(ctr / L) * L;
-    c[k] = (float)w;
-    h[k] = (float)half;
-    wide |= !(half < .25 * L);  // also catches infinite and NaN extents
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const double L = P.csize[a];
+    const double ctr = .5 * (lo[a] + hi[a]), half = .5 * (hi[a] - lo[a]);
+    // a product with the rounded 1 / L may put a centre at a period's edge into the next period: w and the count
+    // of periods agree with each other, which is all that is used
+    const double per = floor(ctr * G.invL[a]);
+    const double w = ctr - per * L;
+    c[a] = (float)w;
+    h[a] = (float)half;
+    // beyond 2^30 periods (also infinite and NaN): the exact test decides
+    wide |= !(half < .25 * L) || !(fabs(per) < 1073741824.0);
+    f[a] = wide ? 0 : (int)per;
+    cell[a] = (int)fmin(fmax(floor(w * G.invCw[a]), 0.0), (double)(G.nc[a] - 1));
   }
-  pc[q] = make_float4(c[0], c[1], c[2], 0.f);
-  ph[q] = make_float4(h[0], h[1], h[2], wide ? 1.f : 0.f);
-  pci[i] = pc[q];
-  phi[i] = ph[q];
+  pci[i] = make_float4(c[0], c[1], c[2], 0.f);
+  phi[i] = make_float4(h[0], h[1], h[2], wide ? 1.f : 0.f);
+  wrap[i] = make_int4(f[0], f[1], f[2], p.meta[i].z);
+  const unsigned key = ((unsigned)cell[2] * G.nc[1] + cell[1]) * G.nc[0] + cell[0];
+  keys[k] = key;
+  place[k] = atomicAdd(&count[key], 1u);
 }
 
+// the bodies in cell order: key, and the FP32 copies with the id in the centre's fourth word
+__global__ void k_bucket_rank_peri(int nSmall, const unsigned long long* tmp, const unsigned* start, unsigned* keys,
+                                   const float4* pci, const float4* phi, float4* pc, float4* ph) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nSmall) return;
+  const unsigned long long v = tmp[e];
+  const unsigned key = (unsigned)(v >> 32);
+  const int i = (int)(unsigned)v;
+  float4 c = pci[i];
+  const float4 h = phi[i];
+  const unsigned s = rankInBucket(tmp, v, start[key], start[key + 1]);
+  keys[s] = key;
+  c.w = __int_as_float(i);
+  pc[s] = c;
+  ph[s] = h;
+}
 
-
-// Candidate pass: thread q takes the q-th box in cell order and runs the FP32 filter against the boxes
-// of the 27 neighbouring cells (wrapped, each cell once) with a larger particle id; it counts (WRITE
-// false) or writes (WRITE true, at its scanned offset) the survivors.  The exact FP64 test runs in a
-// separate dense pass (k_peri_exact): inside this loop the survivors of one warp's 32 boxes differ per
-// lane, and the FP64 test would run with a few lanes at a time.
+// Candidate pass: thread q takes the q-th box in cell order and runs the FP32 filter against the boxes after it in
+// its cell and those of the 13 cells ahead of it (wrapped), so that every pair of cells is seen once; a cell with
+// fewer than 3 cells along some axis meets the same neighbour on both sides, and there the boxes of all (different)
+// neighbouring cells with a larger particle id are tested.  It counts (WRITE false) or writes (WRITE true, at its
+// scanned offset) the survivors; the counting pass keeps each thread's first SWEEP_BUF and the writing pass copies
+// them, walking again only for threads with more (two full walks of all 27 cells took 2 x 280 us at 400k bodies).
+// The exact test runs in a separate dense pass (k_peri_exact): inside this loop the survivors of
+// one warp's 32 boxes differ per lane, and the FP64 test would run with a few lanes at a time.
+struct CandArgs {
+  const unsigned* keys;
+  const float4 *pc, *ph;
+  const unsigned* start;
+  unsigned* buf;  // SWEEP_BUF partners per thread (thread minor), or null
+  int nSmall;
+};
 template <bool WRITE>
-__global__ void k_peri_cand(StepParams P, int nSmall, const PeriGrid* g, const unsigned long long* keys,
-                            const unsigned* vals, const float4* pc, const float4* ph, const int* cellStart,
-                            unsigned* counts, int2* cand, long long cap) {
+__global__ void __launch_bounds__(128) k_peri_cand(StepParams P, CandArgs A, const PeriGrid* g, unsigned* counts, int2* cand,
+                                                   long long cap) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q > nSmall) return;
-  if (q == nSmall) { if (!WRITE) counts[q] = 0; return; }
-  const PeriGrid G = *g;
-  const int i = (int)vals[q];
-  const float4 c1 = pc[q], h1 = ph[q];
-  const float L0 = (float)P.csize[0], L1 = (float)P.csize[1], L2 = (float)P.csize[2];
-  const float iL0 = 1.f / L0, iL1 = 1.f / L1, iL2 = 1.f / L2;
-  const long long key0 = (long long)keys[q];
-  int c[3];
-  c[0] = (int)(key0 % G.nc[0]);
-  c[1] = (int)((key0 / G.nc[0]) % G.nc[1]);
-  c[2] = (int)(key0 / ((long long)G.nc[0] * G.nc[1]));
-  // neighbouring cells per axis, each index once (axes of one or two cells have fewer)
-  int nbr[3][3], nn[3];
-  for (int a = 0; a < 3; a++) {
-    nn[a] = 0;
-    for (int d = -1; d <= 1; d++) {
-      const int v = ((c[a] + d) % G.nc[a] + G.nc[a]) % G.nc[a];
-      bool dup = false;
-      for (int b = 0; b < nn[a]; b++) dup |= (nbr[a][b] == v);
-      if (!dup) nbr[a][nn[a]++] = v;
-    }
-  }
+  if (q > A.nSmall) return;
+  if (q == A.nSmall) { if (!WRITE) counts[q] = 0; return; }
+  const float4 c1 = A.pc[q];
+  const int i = __float_as_int(c1.w);
   unsigned cnt = 0;
   const unsigned long long base = WRITE ? counts[q] : 0;
-  for (int az = 0; az < nn[2]; az++)
-    for (int ay = 0; ay < nn[1]; ay++)
-      for (int ax = 0; ax < nn[0]; ax++) {
-        const long long key = ((long long)nbr[2][az] * G.nc[1] + nbr[1][ay]) * G.nc[0] + nbr[0][ax];
-        const int beg = cellStart[key], end = cellStart[key + 1];
-        for (int q2 = beg; q2 < end; q2++) {
-          const int j = (int)vals[q2];
-          if (j <= i) continue;
-          const float4 h2 = ph[q2];
-          if (h1.w == 0.f && h2.w == 0.f) {
-            const float4 c2 = pc[q2];
-            if (periFar(c1.x, h1.x, c2.x, h2.x, L0, iL0) || periFar(c1.y, h1.y, c2.y, h2.y, L1, iL1) ||
-                periFar(c1.z, h1.z, c2.z, h2.z, L2, iL2))
-              continue;
-          }
-          if (WRITE) {
-            const unsigned long long o = base + cnt;
-            if (o < (unsigned long long)cap) cand[o] = make_int2(i, j);
-          }
-          cnt++;
-        }
+  if (WRITE && A.buf) {
+    const unsigned found = counts[q + 1] - counts[q];
+    if (found <= (unsigned)SWEEP_BUF) {
+      for (unsigned k = 0; k < found; k++) {
+        const int j = (int)A.buf[(long long)k * A.nSmall + q];
+        if (base + k < (unsigned long long)cap) cand[base + k] = make_int2(min(i, j), max(i, j));
       }
+      return;
+    }
+  }
+  const float4 h1 = A.ph[q];
+  const PeriGrid G = *g;
+  const float L0 = (float)P.csize[0], L1 = (float)P.csize[1], L2 = (float)P.csize[2];
+  const float iL0 = 1.f / L0, iL1 = 1.f / L1, iL2 = 1.f / L2;
+  const int key0 = (int)A.keys[q];
+  int c[3];
+  c[0] = key0 % G.nc[0];
+  c[1] = (key0 / G.nc[0]) % G.nc[1];
+  c[2] = key0 / (G.nc[0] * G.nc[1]);
+  auto walk = [&](int beg, int end, bool byId) {
+    for (int q2 = beg; q2 < end; q2++) {
+      const float4 c2 = A.pc[q2];
+      const int j = __float_as_int(c2.w);
+      if (byId && j <= i) continue;
+      const float4 h2 = A.ph[q2];
+      if (h1.w == 0.f && h2.w == 0.f &&
+          (periFar(c1.x, h1.x, c2.x, h2.x, L0, iL0) || periFar(c1.y, h1.y, c2.y, h2.y, L1, iL1) ||
+           periFar(c1.z, h1.z, c2.z, h2.z, L2, iL2)))
+        continue;
+      if (WRITE) {
+        const unsigned long long o = base + cnt;
+        if (o < (unsigned long long)cap) cand[o] = make_int2(min(i, j), max(i, j));
+      } else if (A.buf && cnt < (unsigned)SWEEP_BUF) {
+        A.buf[(long long)cnt * A.nSmall + q] = (unsigned)j;
+      }
+      cnt++;
+    }
+  };
+  if (G.nc[0] >= 3 && G.nc[1] >= 3 && G.nc[2] >= 3) {
+    const int xm = c[0] > 0 ? c[0] - 1 : G.nc[0] - 1, xp = c[0] + 1 < G.nc[0] ? c[0] + 1 : 0;
+    const int ym = c[1] > 0 ? c[1] - 1 : G.nc[1] - 1, yp = c[1] + 1 < G.nc[1] ? c[1] + 1 : 0;
+    const int zp = c[2] + 1 < G.nc[2] ? c[2] + 1 : 0;
+    // the rest of the own cell, and the cell ahead in x: one range unless that cell wraps
+    const int row0 = key0 - c[0];
+    if (xp > c[0]) walk(q + 1, (int)A.start[row0 + xp + 1], false);
+    else {
+      walk(q + 1, (int)A.start[key0 + 1], false);
+      walk((int)A.start[row0 + xp], (int)A.start[row0 + xp + 1], false);
+    }
+    // four whole rows of three cells: (y+1, z) and (y-1 .. y+1, z+1)
+    for (int r = 0; r < 4; r++) {
+      const int y = r == 0 || r == 3 ? yp : (r == 1 ? ym : c[1]), z = r == 0 ? c[2] : zp;
+      const int row = (z * G.nc[1] + y) * G.nc[0];
+      if (xm < c[0] && xp > c[0]) walk((int)A.start[row + xm], (int)A.start[row + xp + 1], false);
+      else {
+        walk((int)A.start[row + xm], (int)A.start[row + xm + 1], false);
+        walk((int)A.start[row + c[0]], (int)A.start[row + c[0] + 1], false);
+        walk((int)A.start[row + xp], (int)A.start[row + xp + 1], false);
+      }
+    }
+  } else {
+    // neighbouring cells per axis, each index once (axes of one cell have one)
+    int nbr[3][3], nn[3];
+    for (int a = 0; a < 3; a++) {
+      nn[a] = 0;
+      for (int d = -1; d <= 1; d++) {
+        const int v = ((c[a] + d) % G.nc[a] + G.nc[a]) % G.nc[a];
+        bool dup = false;
+        for (int b = 0; b < nn[a]; b++) dup |= (nbr[a][b] == v);
+        if (!dup) nbr[a][nn[a]++] = v;
+      }
+    }
+    for (int az = 0; az < nn[2]; az++)
+      for (int ay = 0; ay < nn[1]; ay++)
+        for (int ax = 0; ax < nn[0]; ax++) {
+          const int key = (nbr[2][az] * G.nc[1] + nbr[1][ay]) * G.nc[0] + nbr[0][ax];
+          walk((int)A.start[key], (int)A.start[key + 1], true);
+        }
+  }
   if (!WRITE) counts[q] = cnt;
 }
 
-// Exact pass, one thread per candidate: spatialOverlapPeri (FP64, the reference's operations; an
-// ambiguous contact is an error) and Collider::mayCollide.
-__global__ void k_peri_exact(StepParams P, Particles p, const int2* cand, long long nc, unsigned* flag, int4* per,
-                             DeviceStatus* st) {
+// Exact pass, one thread per candidate: spatialOverlapPeri and Collider::mayCollide.  Boxes that overlap on every
+// axis by more than the FP32 margin for the nearest image (both narrow: no ambiguity) overlap in the reference's
+// test too, whose period is then the one of that image, counted from the wrapped centres; nearly all candidates
+// end there.  The rest (within the margin, or wide) take the reference's FP64 operations, 12 divisions a pair: with
+// those for every candidate this pass took 486 us for the 1.6 M pairs of 400k bodies.
+__global__ void k_peri_exact(StepParams P, Particles p, const int2* cand, long long nc, const float4* pci, const float4* phi,
+                             const int4* wrap, unsigned* flag, int4* per, DeviceStatus* st) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nc) return;
   const int2 ij = cand[k];
+  const float4 c1 = pci[ij.x], h1 = phi[ij.x], c2 = pci[ij.y], h2 = phi[ij.y];
+  const int4 w1 = wrap[ij.x], w2 = wrap[ij.y];
+  const float L0 = (float)P.csize[0], L1 = (float)P.csize[1], L2 = (float)P.csize[2];
+  const float iL0 = 1.f / L0, iL1 = 1.f / L1, iL2 = 1.f / L2;
   int4 pr = make_int4(0, 0, 0, 0);
-  bool amb = false;
-  bool ok = overlapPeri(p.bbmin[ij.x], p.bbmax[ij.x], p.bbmin[ij.y], p.bbmax[ij.y], P.csize, pr, amb);
-  if (amb) { if (atomicCAS(&st->code, 0, WDEM_ERR_TOO_BIG) == 0) st->detail = ij.x; ok = false; }
-  if (ok) ok = mayCollide((unsigned)p.meta[ij.x].z, (unsigned)p.meta[ij.y].z, P.loneMask);
+  bool ok;
+  if (h1.w == 0.f && h2.w == 0.f && periNear(c1.x, h1.x, c2.x, h2.x, L0, iL0) && periNear(c1.y, h1.y, c2.y, h2.y, L1, iL1) &&
+      periNear(c1.z, h1.z, c2.z, h2.z, L2, iL2)) {
+    ok = true;
+    pr = make_int4(w1.x - w2.x - (int)rintf((c2.x - c1.x) * iL0), w1.y - w2.y - (int)rintf((c2.y - c1.y) * iL1),
+                   w1.z - w2.z - (int)rintf((c2.z - c1.z) * iL2), 0);
+  } else {
+    bool amb = false;
+    ok = overlapPeri(p.bbmin[ij.x], p.bbmax[ij.x], p.bbmin[ij.y], p.bbmax[ij.y], P.csize, pr, amb);
+    if (amb) { if (atomicCAS(&st->code, 0, WDEM_ERR_TOO_BIG) == 0) st->detail = ij.x; ok = false; }
+  }
+  if (ok) ok = mayCollide((unsigned)w1.w, (unsigned)w2.w, P.loneMask);
   flag[k] = ok ? 1u : 0u;
   per[k] = pr;
 }
@@ -1184,38 +1105,63 @@ namespace wdem {
 
 
 static int bitsFor(unsigned long long v) { int b = 0; while ((1ull << b) < v) b++; return b < 1 ? 1 : b; }
-// the sweep grid's column cap and the quantisation bits of its keys: column bits + qbits fill 32, 40 or 48
-// bits (4, 5 or 6 radix passes), with at least 12 quantisation bits and at most 24
-static int sweepCols(const ColliderScratch& cs) { return std::min(cs.maxCols, SWEEP_MAX_COLS); }
-static int sweepQbits(const ColliderScratch& cs) {
-  const int cb = bitsFor((unsigned long long)sweepCols(cs) + 1);
-  int total = 32;
-  while (total - cb < 12) total += 8;
-  return std::min(24, total - cb);
+// buckets of the sort: two per body (half a body each on average), at most what cellStart holds
+static int maxBuckets(const ColliderScratch& cs, int nSmall) {
+  return (int)std::min<long long>(cs.maxCols, std::max<long long>(1024, 2ll * nSmall));
+}
+// the sweep grid's column cap and the quantisation bits of its keys: column bits + qbits fit 32 bits, with at
+// least 12 quantisation bits (SWEEP_MAX_COLS) and at most 24
+static int sweepCols(const ColliderScratch& cs, int nSmall) { return std::min(maxBuckets(cs, nSmall), SWEEP_MAX_COLS); }
+static int sweepQbits(const ColliderScratch& cs, int nSmall) {
+  return std::min(24, 32 - bitsFor((unsigned long long)sweepCols(cs, nSmall) + 1));
+}
+// the sort's arrays in the collider's scratch: keys and places by body, (key, id) by bucket, keys and ids in order
+struct SortArrays {
+  unsigned *keyIn, *place, *key, *id, *start;
+  unsigned long long* tmp;
+};
+static SortArrays sortArrays(const ColliderScratch& cs) {
+  SortArrays a;
+  a.keyIn = cs.vals;
+  a.place = cs.valsAlt;
+  a.tmp = cs.keysAlt;
+  a.key = reinterpret_cast<unsigned*>(cs.keys);
+  a.id = a.key + cs.sortCap;
+  a.start = cs.cellStart;
+  return a;
+}
+static void launchExtents(cudaStream_t s, const StepParams& P, Particles p, const int* small, int nSmall,
+                          ColliderScratch& cs, const GridArgs& A) {
+  unsigned long long* ext = (unsigned long long*)cs.temp;
+  cudaMemsetAsync(ext, 0xff, EXT_WORDS * sizeof(unsigned long long), s);
+  const unsigned blocks = (unsigned)std::max(1, std::min((nSmall + EXT_T - 1) / EXT_T, 2 * 152));
+  (k_extents<<<blocks, EXT_T, 0, s>>>(P, p, small, nSmall, ext, A), ++::wdem::g_kernel_launches);
 }
 
 // The collider sub-steps are called from wdem_api.cu through these thin wrappers.
 void col_extents_and_grid(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs) {
-  unsigned long long* ext = (unsigned long long*)cs.temp;
-  (k_extents_init<<<1, 32, 0, s>>>(ext), ++::wdem::g_kernel_launches);
-  if (nSmall > 0) (k_extents<<<(nSmall + 255) / 256, 256, 0, s>>>(p, small, nSmall, ext), ++::wdem::g_kernel_launches);
-  (k_grid_setup<<<1, 1, 0, s>>>(ext, nSmall, sweepCols(cs), sweepQbits(cs), cs.grid), ++::wdem::g_kernel_launches);
+  GridArgs A{sweepCols(cs, nSmall), maxBuckets(cs, nSmall), sweepQbits(cs, nSmall), cs.grid, nullptr};
+  launchExtents(s, StepParams{}, p, small, nSmall, cs, A);
 }
 
 void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs) {
-  if (nSmall > 0) (k_make_keys<<<(nSmall + 255) / 256, 256, 0, s>>>(p, small, nSmall, cs.grid, cs.keys, cs.vals), ++::wdem::g_kernel_launches);
-  int bits = sweepQbits(cs) + bitsFor((unsigned long long)sweepCols(cs) + 1);
-  radix_sort(s, cs.keys, cs.vals, cs.keysAlt, cs.valsAlt, nSmall, bits, cs);
-  int threads = nSmall > 0 ? nSmall : (cs.maxCols + 1);
-  (k_cell_start<<<(threads + 255) / 256, 256, 0, s>>>(cs.keys, nSmall, cs.grid, cs.cellStart), ++::wdem::g_kernel_launches);
-  if (nSmall > 0) (k_sweep_records<<<(nSmall + 255) / 256, 256, 0, s>>>(p, cs.vals, nSmall, cs.srec), ++::wdem::g_kernel_launches);
+  const SortArrays a = sortArrays(cs);
+  const int nb = maxBuckets(cs, nSmall);
+  cudaMemsetAsync(a.start, 0, ((size_t)nb + 1) * sizeof(unsigned), s);
+  if (nSmall <= 0) return;
+  const unsigned blocks = (unsigned)((nSmall + 255) / 256);
+  (k_make_keys<<<blocks, 256, 0, s>>>(p, small, nSmall, cs.grid, a.keyIn, a.place, a.start), ++::wdem::g_kernel_launches);
+  exclusive_scan_u32(s, a.start, nb, cs);
+  (k_bucket_place<<<blocks, 256, 0, s>>>(small, nSmall, a.keyIn, a.place, a.start, cs.grid, a.tmp), ++::wdem::g_kernel_launches);
+  (k_bucket_rank<<<blocks, 256, 0, s>>>(p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec), ++::wdem::g_kernel_launches);
 }
 
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out, long long cap,
                bool write, DeviceStatus* st) {
   SweepArgs A;
   A.rec = cs.srec;
-  A.keys = cs.keys; A.vals = cs.vals; A.cellStart = cs.cellStart; A.large = cs.large; A.nLarge = cs.nLarge;
+  const SortArrays a = sortArrays(cs);
+  A.keys = a.key; A.vals = a.id; A.start = a.start; A.large = cs.large; A.nLarge = cs.nLarge;
   A.nSmall = nSmall; A.loneMask = loneMask;
   A.sceneWall = cs.nScenes > 1 ? cs.sceneWall : nullptr;
   A.buf = cs.sweepBufCap >= sweepThreads(nSmall, cs.nLarge) ? cs.sweepBuf : nullptr;
@@ -1242,28 +1188,34 @@ void col_retain_write(cudaStream_t s, Contacts old, long long nOld, ColliderScra
 void col_periodic_cand(cudaStream_t s, const StepParams& P, Particles p, const int* small, int nSmall,
                        ColliderScratch& cs, bool write) {
   PeriGrid* g = (PeriGrid*)((char*)cs.temp + 256);
+  const SortArrays a = sortArrays(cs);
   const int threads = nSmall + 1;
+  CandArgs A{a.key, cs.periC, cs.periH, a.start, cs.sweepBufCap >= nSmall ? cs.sweepBuf : nullptr, nSmall};
   if (!write) {
-    unsigned long long* ext = (unsigned long long*)cs.temp;
-    (k_extents_init<<<1, 32, 0, s>>>(ext), ++::wdem::g_kernel_launches);
-    if (nSmall > 0) (k_extents<<<(nSmall + 255) / 256, 256, 0, s>>>(p, small, nSmall, ext), ++::wdem::g_kernel_launches);
-    (k_grid_peri<<<1, 1, 0, s>>>(ext, P, cs.maxCols, g), ++::wdem::g_kernel_launches);
-    if (nSmall > 0) (k_keys_peri<<<(nSmall + 255) / 256, 256, 0, s>>>(P, p, small, nSmall, g, cs.keys, cs.vals), ++::wdem::g_kernel_launches);
-    radix_sort(s, cs.keys, cs.vals, cs.keysAlt, cs.valsAlt, nSmall, bitsFor((unsigned long long)cs.maxCols + 1), cs);
-    int t = nSmall > 0 ? nSmall : (cs.maxCols + 1);
-    (k_cell_start_plain<<<(t + 255) / 256, 256, 0, s>>>(cs.keys, nSmall, g, cs.cellStart), ++::wdem::g_kernel_launches);
-    if (nSmall > 0) (k_peri_sorted<<<(nSmall + 255) / 256, 256, 0, s>>>(P, p, cs.vals, nSmall, cs.periC, cs.periH, cs.periCi, cs.periHi), ++::wdem::g_kernel_launches);
-    (k_peri_cand<false><<<(threads + 127) / 128, 128, 0, s>>>(P, nSmall, g, cs.keys, cs.vals, cs.periC, cs.periH, cs.cellStart, cs.counts, nullptr, 0), ++::wdem::g_kernel_launches);
+    const int nb = maxBuckets(cs, nSmall);
+    GridArgs GA{0, nb, 0, nullptr, g};
+    launchExtents(s, P, p, small, nSmall, cs, GA);
+    cudaMemsetAsync(a.start, 0, ((size_t)nb + 1) * sizeof(unsigned), s);
+    if (nSmall > 0) {
+      const unsigned blocks = (unsigned)((nSmall + 255) / 256);
+      (k_keys_peri<<<blocks, 256, 0, s>>>(P, p, small, nSmall, g, a.keyIn, a.place, a.start, cs.periCi, cs.periHi, cs.periWrap),
+       ++::wdem::g_kernel_launches);
+      exclusive_scan_u32(s, a.start, nb, cs);
+      (k_bucket_place<<<blocks, 256, 0, s>>>(small, nSmall, a.keyIn, a.place, a.start, nullptr, a.tmp), ++::wdem::g_kernel_launches);
+      (k_bucket_rank_peri<<<blocks, 256, 0, s>>>(nSmall, a.tmp, a.start, a.key, cs.periCi, cs.periHi, cs.periC, cs.periH),
+       ++::wdem::g_kernel_launches);
+    }
+    (k_peri_cand<false><<<(threads + 127) / 128, 128, 0, s>>>(P, A, g, cs.counts, nullptr, 0), ++::wdem::g_kernel_launches);
     exclusive_scan_u32(s, cs.counts, nSmall + 1, cs);
   } else {
-    (k_peri_cand<true><<<(threads + 127) / 128, 128, 0, s>>>(P, nSmall, g, cs.keys, cs.vals, cs.periC, cs.periH, cs.cellStart, cs.counts, cs.cand, cs.candCap), ++::wdem::g_kernel_launches);
+    (k_peri_cand<true><<<(threads + 127) / 128, 128, 0, s>>>(P, A, g, cs.counts, cs.cand, cs.candCap), ++::wdem::g_kernel_launches);
   }
 }
 
 // part 2: the exact test of nCand candidates; flags scanned, accepted total at candFlag[nCand]
 void col_periodic_exact(cudaStream_t s, const StepParams& P, Particles p, ColliderScratch& cs, long long nCand,
                         DeviceStatus* st) {
-  if (nCand > 0) (k_peri_exact<<<(unsigned)((nCand + 255) / 256), 256, 0, s>>>(P, p, cs.cand, nCand, cs.candFlag, cs.candPer, st), ++::wdem::g_kernel_launches);
+  if (nCand > 0) (k_peri_exact<<<(unsigned)((nCand + 255) / 256), 256, 0, s>>>(P, p, cs.cand, nCand, cs.periCi, cs.periHi, cs.periWrap, cs.candFlag, cs.candPer, st), ++::wdem::g_kernel_launches);
   exclusive_scan_u32(s, cs.candFlag, nCand, cs);
 }
 

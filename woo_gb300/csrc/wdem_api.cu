@@ -5,8 +5,8 @@
 // (src/core/Scene.cpp:420-427):
 //   1. k_leapfrog      forces gathered through the contact CSR, integration, verlet trigger
 //   2. collider        only when a particle left its verlet box (or after an upload): boxes, grid,
-//                      radix sort, sweep, contact history carried over through the old CSR's
-//                      sorted keys, real contacts compacted to the front, CSR
+//                      bucket sort, sweep, contact history carried over through the old CSR's
+//                      sorted rows, real contacts compacted to the front, CSR
 //   3. k_contacts      fused Cg2 + Cp2 + Law2 over the contact list
 #include "wdem_internal.h"
 #include "../../include/wdem.h"
@@ -378,18 +378,17 @@ int ensureScratch(wdem_handle* h, long long nc) {
     CK(dalloc(cs.keys, cap)); CK(dalloc(cs.keysAlt, cap));
     CK(dalloc(cs.vals, cap)); CK(dalloc(cs.valsAlt, cap));
     cs.sortCap = cap;
-    cs.histCap = radix_scratch_words(cap);
-    CK(dalloc(cs.hist, cs.histCap));
   }
   if (h->periodic && (long long)h->smallIds.size() + 1 > cs.periCap) {
     long long cap = (long long)h->smallIds.size() + 1;
     CK(dalloc(cs.periC, cap)); CK(dalloc(cs.periH, cap));
     CK(dalloc(cs.periCi, (size_t)h->N + 1)); CK(dalloc(cs.periHi, (size_t)h->N + 1));
+    CK(dalloc(cs.periWrap, (size_t)h->N + 1));
     cs.periCap = cap;
   }
-  // the counting sweep's pair buffer (not used by the periodic collider)
+  // the counting sweep's partner buffer
   const long long nSweepT = sweepThreads((int)h->smallIds.size(), cs.nLarge);
-  if (!h->periodic && nSweepT > cs.sweepBufCap) {
+  if (nSweepT > cs.sweepBufCap) {
     const long long cap = std::max<long long>(nSweepT, cs.sweepBufCap * 5 / 4);
     CK(dalloc(cs.sweepBuf, (size_t)cap * SWEEP_BUF));
     cs.sweepBufCap = cap;
@@ -400,7 +399,8 @@ int ensureScratch(wdem_handle* h, long long nc) {
     CK(dalloc(cs.retainFlag, cap));
     cs.retainCap = cap;
   }
-  return ensureScan(h, std::max<long long>(std::max<long long>((long long)h->N + 2, cs.sortCap), cs.retainCap));
+  // scans of the pair counts and rows, the buckets, the carry and retain flags
+  return ensureScan(h, std::max<long long>(std::max<long long>((long long)h->N + 2, cs.maxCols), std::max<long long>(cs.sortCap, cs.retainCap)));
 }
 
 // periodic candidate buffers for n candidates (flags scanned in place: n + 1 entries), and the scan
@@ -736,9 +736,9 @@ int wdem_destroy(wdem_handle* h) {
   freeContacts(h->buf[0]); freeContacts(h->buf[1]);
   cudaFree(h->csr.rowptr); cudaFree(h->csr.ent); cudaFree(h->csr.partner);
   ColliderScratch& cs = h->cs;
-  cudaFree(cs.keys); cudaFree(cs.keysAlt); cudaFree(cs.vals); cudaFree(cs.valsAlt); cudaFree(cs.hist);
+  cudaFree(cs.keys); cudaFree(cs.keysAlt); cudaFree(cs.vals); cudaFree(cs.valsAlt);
   cudaFree(cs.scanScratch); cudaFree(cs.largeIdx); cudaFree(cs.rowSub); cudaFree(cs.cellStart); cudaFree(cs.counts); cudaFree(cs.large); cudaFree(cs.grid); cudaFree(cs.srec);
-  cudaFree(cs.retainFlag); cudaFree(cs.temp); cudaFree(cs.periC); cudaFree(cs.periH); cudaFree(cs.periCi); cudaFree(cs.periHi);
+  cudaFree(cs.retainFlag); cudaFree(cs.temp); cudaFree(cs.periC); cudaFree(cs.periH); cudaFree(cs.periCi); cudaFree(cs.periHi); cudaFree(cs.periWrap);
   cudaFree(cs.cand); cudaFree(cs.candPer); cudaFree(cs.candFlag); cudaFree(cs.sweepBuf);
   cudaFree(h->dst);
   cudaFree(h->staging);

@@ -57,7 +57,7 @@ __host__ __device__ __forceinline__ int sceneOf(int metax) { return (metax >> ME
 // one); the exclusive scan of the counts leaves the pair total at counts[sweepThreads]
 __host__ __device__ __forceinline__ int sweepThreads(int nSmall, int nLarge) { return nSmall + (nLarge > 0 ? nLarge : 1); }
 // pairs of one sweep thread kept by the counting pass for the writing pass (a thread with more walks again)
-constexpr int SWEEP_BUF = 8;
+constexpr int SWEEP_BUF = 16;
 // Pair orientation as the geometry functors take it (GeomDispatcher::getFunctor2D swaps a fresh contact,
 // ContactLoop.cpp:144-150): the pair (lower id, higher id) is swapped when its shapes come in the order
 // Sphere+Wall, Ellipsoid+Sphere, Ellipsoid+Wall or Sphere+Facet.
@@ -224,8 +224,9 @@ struct GridParams {
   double lo1, lo2, cell;
   double loS, invQ;  // quantisation along the sweep axis
   double invCell;    // 1 / cell (column binning)
-  int qbits;         // sweep key: column << qbits | quantised lower bound (qbits chosen by the host so that the
-  unsigned qmax;     //   whole key fits the fewest 8-bit radix passes), qmax = 2^qbits - 1
+  int qbits;         // sweep key: column << qbits | quantised lower bound (32 bits), qmax = 2^qbits - 1
+  unsigned qmax;
+  int kbits;         // bucket of a key: its column and the upper kbits bits of its quantised lower bound
   int nSmall;        // spheres in the sort
   int ok;
 };
@@ -315,19 +316,17 @@ void launch_contacts(cudaStream_t s, const StepParams& P, Particles p, Contacts 
 void launch_init_uploaded(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc);
 // ---- collider (k_collider.cu) ----
 struct ColliderScratch {
-  unsigned long long *keys, *keysAlt;   // sort keys (particles, then CSR entries)
-  unsigned *vals, *valsAlt;             // sort payloads
+  unsigned long long *keys, *keysAlt;   // sorts of the bodies, the history carry and the CSR entries
+  unsigned *vals, *valsAlt;
   long long sortCap;                    // capacity of the four sort arrays
-  unsigned* hist;                       // radix histograms (+1 for the scan total)
-  long long histCap;
   unsigned* scanScratch;                // ticket and tile status words of the scans (scan_scratch_words)
   long long scanCap;
   unsigned scanEpoch, scanTickets;      // number of the last scan, tickets its predecessors took
   int* largeIdx;                        // N: index of a body in `large`, -1 for the others
   unsigned* rowSub;                     // 2N: entry counts of the large bodies' partner ranges (k_csr_large)
-  int* cellStart;                       // maxCols + 1
+  unsigned* cellStart;                  // first sorted body of each bucket (maxCols + 1; 16-byte aligned)
   float4* srec;                         // sweep records in sort order: 2 per particle (N capacity)
-  int2* sweepBuf;                       // the counting sweep's first SWEEP_BUF pairs of each thread
+  unsigned* sweepBuf;                   // the counting sweep's first SWEEP_BUF partners of each thread
   long long sweepBufCap;                //   (threads)
   int maxCols;
   unsigned* counts;                     // nSmall+2 pair counts per sorted particle, scanned in place
@@ -340,6 +339,7 @@ struct ColliderScratch {
   long long retainCap;
   float4 *periC, *periH;                // periodic: wrapped FP32 box centres / half-widths in cell order
   float4 *periCi, *periHi;              //   the same by particle id
+  int4* periWrap;                       //   periods taken off the centre per axis, mask, by particle id
   long long periCap;
   int2* cand;                           // periodic: FP32 candidate pairs, their exact-test flags
   int4* candPer;                        //   (scanned in place) and cellDist
@@ -352,7 +352,6 @@ struct ColliderScratch {
 void launch_bboxes(cudaStream_t s, const StepParams& P, Particles p, int n);
 void col_extents_and_grid(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs);
 void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs);
-long long radix_scratch_words(long long n);  // radix-sort scratch (cs.hist) for n keys
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out,
                long long cap, bool write, DeviceStatus* st);
 // periodic collider: 3-D cell grid, FP32 candidates, exact spatialOverlapPeri, emission
@@ -401,7 +400,6 @@ void col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew
                        int n, long long step, int nHist, ColliderScratch& cs);
 // exclusive scan of a[0..n) in place; a[n] receives the total (the array holds n+1 entries)
 void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs);
-int sort_passes_for(int nSmallBits);
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
