@@ -80,8 +80,10 @@ __device__ __forceinline__ void cp2(const StepParams& P, int matA, int matB, dou
 // into the FMA of the sum that follows
 #ifdef WDEM_FMA
 #define HALF(x) (0.5 * (x))
+#define SQRT(x) sqrtRefined(x)
 #else
 #define HALF(x) halfOf(x)
+#define SQRT(x) sqrt(x)
 #endif
 
 // HertzPhys.alpha = mean of the materials' alpha (Hertz.cpp:52) is 0: the noAttraction clamp applies.  When no
@@ -126,8 +128,8 @@ __device__ __noinline__ bool ellPairGeometry(const StepParams& P, const Particle
   ob.w = OB.x; ob.x = OB.y; ob.y = OB.z; ob.z = OB.w;
   const d3 semiA = xyz(SA), semiB = xyz(SB);
   const d3 R = pos2 - pos1;
-  const s33 Ai = symInv(shapeMatrix(oa, semiA));
-  const s33 Bi = symInv(shapeMatrix(ob, semiB));
+  const s33 Ai = invShapeMatrix(oa, semiA);
+  const s33 Bi = invShapeMatrix(ob, semiB);
   double L, Fab;
   unsigned iters = 0, fallback = 0;
   if (P.ellSolver == WDEM_ELL_BRENT) {
@@ -750,9 +752,15 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
         double maxFt = fabs(fx) * tanPhi;
         double ftSq = fy * fy + fz * fz;
         if (ftSq > maxFt * maxFt && !P.noSlip) {
+#ifdef WDEM_FMA
+          const double rn = rsqrtFast(ftSq);
+          double FtNorm = ftSq * rn;
+          double ratio = maxFt * rn;
+#else
           double FtNorm = sqrt(ftSq);
           double ratio = maxFt / FtNorm;
-          if (zeroBits(FtNorm)) ratio = 0.;
+#endif
+          if (zeroBits(ftSq)) FtNorm = ratio = 0.;
           if (P.trackEnergy) ePl = (kt != 0. ? (maxFt) * (FtNorm - maxFt) / kt : 0.);
           fy *= ratio; fz *= ratio;
         }
@@ -796,11 +804,11 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
       // one square root of the overlap for kn, Fne and kt, and its square root for the viscous coefficient (the
       // reference's sqrt(-uN), sqrt(max(-uN, 0)) and sqrt(uN < 0 ? -uN : 0) are the same number for uN < 0, and
       // differ for uN = 0 only in the last one's +0)
-      const double sq = sqrt(-uN);
+      const double sq = SQRT(-uN);
       kn = (3 / 2.) * kn0 * sq;
       double Fne = -kn0 * pown3(sq);
       double Fna = hz[3];
-      double eta = (positiveBits(hz[2]) ? hz[2] * sqrt(sq) : 0.);
+      double eta = (positiveBits(hz[2]) ? hz[2] * SQRT(sq) : 0.);
       double Fnv = eta * velN;
       if (P.noAttraction && hertzAlphaZero(P, p, a, b) && positiveBits(Fne + Fnv)) Fnv = -Fne;
       fx = Fne + Fna + Fnv;
@@ -812,8 +820,13 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
       double maxFt = fabs(dmin(0., fx) * tanPhi);
       double ftSq = fy * fy + fz * fz;
       if (ftSq > maxFt * maxFt) {
+#ifdef WDEM_FMA
+        const double rn = rsqrtFast(ftSq);  // ftSq > 0 here
+        const double FtNorm = ftSq * rn, ratio = maxFt * rn;
+#else
         double FtNorm = sqrt(ftSq);
         double ratio = maxFt / FtNorm;
+#endif
         if (P.trackEnergy) ePl = (.5 * (FtNorm - maxFt) + maxFt) * (FtNorm - maxFt) / kt;
         fy *= ratio; fz *= ratio;
       } else {

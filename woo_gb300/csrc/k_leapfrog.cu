@@ -386,7 +386,7 @@ __device__ __forceinline__ void rotateSphere(const StepParams& P, const Particle
   const double w2 = sqnorm(angVel);
   const double h2 = 0.25 * (w2 * (dt * dt));
   qd q;
-  if (h2 < 1e-6) {
+  if (belowHi(h2, 1e-6)) {
     const double f = (0.5 * dt) * (1.0 - h2 * (1.0 / 6.0) * (1.0 - h2 * 0.05));
     q.w = 1.0 - h2 * 0.5 * (1.0 - h2 * (1.0 / 12.0));
     q.x = angVel.x * f; q.y = angVel.y * f; q.z = angVel.z * f;
@@ -403,7 +403,7 @@ __device__ __forceinline__ void rotateSphere(const StepParams& P, const Particle
   if (!isOneBits(z2)) {
     double rn;
     const double e = z2 - 1.0;
-    if (fabs(e) < 1e-6) rn = 1.0 - e * (0.5 - 0.375 * e);
+    if (belowHi(e, 1e-6)) rn = 1.0 - e * (0.5 - 0.375 * e);
     else {
       WDEM_REAL_BRANCH();
       rn = z2 > 0 ? 1.0 / sqrt(z2) : 1.0;

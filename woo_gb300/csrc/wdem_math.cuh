@@ -20,31 +20,6 @@ struct d3 { double x, y, z; };
 
 __device__ __forceinline__ d3 mk(double x, double y, double z) { d3 r; r.x = x; r.y = y; r.z = z; return r; }
 __device__ __forceinline__ d3 xyz(const double4_32a& v) { return mk(v.x, v.y, v.z); }
-__device__ __forceinline__ d3 operator+(d3 a, d3 b) { return mk(a.x + b.x, a.y + b.y, a.z + b.z); }
-__device__ __forceinline__ d3 operator-(d3 a, d3 b) { return mk(a.x - b.x, a.y - b.y, a.z - b.z); }
-__device__ __forceinline__ d3 operator-(d3 a) { return mk(-a.x, -a.y, -a.z); }
-__device__ __forceinline__ d3 operator*(d3 a, double s) { return mk(a.x * s, a.y * s, a.z * s); }
-__device__ __forceinline__ d3 operator*(double s, d3 a) { return mk(s * a.x, s * a.y, s * a.z); }
-#ifdef WDEM_FMA
-__device__ __forceinline__ d3 operator/(d3 a, double s) { const double r = 1.0 / s; return mk(a.x * r, a.y * r, a.z * r); }
-#else
-__device__ __forceinline__ d3 operator/(d3 a, double s) { return mk(a.x / s, a.y / s, a.z / s); }
-#endif
-__device__ __forceinline__ double dot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ double sqnorm(d3 a) { return a.x * a.x + a.y * a.y + a.z * a.z; }
-// sqnorm with every operation rounded on its own in both variants (never contracted): the contracted
-// variant keeps the sphere distance, the near-cancelling overlap |d| - r1 - r2 and the position update
-// identical to the exact variant, so that contact forces agree to rounding after a step from one state
-__device__ __forceinline__ double sqnormExact(d3 a) {
-  return __dadd_rn(__dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)), __dmul_rn(a.z, a.z));
-}
-// v + a s, never contracted (the position update pos + vel dt)
-__device__ __forceinline__ double addMulExact(double v, double a, double s) { return __dadd_rn(v, __dmul_rn(a, s)); }
-__device__ __forceinline__ d3 cross(d3 a, d3 b) {
-  return mk(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
-__device__ __forceinline__ bool isZero(d3 a) { return a.x == 0 && a.y == 0 && a.z == 0; }
-
 // Predicates on the bit patterns, evaluated on the integer pipe instead of FP64 compares (the FP64
 // pipe is the binding unit of these kernels on GB300).  Each equals its FP64 counterpart exactly.  The
 // two 32-bit halves come out of an asm move, which the compiler cannot see through: a 64-bit bit test
@@ -64,6 +39,95 @@ __device__ __forceinline__ unsigned long long bitsOf(double x) {
   const Halves h = halvesOf(x);
   return ((unsigned long long)h.hi << 32) | h.lo;
 }
+
+#ifdef WDEM_FMA
+// Reciprocal, reciprocal square root and square root of the contracted variant: the FP32 unit's approximation of
+// the significand (PTX rcp.approx / rsqrt.approx, error about 2^-22) is the seed, its exponent set on the integer
+// pipe, and one step of third order in FP64 brings the error below the last rounding: with e = 1 - x y,
+// 1/x = y (1 + e + e^2 + O(e^3)); with e = 1 - x y^2, 1/sqrt(x) = y (1 + e/2 + 3 e^2/8 + O(e^3)) (the binomial
+// series).  3 and 5 FP64 instructions where the compiler's division takes about 8 and rsqrt() 8; the contact law
+// has nine of them.  sqrtRefined ends with s + (x - s^2) / (2 s), the residual exact by FMA (Markstein 1990), 7
+// instructions, correct but for rare last-bit ties.  Zeros, subnormals, infinities, NaN and exponents whose seed
+// would leave the normal range take the IEEE operation.
+__device__ __forceinline__ float significandF(Halves h) { return __uint_as_float(0x3f800000u | ((h.hi & 0xfffffu) << 3) | (h.lo >> 29)); }
+// y * 2^k for y in (0.25, 2] as a double, on the integer pipe (exact)
+__device__ __forceinline__ double scaledSeed(float y, int k, unsigned sign) {
+  const unsigned u = __float_as_uint(y);
+  return fromHalves(u << 29, sign | ((((u >> 23) + 896u + (unsigned)k) << 20) | ((u & 0x7fffffu) >> 3)));
+}
+__device__ __forceinline__ double recipFast(double x) {
+  const Halves h = halvesOf(x);
+  const int e = (int)((h.hi >> 20) & 0x7ff);
+  if (e < 4 || e > 2040) {
+    WDEM_REAL_BRANCH();
+    return 1.0 / x;
+  }
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(significandF(h)));
+  const double y = scaledSeed(r, 1023 - e, h.hi & 0x80000000u);
+  const double d = __fma_rn(-x, y, 1.0);
+  return __fma_rn(__fma_rn(d, d, d), y, y);
+}
+// seed of 1/sqrt(x), x positive and normal: false when x is not
+__device__ __forceinline__ bool rsqrtSeed(double x, double& y) {
+  const Halves h = halvesOf(x);
+  const int e = (int)(h.hi >> 20);  // with the sign: negative numbers are above 2047
+  if (e < 4 || e > 2040) return false;
+  const int odd = (e - 1023) & 1;
+  float r;
+  const float m = significandF(h);
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(odd ? 2.f * m : m));
+  y = scaledSeed(r, -((e - 1023 - odd) / 2), 0u);
+  return true;
+}
+__device__ __forceinline__ double rsqrtFast(double x) {
+  double y;
+  if (!rsqrtSeed(x, y)) {
+    WDEM_REAL_BRANCH();
+    return rsqrt(x);
+  }
+  const double d = __fma_rn(-(x * y), y, 1.0);
+  return __fma_rn(y * d, __fma_rn(0.375, d, 0.5), y);
+}
+__device__ __forceinline__ double sqrtRefined(double x) {
+  double y;
+  if (!rsqrtSeed(x, y)) {
+    WDEM_REAL_BRANCH();
+    return sqrt(x);
+  }
+  const double s0 = x * y;
+  const double d = __fma_rn(-s0, y, 1.0);
+  const double s = __fma_rn(s0 * d, __fma_rn(0.375, d, 0.5), s0);
+  const Halves hy = halvesOf(y);  // y / 2
+  return __fma_rn(__fma_rn(-s, s, x), fromHalves(hy.lo, hy.hi - 0x00100000u), s);
+}
+#endif
+
+__device__ __forceinline__ d3 operator+(d3 a, d3 b) { return mk(a.x + b.x, a.y + b.y, a.z + b.z); }
+__device__ __forceinline__ d3 operator-(d3 a, d3 b) { return mk(a.x - b.x, a.y - b.y, a.z - b.z); }
+__device__ __forceinline__ d3 operator-(d3 a) { return mk(-a.x, -a.y, -a.z); }
+__device__ __forceinline__ d3 operator*(d3 a, double s) { return mk(a.x * s, a.y * s, a.z * s); }
+__device__ __forceinline__ d3 operator*(double s, d3 a) { return mk(s * a.x, s * a.y, s * a.z); }
+#ifdef WDEM_FMA
+__device__ __forceinline__ d3 operator/(d3 a, double s) { const double r = recipFast(s); return mk(a.x * r, a.y * r, a.z * r); }
+#else
+__device__ __forceinline__ d3 operator/(d3 a, double s) { return mk(a.x / s, a.y / s, a.z / s); }
+#endif
+__device__ __forceinline__ double dot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ double sqnorm(d3 a) { return a.x * a.x + a.y * a.y + a.z * a.z; }
+// sqnorm with every operation rounded on its own in both variants (never contracted): the contracted
+// variant keeps the sphere distance, the near-cancelling overlap |d| - r1 - r2 and the position update
+// identical to the exact variant, so that contact forces agree to rounding after a step from one state
+__device__ __forceinline__ double sqnormExact(d3 a) {
+  return __dadd_rn(__dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)), __dmul_rn(a.z, a.z));
+}
+// v + a s, never contracted (the position update pos + vel dt)
+__device__ __forceinline__ double addMulExact(double v, double a, double s) { return __dadd_rn(v, __dmul_rn(a, s)); }
+__device__ __forceinline__ d3 cross(d3 a, d3 b) {
+  return mk(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+}
+__device__ __forceinline__ bool isZero(d3 a) { return a.x == 0 && a.y == 0 && a.z == 0; }
+
 __device__ __forceinline__ bool zeroBits(double x) { const Halves h = halvesOf(x); return ((h.hi << 1) | h.lo) == 0; }  // x == 0
 __device__ __forceinline__ bool isZeroBits(d3 a) {
   const Halves x = halvesOf(a.x), y = halvesOf(a.y), z = halvesOf(a.z);
@@ -90,6 +154,9 @@ __device__ __forceinline__ bool nanBits(double x) {
   return m > 0x7ff00000u || (m == 0x7ff00000u && h.lo != 0);
 }
 __device__ __forceinline__ bool isOneBits(double x) { const Halves h = halvesOf(x); return h.hi == 0x3ff00000u && h.lo == 0; }  // x == 1.0
+__device__ __forceinline__ bool sameBits(double a, double b) { const Halves x = halvesOf(a), y = halvesOf(b); return x.hi == y.hi && x.lo == y.lo; }
+// |x| < bound, a positive finite constant whose low 32 bits are ignored (a switch between two formulas)
+__device__ __forceinline__ bool belowHi(double x, double bound) { return (halvesOf(x).hi & 0x7fffffffu) < halvesOf(bound).hi; }
 __device__ __forceinline__ bool finiteBits(double x) { return (halvesOf(x).hi & 0x7ff00000u) != 0x7ff00000u; }
 // a * b for finite a and b == +-0: the zero with the product's sign
 __device__ __forceinline__ double signedZero(double a, double b) {
@@ -102,7 +169,7 @@ __device__ __forceinline__ bool signsDiffer(double a, double b) { return ((halve
 __device__ __forceinline__ d3 normalized(d3 a) {
   double z = sqnorm(a);
 #ifdef WDEM_FMA
-  if (z > 0 && z != 1.0) { WDEM_REAL_BRANCH(); const double r = rsqrt(z); a.x *= r; a.y *= r; a.z *= r; }
+  if (positiveBits(z)) { const double r = rsqrtFast(z); a.x *= r; a.y *= r; a.z *= r; }
 #else
   if (z > 0 && z != 1.0) { WDEM_REAL_BRANCH(); double n = sqrt(z); a.x /= n; a.y /= n; a.z /= n; }
 #endif
@@ -118,7 +185,7 @@ __device__ __forceinline__ double qdiv(double x, double y) {
 // v / s per component (v / m, the acceleration of a node): three qdiv; contracted variant: one reciprocal
 __device__ __forceinline__ d3 divBy(d3 v, double s) {
 #ifdef WDEM_FMA
-  const double r = 1.0 / s;
+  const double r = recipFast(s);
   return mk(v.x * r, v.y * r, v.z * r);
 #else
   return mk(qdiv(v.x, s), qdiv(v.y, s), qdiv(v.z, s));
@@ -128,7 +195,7 @@ __device__ __forceinline__ d3 divBy(d3 v, double s) {
 // divisors are equal (spheres), else three
 __device__ __forceinline__ d3 divByEach(d3 v, d3 d) {
 #ifdef WDEM_FMA
-  if (d.x == d.y && d.y == d.z) { const double r = 1.0 / d.x; return mk(v.x * r, v.y * r, v.z * r); }
+  if (sameBits(d.x, d.y) && sameBits(d.y, d.z)) { const double r = recipFast(d.x); return mk(v.x * r, v.y * r, v.z * r); }
   return mk(v.x / d.x, v.y / d.y, v.z / d.z);
 #else
   return mk(qdiv(v.x, d.x), qdiv(v.y, d.y), qdiv(v.z, d.z));
@@ -196,9 +263,15 @@ __device__ __forceinline__ qd quatFromCols(d3 c0, d3 c1, d3 c2) {
   const double mi = pick(i0, m00, pick(i1, m11, m22)), mj = pick(i0, m11, pick(i1, m22, m00)),
                mk_ = pick(i0, m22, pick(i1, m00, m11));
   const double u = pick(pos, tr, mi - mj - mk_);
+#ifdef WDEM_FMA
+  const double u1 = u + 1.0, rt = rsqrtFast(u1);
+  const double d = halfOf(u1 * rt);
+  const double t = halfOf(rt);
+#else
   double t = sqrt(u + 1.0);
   const double d = halfOf(t);
   t = 0.5 / t;
+#endif
   const bool p0 = pos || i0;
   const double e1 = (pick(p0, m21, pick(i1, m02, m10)) - pick(p0, m12, pick(i1, m20, m01))) * t;
   const bool p2 = pos || i2;
@@ -231,7 +304,7 @@ __device__ __forceinline__ qd qmul(qd a, qd b) {
 __device__ __forceinline__ qd qnormalized(qd q) {
   double z2 = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
 #ifdef WDEM_FMA
-  if (!isOneBits(z2) && z2 > 0) { WDEM_REAL_BRANCH(); const double r = rsqrt(z2); q.x *= r; q.y *= r; q.z *= r; q.w *= r; }
+  if (!isOneBits(z2) && positiveBits(z2)) { const double r = rsqrtFast(z2); q.x *= r; q.y *= r; q.z *= r; q.w *= r; }
 #else
   if (!isOneBits(z2) && z2 > 0) { WDEM_REAL_BRANCH(); double n = sqrt(z2); q.x /= n; q.y /= n; q.z /= n; q.w /= n; }
 #endif
