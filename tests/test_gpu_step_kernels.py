@@ -104,3 +104,34 @@ def test_more_pairs_than_the_sweep_keeps(wdem_lib, periodic):
     h, _ = _run_both(spec, (1, 20))
     c = h.download_contacts()
     assert np.bincount(np.concatenate([c.idA, c.idB])).max() > 40
+
+
+@pytest.mark.parametrize("depth, graphs", [(2, abi.GRAPHS_OFF), (32, abi.GRAPHS_OFF), (32, abi.GRAPHS_ON)])
+def test_energy_of_queued_steps(wdem_lib, depth, graphs):
+    """Energy sums of queued steps, with collider rebuilds inside the queues, equal those of single steps bitwise."""
+    spec = scenes.random_cloud(700, 6, dense=0.85, trackEnergy=1)
+    a, b = gpu_handle(spec), gpu_handle(spec)
+    a.set_queue_depth(1)
+    b.set_queue_depth(depth)
+    b.set_step_graphs(graphs)
+    for k in (3, 60, 1, 130):
+        a.step(k)
+        b.step(k)
+        assert a.energy() == b.energy()
+    assert b.status().nFullRuns == a.status().nFullRuns > 3
+
+
+@pytest.mark.parametrize("n", [2041, 2042, 2043, 4096])
+def test_energy_sums_at_slice_edges(wdem_lib, n):
+    """Particle counts (with 6 walls) around multiples of 2048, where the sums get another block: the energies agree
+    with the oracle's, whose sums run in another order, to 1e-12."""
+    side = 0.0125 * np.ceil(n ** (1.0 / 3.0))
+    spec = scenes.random_cloud(n, n, box=(side, side, side), rmin=0.004, rmax=0.005, dense=0.8, trackEnergy=1)
+    h = gpu_handle(spec)
+    o = bridge.Oracle(spec.params, spec.particles)
+    h.step(5)
+    o.step(5)
+    eg, eo = h.energy(), o.energy()
+    eo = eo if isinstance(eo, dict) else dict(zip(abi.ENERGY_NAMES, eo))
+    for k in abi.ENERGY_NAMES:
+        assert abs(eg[k] - eo[k]) <= 1e-12 * max(abs(eo[k]), 1e-300), k

@@ -1225,9 +1225,16 @@ void col_periodic_emit(cudaStream_t s, ColliderScratch& cs, long long nCand, int
 }
 
 void launch_stress(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc, double* scratch9,
-                   double* partials, double* out9) {
+                   double* partials, double* out9, DeviceStatus* st) {
   if (nc > 0) (k_stress_terms<<<(unsigned)((nc + 255) / 256), 256, 0, s>>>(P, p, c, nc, scratch9), ++::wdem::g_kernel_launches);
-  for (int q = 0; q < 9; q++) energy_accumulate(s, scratch9 + (long long)q * nc, nc, partials, out9 + q, true);
+  SumSet S{};
+  for (int q = 0; q < 9; q++) {
+    S.x[q] = scratch9 + (long long)q * nc;
+    S.n[q] = nc;
+    S.acc[q] = out9 + q;
+  }
+  S.reset = (1 << 9) - 1;
+  launch_sums(s, P, S, 0, 9, partials, st);
 }
 
 static RowCount rowCount(int n, const Csr& csr, const ColliderScratch& cs) {

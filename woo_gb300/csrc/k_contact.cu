@@ -1367,8 +1367,7 @@ void launch_contacts(cudaStream_t s, const StepParams& P, Particles p, Contacts 
     cudaMemsetAsync(&st->rotCount, 0, 2 * sizeof(unsigned), s);  // rotCount, touchCount; otherwise cleared by the cull kernel
     return;
   }
-  unsigned* count = &st->workCount;  // workCount, workPot
-  cudaMemsetAsync(count, 0, 2 * sizeof(unsigned), s);
+  unsigned* count = &st->workCount;  // workCount, workPot (cleared by the step's integrator)
   if (full) cudaMemsetAsync(&st->actCount, 0, sizeof(unsigned), s);
   // the FP64 pass loops over the work list (length known on the device only): by default 4 blocks of 128
   // per SM fill the GPU at its register count, and no more blocks are launched to find the list short

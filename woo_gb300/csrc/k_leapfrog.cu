@@ -86,6 +86,12 @@ __device__ __forceinline__ d3 gravityForce(const StepParams& P, double mass, uns
             (zeroBits(P.gravity[2]) && mf) ? signedZero(mass, P.gravity[2]) : mass * P.gravity[2]);
 }
 
+// the work list of this step's contact pass starts empty (the last one has been consumed)
+__device__ __forceinline__ void clearWork(DeviceStatus* st) {
+  st->workCount = 0;
+  st->workPot = 0;
+}
+
 // Raises the collider trigger.  All particles of a free-falling cloud cross the verlet distance in the
 // same step, and a million stores to one word serialise in the memory system: one store per warp, and
 // none once the flag is seen set.
@@ -168,11 +174,68 @@ __device__ __noinline__ double asphericalErot(qd ori, d3 inertia, d3 w) {
   return .5 * dot(w, mvec(M, w));
 }
 
+// leapfrogSphericalRotate of a sphere with angVel != 0: q = AngleAxis(|w| dt, w/|w|) q, normalised.
+// A sphere's orientation feeds nothing else in the step (sphere contacts do not read it): it is
+// integrated to within a few ulp of the reference's operations at a fraction of their cost, with FMAs in both
+// variants.  For the half angles of a DEM step (h = |w| dt/2 < 1e-3) the Taylor polynomials sin h = h (1 - h^2/6
+// (1 - h^2/20)) and cos h = 1 - h^2/2 (1 - h^2/12) (truncation errors h^7/5040 and h^6/720, far below an
+// ulp) need neither |w| nor the axis: the vector part sin(h) w/|w| = w dt/2 (1 - h^2/6 (1 - h^2/20))
+// with h^2 = |w|^2 dt^2/4; below h = 1e-4 their last factors are 1 to within 2^-57 (h^4/120 and h^4/24).  The
+// normalisation 1/sqrt(z) of a product of unit quaternions (|z - 1| a few ulp) is its Taylor polynomial 1 - e/2 +
+// 3e^2/8, e = z - 1 (error 5e^3/16, far below an ulp), and q - q e/2 for |e| < 1e-8 (3e^2/8 < 2^-54).
+// 34 FP64 instructions for a slow spin (62 and 44 before in the exact and the contracted variant); the rotation of
+// all spheres of a cloud is two fifths of its integration.
+__device__ __forceinline__ void rotateSphere(const StepParams& P, const Particles& p, unsigned i, const double4_32a o4,
+                                             d3 angVel, int mat) {
+  const double hd = halfOf(dtOf(P, mat));
+  const double w2 = __fma_rn(angVel.z, angVel.z, __fma_rn(angVel.y, angVel.y, angVel.x * angVel.x));
+  const double h2 = w2 * (P.matDt ? hd * hd : P.hdt2);
+  qd q;
+  if (belowHi(h2, 1e-8)) {
+    const double f = __fma_rn(-h2, P.matDt ? hd * (1.0 / 6.0) : P.hdt6, hd);
+    q.w = __fma_rn(h2, -0.5, 1.0);
+    q.x = angVel.x * f; q.y = angVel.y * f; q.z = angVel.z * f;
+  } else if (belowHi(h2, 1e-6)) {
+    WDEM_REAL_BRANCH();
+    const double f = hd * (1.0 - h2 * (1.0 / 6.0) * (1.0 - h2 * 0.05));
+    q.w = 1.0 - h2 * 0.5 * (1.0 - h2 * (1.0 / 12.0));
+    q.x = angVel.x * f; q.y = angVel.y * f; q.z = angVel.z * f;
+  } else {
+    WDEM_REAL_BRANCH();
+    const double w = sqrt(w2);
+    const double inv = 1.0 / w;
+    double sh, ch;
+    sincos(w * hd, &sh, &ch);
+    q.w = ch; q.x = sh * (angVel.x * inv); q.y = sh * (angVel.y * inv); q.z = sh * (angVel.z * inv);
+  }
+  // q o, o = (o4.x; o4.y, o4.z, o4.w): the products with q's small vector part first, so that each component is
+  // rounded once at its own size
+  double r[4];
+  r[0] = __fma_rn(q.w, o4.x, __fma_rn(-q.z, o4.w, __fma_rn(-q.y, o4.z, -q.x * o4.y)));
+  r[1] = __fma_rn(q.w, o4.y, __fma_rn(-q.z, o4.z, __fma_rn(q.y, o4.w, q.x * o4.x)));
+  r[2] = __fma_rn(q.w, o4.z, __fma_rn(-q.x, o4.w, __fma_rn(q.z, o4.y, q.y * o4.x)));
+  r[3] = __fma_rn(q.w, o4.w, __fma_rn(-q.y, o4.y, __fma_rn(q.x, o4.z, q.z * o4.x)));
+  const double z2 = __fma_rn(r[0], r[0], __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], r[1] * r[1])));
+  const double e = z2 - 1.0;
+  if (belowHi(e, 1.6e-16)) {
+    // z = 1 or the number below: a correction of half an ulp would only add its own rounding
+  } else if (belowHi(e, 1e-8)) {
+    const double g = flipSign(halfOf(e));
+    for (int k = 0; k < 4; k++) r[k] = __fma_rn(r[k], g, r[k]);
+  } else {
+    WDEM_REAL_BRANCH();
+    const double rn = belowHi(e, 1e-6) ? 1.0 - e * (0.5 - 0.375 * e) : (z2 > 0 ? 1.0 / sqrt(z2) : 1.0);
+    for (int k = 0; k < 4; k++) r[k] *= rn;
+  }
+  p.ori[i] = make_double4_32a(r[0], r[1], r[2], r[3]);
+}
+
 template <bool FROM_ARRAYS, bool PERI, bool ELL>
 __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int n, Contacts c, Csr csr, DeviceStatus* st) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   const long long step = stepOf(P, st);
   if (i >= n || haltedIntegrator(st, step)) return;
+  if (i == 0) clearWork(st);
   // the marks of the last contact pass are consumed here
   const unsigned marks = p.rowMask[i];
   p.rowMask[i] = 0;
@@ -315,9 +378,16 @@ __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int
   // leapfrogTranslate (:275-278)
   pos = mk(addMulExact(pos.x, vel.x, dt), addMulExact(pos.y, vel.y, dt), addMulExact(pos.z, vel.z, dt));
   // leapfrogSphericalRotate (:280-297): q = AngleAxis(|w| dt, w/|w|) * q, normalised
-  double4_32a o4 = p.ori[i];
+  const double4_32a o4 = p.ori[i];
   qd ori; ori.w = o4.x; ori.x = o4.y; ori.y = o4.z; ori.z = o4.w;
-  if (ELL && asph) {
+  if (!ELL) {
+    // spheres only: no contact reads the orientation
+    if (!isZeroBits(angVel)) rotateSphere(P, p, (unsigned)i, o4, angVel, meta.y);
+    else {
+      ori = qnormalized(ori);
+      p.ori[i] = make_double4_32a(ori.w, ori.x, ori.y, ori.z);
+    }
+  } else if (asph) {
     if (isZeroBits(inertia)) { if (atomicCAS(&st->code, 0, WDEM_ERR_STATE) == 0) st->detail = i; }
     else asphericalRotate(P, p, i, T, inertia, ori, angVel, dt);
   } else {
@@ -336,7 +406,7 @@ __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int
   p.posf[i] = make_float4((float)pos.x, (float)pos.y, (float)pos.z, (float)pr.w);
   p.velm[i] = make_double4_32a(vel.x, vel.y, vel.z, mass);
   p.angw[i] = make_double4_32a(angVel.x, angVel.y, angVel.z, w4.w);
-  p.ori[i] = make_double4_32a(ori.w, ori.x, ori.y, ori.z);
+  if (ELL) p.ori[i] = make_double4_32a(ori.w, ori.x, ori.y, ori.z);
   // a non-finite position can never be collided again (NaN boxes overlap nothing): stop with an error,
   // as Woo stops on a NaN force
   if (!finiteBits(pos.x) || !finiteBits(pos.y) || !finiteBits(pos.z)) {
@@ -369,48 +439,6 @@ __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int
     const double d2 = sqnorm(dd);
     raiseDirty(st, dirty || (d2 > 0. ? d2 : 0.) + moveDueToRot2 > P.maxD2, step);
   }
-}
-
-// leapfrogSphericalRotate of a sphere with angVel != 0: q = AngleAxis(|w| dt, w/|w|) q, normalised.
-// A sphere's orientation feeds nothing else in the step (sphere contacts do not read it): it is
-// integrated to within a few ulp of the reference's operations at a fraction of their cost.  For the
-// half angles of a DEM step (h = |w| dt/2 < 1e-3) the Taylor polynomials sin h = h (1 - h^2/6 (1 -
-// h^2/20)) and cos h = 1 - h^2/2 (1 - h^2/12) (truncation errors h^7/5040 and h^6/720, far below an
-// ulp) need neither |w| nor the axis: the vector part sin(h) w/|w| = w dt/2 (1 - h^2/6 (1 - h^2/20))
-// with h^2 = |w|^2 dt^2/4.  The normalisation 1/sqrt(z) of a product of unit quaternions (|z - 1| a
-// few ulp) is its Taylor polynomial 1 - e/2 + 3e^2/8, e = z - 1 (error 5e^3/16, far below an ulp).
-__device__ __forceinline__ void rotateSphere(const StepParams& P, const Particles& p, unsigned i, const double4_32a o4,
-                                             d3 angVel, int mat) {
-  qd ori; ori.w = o4.x; ori.x = o4.y; ori.y = o4.z; ori.z = o4.w;
-  const double dt = dtOf(P, mat);
-  const double w2 = sqnorm(angVel);
-  const double h2 = 0.25 * (w2 * (dt * dt));
-  qd q;
-  if (belowHi(h2, 1e-6)) {
-    const double f = (0.5 * dt) * (1.0 - h2 * (1.0 / 6.0) * (1.0 - h2 * 0.05));
-    q.w = 1.0 - h2 * 0.5 * (1.0 - h2 * (1.0 / 12.0));
-    q.x = angVel.x * f; q.y = angVel.y * f; q.z = angVel.z * f;
-  } else {
-    WDEM_REAL_BRANCH();
-    const double angle = sqrt(w2);
-    const double inv = 1.0 / angle;
-    double sh, ch;
-    sincos(0.5 * (angle * dt), &sh, &ch);
-    q.w = ch; q.x = sh * (angVel.x * inv); q.y = sh * (angVel.y * inv); q.z = sh * (angVel.z * inv);
-  }
-  ori = qmul(q, ori);
-  const double z2 = ori.x * ori.x + ori.y * ori.y + ori.z * ori.z + ori.w * ori.w;
-  if (!isOneBits(z2)) {
-    double rn;
-    const double e = z2 - 1.0;
-    if (belowHi(e, 1e-6)) rn = 1.0 - e * (0.5 - 0.375 * e);
-    else {
-      WDEM_REAL_BRANCH();
-      rn = z2 > 0 ? 1.0 / sqrt(z2) : 1.0;
-    }
-    ori.x *= rn; ori.y *= rn; ori.z *= rn; ori.w *= rn;
-  }
-  p.ori[i] = make_double4_32a(ori.w, ori.x, ori.y, ori.z);
 }
 
 // The same step as k_leapfrog<false, PERI, false> without energy tracking, for one particle, issuing
@@ -738,45 +766,93 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_leapfrog_fast(StepParams P, P
 // in flight at once.  The pass is bound by these dependent chains (list entry, row, records, FP64) more than by
 // bytes or FP64 issue, so two shorter chains side by side beat one.
 static const int LIST_T = 256, LIST_ITEMS = LIST_T / 2;
+// One particle's threads: turns tells which.  e0, e1: its CSR row.
+template <bool PERI>
+__device__ __forceinline__ void integrateTouched(const StepParams& P, const Particles& p, int i, unsigned mask, bool turns,
+                                                 long long want, const Contacts& c, const Csr& csr, DeviceStatus* st) {
+  const int e0 = csr.rowptr[i], e1 = csr.rowptr[i + 1];
+  if (!turns) {
+    const FastRec rec = loadFast(p, i);
+    d3 F = gravityForce(P, rec.vm.w, (unsigned)rec.meta.w), T;
+    gatherRowMasked<SUM_F>(want, e0, e1, mask, c, F, T);
+    p.touched[i] = 0;
+    p.rowMask[i] = 0;
+    translateFast<PERI>(P, p, i, st, true, rec, F);
+  } else {
+    const int4 meta = p.meta[i];
+    const double4_32a w4 = p.angw[i], in4 = p.inert[i], o4 = p.ori[i];
+    d3 F, T = mk(0, 0, 0), angVel;
+    gatherRowMasked<SUM_T>(want, e0, e1, mask, c, F, T);
+    if (spinFast<PERI>(P, p, i, meta, w4, T, &in4, angVel)) rotateSphere(P, p, (unsigned)i, o4, angVel, meta.y);
+  }
+}
+
 template <bool PERI>
 __global__ void __launch_bounds__(LIST_T) k_leapfrog_lists(StepParams P, Particles p, int n, Contacts c, Csr csr,
                                                             DeviceStatus* st) {
   if (haltedIntegrator(st, stepOf(P, st))) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) clearWork(st);
   const unsigned nt = st->touchCount < (unsigned)n ? st->touchCount : (unsigned)n;
   const unsigned nr = st->rotCount < (unsigned)n ? st->rotCount : (unsigned)n;
   const long long want = seqOf(P, st) - 1;
   const bool turns = threadIdx.x >= LIST_ITEMS;
   const unsigned lane = threadIdx.x & (LIST_ITEMS - 1);
-  for (unsigned base = blockIdx.x * LIST_ITEMS; base < nt; base += gridDim.x * LIST_ITEMS) {
-    const unsigned k = base + lane;
-    const bool live = k < nt;
-    const int i = live ? (int)p.touchList[k] : 0;
-    unsigned mask = 0;
-    if (live) mask = p.rowMask[i];
-    __syncthreads();  // both threads of a particle have its mask
-    if (live) {
-      if (!turns) {
-        const int e0 = csr.rowptr[i], e1 = csr.rowptr[i + 1];
-        const FastRec rec = loadFast(p, i);
-        d3 F = gravityForce(P, rec.vm.w, (unsigned)rec.meta.w), T;
-        gatherRowMasked<SUM_F>(want, e0, e1, mask, c, F, T);
-        p.touched[i] = 0;
-        p.rowMask[i] = 0;
-        translateFast<PERI>(P, p, i, st, true, rec, F);
-      } else {
-        const int e0 = csr.rowptr[i], e1 = csr.rowptr[i + 1];
-        const int4 meta = p.meta[i];
-        const double4_32a w4 = p.angw[i], in4 = p.inert[i], o4 = p.ori[i];
-        d3 F, T = mk(0, 0, 0), angVel;
-        gatherRowMasked<SUM_T>(want, e0, e1, mask, c, F, T);
-        if (spinFast<PERI>(P, p, i, meta, w4, T, &in4, angVel)) rotateSphere(P, p, (unsigned)i, o4, angVel, meta.y);
+  // tasks of one block: LIST_ITEMS touched particles, then LIST_T listed rotations; different blocks take them as
+  // long as there are blocks
+  const unsigned tt = (nt + LIST_ITEMS - 1) / LIST_ITEMS, tr = (nr + LIST_T - 1) / LIST_T;
+  for (unsigned task = blockIdx.x; task < tt + tr; task += gridDim.x) {
+    if (task < tt) {
+      const unsigned k = task * LIST_ITEMS + lane;
+      const bool live = k < nt;
+      const int i = live ? (int)p.touchList[k] : 0;
+      unsigned mask = 0;
+      if (live) mask = p.rowMask[i];
+      __syncthreads();  // both threads of a particle have its mask
+      if (live) integrateTouched<PERI>(P, p, i, mask, turns, want, c, csr, st);
+    } else {
+      const unsigned k = (task - tt) * LIST_T + threadIdx.x;
+      if (k < nr) {
+        const unsigned i = p.rotList[k];
+        const double4_32a o4 = p.ori[i];
+        rotateSphere(P, p, i, o4, xyz(p.angw[i]), p.meta[i].y);
       }
     }
   }
-  for (unsigned k = blockIdx.x * LIST_T + threadIdx.x; k < nr; k += gridDim.x * LIST_T) {
-    const unsigned i = p.rotList[k];
-    const double4_32a o4 = p.ori[i];
-    rotateSphere(P, p, i, o4, xyz(p.angw[i]), p.meta[i].y);
+}
+
+// The whole integration in one launch, two threads a particle as in the list pass, for all particles in id order:
+// no lists, no second launch, and the records are read where the flags are.  Warps mix touched and untouched
+// particles, which costs FP64 issue where few are touched and many warps compete for it: taken up to ALL_PER_SM
+// particles an SM (4 warps per scheduler).  Whole steps with it and with the two passes: 10k spheres 62.2 and 66.7
+// us; 36k in a bed 109.1 and 110.4, falling 48.8 and 52.2, sheared 123.9 and 128.0; 50k 129.4 and 125.5, 57.7 and
+// 55.4, 112.1 and 107.8; 1M falling 555 and 410.
+static const int ALL_PER_SM = 256;
+template <bool PERI>
+__global__ void __launch_bounds__(LIST_T) k_leapfrog_all(StepParams P, Particles p, int n, Contacts c, Csr csr,
+                                                          DeviceStatus* st) {
+  const bool turns = threadIdx.x >= LIST_ITEMS;
+  const int i = blockIdx.x * LIST_ITEMS + (threadIdx.x & (LIST_ITEMS - 1));
+  const bool live = i < n;
+  int4 meta = make_int4(0, 0, 0, 63);
+  unsigned mask = 0;
+  uint8_t tch = 0;
+  if (live) {
+    meta = p.meta[i];
+    tch = p.touched[i];
+    mask = p.rowMask[i];
+  }
+  if (haltedIntegrator(st, stepOf(P, st))) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) clearWork(st);
+  __syncthreads();  // both threads of a particle have its flag and mask
+  if (!live) return;
+  if (((unsigned)meta.w & 63u) != 63u && tch != 0) {
+    integrateTouched<PERI>(P, p, i, mask, turns, seqOf(P, st) - 1, c, csr, st);
+  } else if (!turns) {
+    translateFast<PERI>(P, p, i, st, false, loadFast(p, i), mk(0, 0, 0));
+  } else {
+    const double4_32a w4 = p.angw[i], o4 = p.ori[i];
+    d3 angVel;
+    if (spinFast<PERI>(P, p, i, meta, w4, mk(0, 0, 0), nullptr, angVel)) rotateSphere(P, p, (unsigned)i, o4, angVel, meta.y);
   }
 }
 
@@ -816,7 +892,14 @@ void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, in
   if (n <= 0) return;
   unsigned blocks = (n + 255) / 256;
   const unsigned listBlocks = (unsigned)((n + LIST_ITEMS - 1) / LIST_ITEMS);
-  if (!fromArrays && !P.hasEll && !P.lfEnergy && p.touched && p.rotList) {
+  if (!fromArrays && !P.hasEll && !P.lfEnergy) {
+    const int sms = P.numSMs > 0 ? P.numSMs : 152;
+    if (n <= ALL_PER_SM * sms) {
+      if (P.periodic) k_leapfrog_all<true><<<listBlocks, LIST_T, 0, s>>>(P, p, n, c, csr, st);
+      else k_leapfrog_all<false><<<listBlocks, LIST_T, 0, s>>>(P, p, n, c, csr, st);
+      ++::wdem::g_kernel_launches;
+      return;
+    }
     // st->rotCount and st->touchCount are zero here: k_contacts_cull clears them for the next step (and
     // the handle starts at zero)
     if (P.periodic) {
@@ -1067,41 +1150,57 @@ WDEM_VARIANT_END
 namespace wdem {
 WDEM_VARIANT_BEGIN
 
-// Deterministic sum: each block reduces a fixed slice in a fixed shared-memory tree, then one block
-// sums the block partials the same way.  The result is independent of scheduling.
-static const int ER_T = 256;
-__global__ void k_esum(const double* x, long long n, double* partials) {
-  __shared__ double sh[ER_T];
-  long long base = (long long)blockIdx.x * ER_T * 8;
-  double acc = 0;
-  for (int k = 0; k < 8; k++) {
-    long long i = base + (long long)k * ER_T + threadIdx.x;
-    if (i < n) acc = acc + x[i];
-  }
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int off = ER_T / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < off) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + off];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
-}
-__global__ void k_efinal(const double* partials, long long nb, double* acc, int reset) {
-  __shared__ double sh[ER_T];
-  double a = 0;
-  for (long long i = threadIdx.x; i < nb; i += ER_T) a = a + partials[i];
+// Deterministic sums: each block reduces a fixed slice of one array in a fixed shared-memory tree, and the last
+// block of an array to finish sums the block partials the same way; the result is independent of scheduling.  All
+// sums of a step run in one launch, an array per grid row: a step with its energy tracked had 8 sums of two
+// launches each, half of its time at 30k bodies (63 of 125 us).
+static const int ER_T = 256, ER_SLICE = ER_T * 8;
+long long sum_blocks(long long n) { return std::max<long long>(1, (n + ER_SLICE - 1) / ER_SLICE); }
+__device__ __forceinline__ double treeSum(double* sh, double a) {
   sh[threadIdx.x] = a;
   __syncthreads();
   for (int off = ER_T / 2; off > 0; off >>= 1) {
     if (threadIdx.x < off) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + off];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *acc = reset ? sh[0] : *acc + sh[0];
+  return sh[0];
 }
-void energy_accumulate(cudaStream_t s, const double* x, long long n, double* partials, double* acc, bool reset) {
-  long long nb = (n + ER_T * 8 - 1) / (ER_T * 8);
-  if (nb > 0) (k_esum<<<(unsigned)nb, ER_T, 0, s>>>(x, n, partials), ++::wdem::g_kernel_launches);
-  (k_efinal<<<1, ER_T, 0, s>>>(partials, nb, acc, reset ? 1 : 0), ++::wdem::g_kernel_launches);
+__global__ void __launch_bounds__(ER_T) k_sums(StepParams P, SumSet S, int row0, long long stride, double* partials,
+                                               unsigned* tickets, const DeviceStatus* st) {
+  __shared__ double sh[ER_T];
+  __shared__ bool last;
+  const int y = row0 + blockIdx.y;
+  if (S.guarded && (y < S.contactRow ? haltedIntegrator(st, stepOf(P, st)) : haltedContacts(st, stepOf(P, st)))) return;
+  const long long n = S.n[y], nb = (n + ER_SLICE - 1) / ER_SLICE, blocks = nb > 0 ? nb : 1;
+  if ((long long)blockIdx.x >= blocks) return;
+  const double* x = S.x[y];
+  const long long base = (long long)blockIdx.x * ER_SLICE;
+  double acc = 0;
+  for (int k = 0; k < 8; k++) {
+    const long long i = base + (long long)k * ER_T + threadIdx.x;
+    if (i < n) acc = acc + x[i];
+  }
+  acc = treeSum(sh, acc);
+  if (threadIdx.x == 0) {
+    *(volatile double*)(partials + y * stride + blockIdx.x) = acc;
+    __threadfence();
+    last = atomicAdd(&tickets[y], 1u) == (unsigned)(blocks - 1);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0;
+  for (long long i = threadIdx.x; i < nb; i += ER_T) a = a + *(volatile const double*)(partials + y * stride + i);
+  a = treeSum(sh, a);
+  if (threadIdx.x == 0) {
+    *S.acc[y] = (S.reset >> y) & 1 ? a : *S.acc[y] + a;
+    tickets[y] = 0;
+  }
+}
+void launch_sums(cudaStream_t s, const StepParams& P, const SumSet& S, int row0, int rows, double* partials, DeviceStatus* st) {
+  long long nb = 1;
+  for (int y = row0; y < row0 + rows; y++) nb = std::max(nb, sum_blocks(S.n[y]));
+  (k_sums<<<dim3((unsigned)nb, (unsigned)rows), ER_T, 0, s>>>(P, S, row0, nb, partials, st->sumTickets, st), ++::wdem::g_kernel_launches);
 }
 
 WDEM_VARIANT_END

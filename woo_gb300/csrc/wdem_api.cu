@@ -277,7 +277,7 @@ void freeContacts(ContactBuf& b) {
   for (int k = 0; k < HIST_COUNT; k++) cudaFree(c.hist[k]);
   cudaFree(c.out); cudaFree(c.slot); cudaFree(c.rowBit);
   for (int k = 0; k < 7; k++) cudaFree(c.geom[k]);
-  for (int k = 0; k < EC_COUNT; k++) cudaFree(c.energy[k]);
+  cudaFree(c.energy[0]);
   cudaFree(c.cdist);
   cudaFree(c.work);
   cudaFree(c.lam);
@@ -303,7 +303,8 @@ cudaError_t allocContacts(ContactBuf& b, long long cap, bool hertz, bool geom, b
   if ((e = dalloc(c.slot, cap))) return e;
   if ((e = dalloc(c.rowBit, cap))) return e;
   if (geom) for (int k = 0; k < 7; k++) if ((e = dalloc(c.geom[k], cap))) return e;
-  for (int k = 0; k < EC_COUNT; k++) if ((e = dalloc(c.energy[k], cap))) return e;
+  if ((e = dalloc(c.energy[0], (size_t)EC_COUNT * cap))) return e;
+  for (int k = 1; k < EC_COUNT; k++) c.energy[k] = c.energy[0] + (size_t)k * cap;
   if ((e = dalloc(c.work, cap))) return e;
   if ((e = dalloc(c.act, cap))) return e;
   if (peri && (e = dalloc(c.cdist, cap))) return e;
@@ -426,7 +427,7 @@ int ensureCsr(wdem_handle* h, long long nc) {
 }
 
 int ensurePartials(wdem_handle* h, long long n) {
-  long long need = n / 2048 + 16;
+  const long long need = SUM_ROWS * sum_blocks(n);
   if (need > h->ePartialsCap) {
     CK(dalloc(h->ePartials, need));
     h->ePartialsCap = need;
@@ -522,10 +523,16 @@ int rebuild(wdem_handle* h) {
   return WDEM_OK;
 }
 
+void setStepDt(StepParams& P, double dt) {
+  P.dt = dt;
+  P.hdt2 = (0.5 * dt) * (0.5 * dt);
+  P.hdt6 = (0.5 * dt) * (1.0 / 6.0);
+}
+
 void fillStepParams(wdem_handle* h) {
   const wdem_params& r = h->raw;
   StepParams& P = h->P;
-  P.dt = r.dt;
+  setStepDt(P, r.dt);
   P.step = h->step;
   P.shContactsBlock = h->launchShape.contactsBlock; P.shContactsPerSM = h->launchShape.contactsPerSM;
   P.shCullBlock = h->launchShape.cullBlock; P.shLeapBlock = h->launchShape.integratorBlock; P.shListsPerSM = h->launchShape.listsPerSM;
@@ -1084,8 +1091,7 @@ int wdem_upload_contacts(wdem_handle* h, const wdem_contacts* c) {
 // the trigger, the contact pass of k and all later queued kernels return at once.  The host then sees
 // haltAt, rebuilds and runs the contact pass of step k, exactly the sequence of the one-step path.  Only
 // the configurations whose host-side per-step work is none are queued: no periodic cell (integrated on
-// the host each step), no energy tracking (host-launched reductions), no updatePhys='once', no phase
-// timing.
+// the host each step), no updatePhys='once', no phase timing.
 // pown (src/supp/base/Math.hpp:166-175): x^n by squaring, x^n = (x^2)^(n/2) x^(n%2)
 static double powUint(double x, unsigned n) {
   const unsigned d = n >> 1, r = n & 1;
@@ -1135,13 +1141,37 @@ static int dynDtAfterContacts(wdem_handle* h, long long s) {
 static void applyNextDt(wdem_handle* h) {
   if (std::isnan(h->nextDt)) return;
   h->raw.dt = h->nextDt;
-  h->P.dt = h->nextDt;
+  setStepDt(h->P, h->nextDt);
   h->nextDt = std::numeric_limits<double>::quiet_NaN();
+}
+
+// Energy terms of a step: the rows of the integrator's per-particle terms, then of the contact pass's
+enum { EP_ROWS = 3 };
+static void clearContactEnergy(wdem_handle* h) {
+  const ContactBuf& b = h->buf[h->cur];
+  if (h->nContacts > 0)
+    cudaMemset2DAsync(b.c.energy[0], b.cap * sizeof(double), 0, h->nContacts * sizeof(double), EC_COUNT, h->stream);
+}
+static void sumEnergies(wdem_handle* h, const StepParams& P, int row0) {
+  SumSet S{};
+  const double* lf[EP_ROWS] = {h->d.energy[EP_GRAV], h->d.energy[EP_DAMP], h->d.energy[EP_KIN]};
+  const int lfTo[EP_ROWS] = {WDEM_E_GRAV, WDEM_E_NONVISCDAMP, WDEM_E_KINETIC};
+  const int cTo[EC_COUNT] = {WDEM_E_ELAST, WDEM_E_PLAST, WDEM_E_VISCN, WDEM_E_VISCT, WDEM_E_BROKEN};
+  for (int k = 0; k < EP_ROWS; k++) { S.x[k] = lf[k]; S.n[k] = h->n; S.acc[k] = h->dEnergy + lfTo[k]; }
+  for (int k = 0; k < EC_COUNT; k++) {
+    S.x[EP_ROWS + k] = h->buf[h->cur].c.energy[k];
+    S.n[EP_ROWS + k] = h->nContacts;
+    S.acc[EP_ROWS + k] = h->dEnergy + cTo[k];
+  }
+  S.reset = (1 << EP_KIN) | (1 << (EP_ROWS + EC_ELAST));  // EnergyTracker's resettable entries
+  S.contactRow = EP_ROWS;
+  S.guarded = 1;
+  launch_sums(h->stream, P, S, row0, EP_ROWS + EC_COUNT - row0, h->ePartials, h->dst);
 }
 
 // steps may run queued (no host-side per-step work, queue depth not set to 1)
 static bool queueEligible(const wdem_handle* h) {
-  return !(h->timing || h->periodic || h->P.trackEnergy || h->needRebuild || h->forcesInArrays ||
+  return !(h->timing || h->periodic || h->needRebuild || h->forcesInArrays ||
            h->verletDistResolved == 0 || h->updatePhys == WDEM_UPDATE_PHYS_ONCE || h->maxAhead < 2);
 }
 
@@ -1167,8 +1197,10 @@ static void launchQueue(wdem_handle* h, StepParams P, int ahead, bool full, bool
     P.step = step0 + g;
     P.seq = seq0 + 1 + g;
     (h->raw.arith != WDEM_ARITH_EXACT ? contracted::launch_leapfrog : launch_leapfrog)(s, P, h->d, h->n, 0, h->buf[h->cur].c, h->csr, h->dst);
+    if (P.trackEnergy) clearContactEnergy(h);
     (h->raw.arith != WDEM_ARITH_EXACT ? contracted::launch_contacts : launch_contacts)(s, P, h->d, h->buf[h->cur].c, h->nContacts, h->dst, g == 0 && full,
                     warm ? h->mlpWbf : nullptr, warm ? h->mlpW : nullptr);
+    if (P.trackEnergy) sumEnergies(h, P, 0);
   }
 }
 
@@ -1192,7 +1224,8 @@ static int replayQueue(wdem_handle* h, int ahead, bool full, bool warm) {
     sig.insert(sig.end(), b, b + nb);
   };
   const int n = h->n, arith = h->raw.arith;
-  const void* wp[2] = {warm ? (const void*)h->mlpWbf : nullptr, warm ? (const void*)h->mlpW : nullptr};
+  const void* wp[4] = {warm ? (const void*)h->mlpWbf : nullptr, warm ? (const void*)h->mlpW : nullptr,
+                       P.trackEnergy ? (const void*)h->ePartials : nullptr, P.trackEnergy ? (const void*)h->dEnergy : nullptr};
   put(&P, sizeof P); put(&h->d, sizeof h->d); put(&h->buf[h->cur].c, sizeof(Contacts)); put(&h->csr, sizeof h->csr);
   put(&h->nContacts, sizeof h->nContacts); put(&n, sizeof n); put(&arith, sizeof arith); put(&h->dst, sizeof h->dst);
   put(wp, sizeof wp);
@@ -1252,6 +1285,10 @@ static int runQueued(wdem_handle* h, int ahead, int& done, bool& statusCurrent) 
   const long long q0 = h->seq;
   const bool full = !h->actValid;
   h->P.denseTouch = h->denseTouch ? 1 : 0;
+  if (h->P.trackEnergy) {
+    int rc0;
+    if ((rc0 = ensurePartials(h, std::max<long long>(h->n, h->nContacts)))) return rc0;
+  }
   const int viaGraph = replayQueue(h, ahead, full, warm);
   if (viaGraph < 0) return viaGraph;
   if (viaGraph == 0) {
@@ -1283,8 +1320,13 @@ static int runQueued(wdem_handle* h, int ahead, int& done, bool& statusCurrent) 
     CK(cudaMemsetAsync(&h->dst->dirty, 0, sizeof(int), s));
     CK(cudaMemsetAsync(&h->dst->haltAt, 0, sizeof(long long), s));
     if ((rc = rebuild(h))) return rc;
+    if (h->P.trackEnergy) {
+      if ((rc = ensurePartials(h, std::max<long long>(h->n, h->nContacts)))) return rc;
+      clearContactEnergy(h);
+    }
     (h->raw.arith != WDEM_ARITH_EXACT ? contracted::launch_contacts : launch_contacts)(s, h->P, h->d, h->buf[h->cur].c, h->nContacts, h->dst, !h->actValid, warm ? h->mlpWbf : nullptr,
                     warm ? h->mlpW : nullptr);
+    if (h->P.trackEnergy) sumEnergies(h, h->P, EP_ROWS);  // the integrator's terms were summed in the queue
     h->actValid = true;
     h->sinceRebuild += (int)(k - s0) + 1;
     h->rebuildInterval = 0.75 * h->rebuildInterval + 0.25 * h->sinceRebuild;
@@ -1393,13 +1435,6 @@ int wdem_step(wdem_handle* h, int32_t nSteps) {
       // kinetic is resettable (EnergyTracker::resetResettables at the start of the step)
       CK(cudaMemsetAsync(h->dEnergy + WDEM_E_KINETIC, 0, sizeof(double), s));
     }
-    if (h->P.lfEnergy) {
-      int rc0;
-      if ((rc0 = ensurePartials(h, std::max<long long>(h->n, h->nContacts)))) return rc0;
-      energy_accumulate(s, h->d.energy[EP_GRAV], h->n, h->ePartials, h->dEnergy + WDEM_E_GRAV, false);
-      energy_accumulate(s, h->d.energy[EP_DAMP], h->n, h->ePartials, h->dEnergy + WDEM_E_NONVISCDAMP, false);
-      energy_accumulate(s, h->d.energy[EP_KIN], h->n, h->ePartials, h->dEnergy + WDEM_E_KINETIC, true);
-    }
     h->forcesInArrays = false;
     CK(cudaMemcpyAsync(h->hst, h->dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1418,9 +1453,9 @@ int wdem_step(wdem_handle* h, int32_t nSteps) {
       PhaseTimer t(h, PH_COLLIDER);
       if ((rc = rebuild(h))) return rc;
     }
-    if (h->P.trackEnergy && h->nContacts > 0) {
-      for (int k = 0; k < EC_COUNT; k++)
-        CK(cudaMemsetAsync(h->buf[h->cur].c.energy[k], 0, sizeof(double) * h->nContacts, s));
+    if (h->P.trackEnergy) {
+      if ((rc = ensurePartials(h, std::max<long long>(h->n, h->nContacts)))) return rc;
+      clearContactEnergy(h);
     }
     {
       PhaseTimer t(h, PH_CONTACTS);
@@ -1429,17 +1464,7 @@ int wdem_step(wdem_handle* h, int32_t nSteps) {
                       warm ? h->mlpW : nullptr);
       h->actValid = true;
     }
-    if (h->P.trackEnergy) {
-      int rc0;
-      if ((rc0 = ensurePartials(h, std::max<long long>(h->n, h->nContacts)))) return rc0;
-      const Contacts& cc = h->buf[h->cur].c;
-      const long long nc = h->nContacts;
-      energy_accumulate(s, cc.energy[EC_ELAST], nc, h->ePartials, h->dEnergy + WDEM_E_ELAST, true);
-      energy_accumulate(s, cc.energy[EC_PLAST], nc, h->ePartials, h->dEnergy + WDEM_E_PLAST, false);
-      energy_accumulate(s, cc.energy[EC_VISCN], nc, h->ePartials, h->dEnergy + WDEM_E_VISCN, false);
-      energy_accumulate(s, cc.energy[EC_VISCT], nc, h->ePartials, h->dEnergy + WDEM_E_VISCT, false);
-      energy_accumulate(s, cc.energy[EC_BROKEN], nc, h->ePartials, h->dEnergy + WDEM_E_BROKEN, false);
-    }
+    if (h->P.trackEnergy) sumEnergies(h, h->P, h->P.lfEnergy ? 0 : EP_ROWS);
     if (h->updatePhys == WDEM_UPDATE_PHYS_ONCE) { h->updatePhys = WDEM_UPDATE_PHYS_NEVER; h->raw.updatePhys = WDEM_UPDATE_PHYS_NEVER; }
     if ((rc = dynDtAfterContacts(h, h->step))) return rc;  // DynDt, the engine after ContactLoop
     if (h->periodic) h->cell.setNextGradV();  // epilogue (Scene.cpp:430)
@@ -2098,7 +2123,7 @@ int wdem_get_stress(wdem_handle* h, double* stress) {
   int rc;
   if ((rc = ensurePartials(h, std::max<long long>(nc, 1)))) return rc;
   if (h->periodic) fillCellParams(h);
-  launch_stress(s, h->P, h->d, h->buf[h->cur].c, nc, h->stressTerms, h->ePartials, h->dStress);
+  launch_stress(s, h->P, h->d, h->buf[h->cur].c, nc, h->stressTerms, h->ePartials, h->dStress, h->dst);
   double v[9];
   CK(cudaMemcpyAsync(v, h->dStress, sizeof(v), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));

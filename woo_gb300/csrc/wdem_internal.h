@@ -101,6 +101,7 @@ enum { MCLS_PZERO = 0, MCLS_NZERO = 1, MCLS_ONE = 2, MCLS_GEN = 3 };
 // Engine + functor attributes as the kernels see them.
 struct StepParams {
   double dt;
+  double hdt2, hdt6;        // (dt/2)^2 and dt/12, for the rotation of spheres
   long long step;
   long long seq;            // number of this step's contact pass (never reset); stamps the pass's force records
   int dw;                   // the contact law of real sphere/wall contacts in double-word FP32 (WDEM_ARITH_DW)
@@ -201,7 +202,7 @@ struct Contacts {
   uchar2* rowBit;    // the same entries as positions in their rows, min(position, 31)
   double4_32a* out;  // OUT_RECORDS records per CSR entry e: out[OUT_RECORDS * e + OUT_F / OUT_T] (capacity 2C entries)
   double* geom[7];  // optional (download): L6Geom.uN, vel (3), angVel (3); null when not kept
-  double* energy[EC_COUNT];  // per-contact energy terms of this step when tracked (else null)
+  double* energy[EC_COUNT];  // per-contact energy terms of this step when tracked (one allocation, C apart)
   int4* cdist;      // periodic: Contact.cellDist (x, y, z, unused); null otherwise
   unsigned* work;   // indices of the contacts the heavy pass processes this step (capacity = contacts)
   unsigned* act;    // contacts the cull walks until the next rebuild (not dead, not wall + wall, not far)
@@ -248,6 +249,7 @@ struct DeviceStatus {
   double ext[12];     // box extents reduction scratch (as ordered ints)
   long long stepBase;  // graph replays: Scene.step of the replay's first step
   long long seqBase;   //   and the contact-pass number before it
+  unsigned sumTickets[9];  // blocks done per row of the running sums (left at 0)
 };
 
 #ifdef __CUDACC__
@@ -296,8 +298,18 @@ double fp64_probe(cudaStream_t s, double* scratch, int sms, float* msOut);
 void launch_refresh_posf(cudaStream_t s, Particles p, int n);
 // angw.w = RN(RN(m g[gravAxis]) / m), the acceleration of a particle under gravity alone
 void launch_grav_acc(cudaStream_t s, const StepParams& P, Particles p, int n);
-// deterministic sum of x[0..n) added to *acc (or stored, when reset): fixed-order block trees
-void energy_accumulate(cudaStream_t s, const double* x, long long n, double* partials, double* acc, bool reset);
+// Deterministic sums (fixed-order block trees) of rows x[y][0..n[y]), added to *acc[y] or stored there (bit y of
+// reset).  guarded: the sums of a queued step, which follow its integrator (rows before contactRow) or its contact
+// pass (the others) in returning at once behind a collider trigger.
+enum { SUM_ROWS = 9 };
+struct SumSet {
+  const double* x[SUM_ROWS];
+  long long n[SUM_ROWS];
+  double* acc[SUM_ROWS];
+  int reset, contactRow, guarded;
+};
+long long sum_blocks(long long n);  // partials per row for sums of up to n values
+void launch_sums(cudaStream_t s, const StepParams& P, const SumSet& S, int row0, int rows, double* partials, DeviceStatus* st);
 // ---- the contracted variant of k_leapfrog.cu and k_contact.cu (compiled with WDEM_FMA, wdem_variant.h):
 // the same launchers, FP64 multiply-adds contracted, one reciprocal per vector division
 namespace contracted {
@@ -387,7 +399,7 @@ cudaError_t noalloc_scratch(int device, void** addr);
 cudaError_t launch_stress_noalloc(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc,
                                   void* scratch, double* out9);
 void launch_stress(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc, double* scratch9,
-                   double* partials, double* out9);
+                   double* partials, double* out9, DeviceStatus* st);
 void col_retain_flags(cudaStream_t s, const StepParams& P, Particles p, Contacts old, long long nOld, ColliderScratch& cs);
 void col_retain_write(cudaStream_t s, Contacts old, long long nOld, ColliderScratch& cs, int2* out, long long base,
                       long long cap);
