@@ -139,6 +139,29 @@ __device__ __forceinline__ void tcLoad16(uint32_t taddr, float* v) {
   for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
 
+// W[l] (K inputs x N outputs, row-major BF16 in global memory) as the K-major operand of N rows x K columns (the
+// forward B operand, transposed) or of K rows x N columns (the backward one, as stored): 16-byte loads, every
+// thread 8 outputs of one input.  Rows of 2-byte loads down the columns took 32 dependent rounds of global loads
+// per 64 x 64 matrix.
+template <int K, int N>
+__device__ __forceinline__ void stageTransposed(unsigned char* sm, int dst, const uint16_t* w) {
+  for (int e = threadIdx.x; e < K * N / 8; e += blockDim.x) {
+    const int k = e / (N / 8), n0 = e % (N / 8) * 8;
+    const uint4 q = *reinterpret_cast<const uint4*>(w + k * N + n0);
+    const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      *reinterpret_cast<uint16_t*>(sm + dst + kmajorOff(n0 + j, k, K)) = (uint16_t)(v[j >> 1] >> (16 * (j & 1)));
+  }
+}
+template <int K, int N>
+__device__ __forceinline__ void stageRows(unsigned char* sm, int dst, const uint16_t* w) {
+  for (int e = threadIdx.x; e < K * N / 8; e += blockDim.x) {
+    const int k = e / (N / 8), n0 = e % (N / 8) * 8;
+    *reinterpret_cast<uint4*>(sm + dst + kmajorOff(k, n0, N)) = *reinterpret_cast<const uint4*>(w + k * N + n0);
+  }
+}
+
 // one layer: D = A (128 x K, at aOff) x B^T (N x K, at bOff), issued by thread 0, waited for by all;
 // false when the wait gave up
 template <int K, int N>
@@ -191,15 +214,9 @@ __global__ void __launch_bounds__(128, 1) k_mlp_tc(Particles p, Contacts c, cons
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smRaw) + 1023) & ~uintptr_t(1023));
   const int t = threadIdx.x, warp = t >> 5;
   // weights as B operands (W transposed: output rows, input columns), biases
-  for (int e = t; e < H * 16; e += blockDim.x) {
-    const int n = e / 16, k = e % 16;
-    *reinterpret_cast<uint16_t*>(sm + TC_W1 + kmajorOff(n, k, 16)) = wbf[OFF_W1 + k * H + n];
-  }
-  for (int e = t; e < H * H; e += blockDim.x) {
-    const int n = e / H, k = e % H;
-    *reinterpret_cast<uint16_t*>(sm + TC_W2 + kmajorOff(n, k, H)) = wbf[OFF_W2 + k * H + n];
-    *reinterpret_cast<uint16_t*>(sm + TC_W3 + kmajorOff(n, k, H)) = wbf[OFF_W3 + k * H + n];
-  }
+  stageTransposed<16, H>(sm, TC_W1, wbf + OFF_W1);
+  stageTransposed<H, H>(sm, TC_W2, wbf + OFF_W2);
+  stageTransposed<H, H>(sm, TC_W3, wbf + OFF_W3);
   for (int e = t; e < TC_N4 * H; e += blockDim.x) {
     const int n = e / H, k = e % H;
     *reinterpret_cast<uint16_t*>(sm + TC_W4 + kmajorOff(n, k, H)) = n < 8 ? wbf[OFF_W4 + k * 8 + n] : (uint16_t)0;
@@ -305,8 +322,9 @@ __global__ void __launch_bounds__(128, 1) k_mlp_tc(Particles p, Contacts c, cons
 // accumulators stay in TMEM across all tiles of the CTA) and dA_{l-1} = dZ_l W_l^T (M = 128 samples, N = 64
 // inputs, K = outputs), whose epilogue masks by ReLU' (H_{l-1} > 0) and rounds to BF16 the next dZ.  The
 // transposed operands (H^T, dZ^T: samples along K) are written by each thread into its sample's column.
-// Bias gradients and the loss are summed from the FP32 values (warp shuffles, then shared atomics), as in
-// the warp-level kernel; the CTA adds everything to the global gradient once, at the end.
+// Bias gradients and the loss are summed from the FP32 values (per lane over the tiles); the CTA adds everything to
+// the global gradient once, at the end.  64k records (512 tiles, 3.4 a CTA): 462 -> 148 us a call with the host's
+// copies, of which the kernel was 230 us; 300 records 132 -> 78.
 constexpr int TT_FW1 = 0;                          // forward B operands (W^T: outputs x inputs)
 constexpr int TT_FW2 = TT_FW1 + H * 16 * 2;
 constexpr int TT_FW3 = TT_FW2 + H * H * 2;
@@ -356,29 +374,49 @@ __device__ __forceinline__ void tcIssue(unsigned char* sm, int aOff, int bOff, u
     tcMma(d, tcDesc(a0 + 256 * ks, 128, K / 8 * 128), tcDesc(b0 + 256 * ks, 128, K / 8 * 128), tcIdesc(TC_M, N),
           (ks > 0 || accumulate) ? 1 : 0);
 }
-// column sums of the warp (FP32, shuffles) added to the CTA's sums
-__device__ __forceinline__ void warpColumnAdd(float* dst, const float* v, int cols) {
-  for (int c = 0; c < cols; c++) {
-    float x = v[c];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&dst[c], x);
+// Sums over the warp of 32 columns, one value of each per lane: column `lane` to lane `lane`.  Half of the columns
+// change lanes in each of 5 rounds (31 shuffles; a butterfly per column takes 160).
+__device__ __forceinline__ float warpColumnSums(float* v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int m = 16; m >= 1; m >>= 1) {
+    const bool up = (lane & m) != 0;
+#pragma unroll
+    for (int j = 0; j < m; j++) {
+      const float keep = up ? v[j + m] : v[j], send = up ? v[j] : v[j + m];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+    }
   }
+  return v[0];
 }
-// the sample's column of a transposed operand: element (r, t) of an R x 128 K-major tile, r = 0 .. cols-1
-__device__ __forceinline__ void putColumn(unsigned char* sm, int off, int t, const uint16_t* v, int cols) {
-  for (int r = 0; r < cols; r++) *reinterpret_cast<uint16_t*>(sm + off + kmajorOff(r, t, TC_M)) = v[r];
+// The sample's column of a transposed operand: element (r, t) of an R x 128 K-major tile, r = 0 .. cols-1.  Two
+// neighbouring samples exchange halves so that each writes 4 bytes, every other row.
+template <int COLS>
+__device__ __forceinline__ void putColumn(unsigned char* sm, int off, int t, const uint16_t* v) {
+  const bool odd = t & 1;
+#pragma unroll
+  for (int r = 0; r < COLS; r += 2) {
+    const uint32_t own = pk(v[r], v[r + 1]);
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+    const uint32_t w = odd ? (other >> 16) | (own & 0xffff0000u) : (own & 0xffffu) | (other << 16);
+    *reinterpret_cast<uint32_t*>(sm + off + kmajorOff(odd ? r + 1 : r, t & ~1, TC_M)) = w;
+  }
 }
 // this thread's row of a 128 x 64 activation tile
 __device__ __forceinline__ void getRow64(const unsigned char* sm, int off, int t, uint16_t* v) {
+#pragma unroll
   for (int c = 0; c < H; c += 8) {
     const uint4 q = *reinterpret_cast<const uint4*>(sm + off + kmajorOff(t, c, H));
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
     for (int k = 0; k < 4; k++) { v[c + 2 * k] = (uint16_t)(w[k] & 0xffff); v[c + 2 * k + 1] = (uint16_t)(w[k] >> 16); }
   }
 }
-// dZ_prev = dA (this thread's accumulator row) masked by ReLU' of the activation row hv; bias-gradient sums;
-// dZ_prev as the next A operand (row t) and as the transposed B operand (column t)
-__device__ __forceinline__ void backEpilogue(unsigned char* sm, uint32_t tRow, const uint16_t* hv, float* gb, int t) {
+// dZ_prev = dA (this thread's accumulator row) masked by ReLU' of the activation row hv; bias-gradient sums of
+// columns lane and 32 + lane into gb (registers: the CTA's sums are made once, at the end; 64 columns of shuffles
+// and shared FP32 atomics per layer and tile were most of a tile's time); dZ_prev as the next A operand (row t) and
+// as the transposed B operand (column t)
+__device__ __forceinline__ void backEpilogue(unsigned char* sm, uint32_t tRow, const uint16_t* hv, float (&gb)[2], int t) {
   float z[H];
 #pragma unroll
   for (int c = 0; c < H; c += 16) tcLoad16(tRow + c, z + c);
@@ -388,13 +426,22 @@ __device__ __forceinline__ void backEpilogue(unsigned char* sm, uint32_t tRow, c
     z[c] = fbf(hv[c]) > 0.f ? z[c] : 0.f;
     zb[c] = bf(z[c]);
   }
-  warpColumnAdd(gb, z, H);
+#pragma unroll
   for (int c = 0; c < H; c += 8) {
     uint32_t w[4];
+#pragma unroll
     for (int k = 0; k < 4; k++) w[k] = pk(zb[c + 2 * k], zb[c + 2 * k + 1]);
     *reinterpret_cast<uint4*>(sm + TT_DZ + kmajorOff(t, c, H)) = make_uint4(w[0], w[1], w[2], w[3]);
   }
-  putColumn(sm, TT_DZT, t, zb, H);
+  putColumn<H>(sm, TT_DZT, t, zb);
+  gb[0] += warpColumnSums(z);
+  gb[1] += warpColumnSums(z + 32);
+}
+
+// four floats added in global memory by one instruction (16-byte aligned)
+__device__ __forceinline__ void addGlobal4(float* p, const float* v) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+               : "memory");
 }
 
 __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const int* idx, long long n, float invN,
@@ -404,17 +451,11 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smRaw) + 1023) & ~uintptr_t(1023));
   const int t = threadIdx.x, warp = t >> 5;
   // weights: forward B (W^T) and backward B (W), biases; the padded rows of H^T stay zero
-  for (int e = t; e < H * 16; e += blockDim.x) {
-    const int nn = e / 16, k = e % 16;
-    *reinterpret_cast<uint16_t*>(sm + TT_FW1 + kmajorOff(nn, k, 16)) = wbf[OFF_W1 + k * H + nn];
-  }
-  for (int e = t; e < H * H; e += blockDim.x) {
-    const int a = e / H, b = e % H;
-    *reinterpret_cast<uint16_t*>(sm + TT_FW2 + kmajorOff(a, b, H)) = wbf[OFF_W2 + b * H + a];
-    *reinterpret_cast<uint16_t*>(sm + TT_FW3 + kmajorOff(a, b, H)) = wbf[OFF_W3 + b * H + a];
-    *reinterpret_cast<uint16_t*>(sm + TT_BW3 + kmajorOff(a, b, H)) = wbf[OFF_W3 + a * H + b];
-    *reinterpret_cast<uint16_t*>(sm + TT_BW2 + kmajorOff(a, b, H)) = wbf[OFF_W2 + a * H + b];
-  }
+  stageTransposed<16, H>(sm, TT_FW1, wbf + OFF_W1);
+  stageTransposed<H, H>(sm, TT_FW2, wbf + OFF_W2);
+  stageTransposed<H, H>(sm, TT_FW3, wbf + OFF_W3);
+  stageRows<H, H>(sm, TT_BW3, wbf + OFF_W3);
+  stageRows<H, H>(sm, TT_BW2, wbf + OFF_W2);
   for (int e = t; e < TC_N4 * H; e += blockDim.x) {
     const int a = e / H, b = e % H;  // forward: output a, input b
     *reinterpret_cast<uint16_t*>(sm + TT_FW4 + kmajorOff(a, b, H)) = a < 8 ? wbf[OFF_W4 + b * 8 + a] : (uint16_t)0;
@@ -449,6 +490,8 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
   unsigned phase = 0;
   bool ok = true, first = true;
   float myLoss = 0.f;
+  // bias-gradient sums: columns lane, 32 + lane of layers 1-3; of the output layer, all lanes alike
+  float gb1[2] = {0.f, 0.f}, gb2[2] = {0.f, 0.f}, gb3[2] = {0.f, 0.f}, gb4[ELL_TARGETS] = {0.f, 0.f, 0.f, 0.f};
   for (long long base = (long long)blockIdx.x * TC_M; base < n && ok; base += (long long)gridDim.x * TC_M) {
     const long long s = base + t;
     const bool valid = s < n;
@@ -482,17 +525,22 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
           myLoss += c_lossW[k] * e * e * invN;
           d[k] = 2.f * c_lossW[k] * e * invN;
         }
-      warpColumnAdd(gb + 3 * H, d, ELL_TARGETS);
+#pragma unroll
+      for (int k = 0; k < ELL_TARGETS; k++) {
+        float x = d[k];
+        for (int q = 16; q > 0; q >>= 1) x += __shfl_xor_sync(0xffffffffu, x, q);
+        gb4[k] += x;
+      }
       uint16_t db[16];
       for (int k = 0; k < 16; k++) db[k] = bf(d[k]);
       uint32_t w[8];
       for (int k = 0; k < 8; k++) w[k] = pk(db[2 * k], db[2 * k + 1]);
       *reinterpret_cast<uint4*>(sm + TT_DZ + kmajorOff(t, 0, TC_N4)) = make_uint4(w[0], w[1], w[2], w[3]);
       *reinterpret_cast<uint4*>(sm + TT_DZ + kmajorOff(t, 8, TC_N4)) = make_uint4(w[4], w[5], w[6], w[7]);
-      putColumn(sm, TT_DZT, t, db, TC_N4);
+      putColumn<TC_N4>(sm, TT_DZT, t, db);
       uint16_t hv[H];
       getRow64(sm, TT_H3, t, hv);
-      putColumn(sm, TT_AT, t, hv, H);
+      putColumn<H>(sm, TT_AT, t, hv);
     }
     const bool acc = !first;
     // layer 4: dW4, dA3
@@ -504,9 +552,9 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
     {
       uint16_t hv[H];
       getRow64(sm, TT_H3, t, hv);
-      backEpilogue(sm, tRow, hv, gb + 2 * H, t);
+      backEpilogue(sm, tRow, hv, gb3, t);
       getRow64(sm, TT_H2, t, hv);
-      putColumn(sm, TT_AT, t, hv, H);
+      putColumn<H>(sm, TT_AT, t, hv);
     }
     // layer 3: dW3, dA2
     if (!(ok = tcRound(sm, bar, phase, [&] {
@@ -517,9 +565,9 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
     {
       uint16_t hv[H];
       getRow64(sm, TT_H2, t, hv);
-      backEpilogue(sm, tRow, hv, gb + H, t);
+      backEpilogue(sm, tRow, hv, gb2, t);
       getRow64(sm, TT_H1, t, hv);
-      putColumn(sm, TT_AT, t, hv, H);
+      putColumn<H>(sm, TT_AT, t, hv);
     }
     // layer 2: dW2, dA1
     if (!(ok = tcRound(sm, bar, phase, [&] {
@@ -530,11 +578,11 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
     {
       uint16_t hv[H];
       getRow64(sm, TT_H1, t, hv);
-      backEpilogue(sm, tRow, hv, gb, t);
+      backEpilogue(sm, tRow, hv, gb1, t);
       // X^T in rows 0..15 of the transposed operand, zeros over the rows of H1^T above them
       uint16_t xv[H];
       for (int k = 0; k < H; k++) xv[k] = k < 16 ? xb[k] : (uint16_t)0;
-      putColumn(sm, TT_AT, t, xv, H);
+      putColumn<H>(sm, TT_AT, t, xv);
     }
     // layer 1: dW1
     if (!(ok = tcRound(sm, bar, phase, [&] { tcIssue<TC_M, H>(sm, TT_AT, TT_DZT, tmem + TT_DW1, acc); }))) break;
@@ -548,23 +596,30 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
   // the CTA's sums into the global gradient: weight rows are TMEM lanes (inputs), columns the outputs
   if (ok && !first) {
     const int m = 32 * warp + (t & 31);  // this thread's input row
-    for (int c = 0; c < TC_N4; c += 16) {
-      float v[16];
-      tcLoad16(tmem + lane0 + TT_DW4 + c, v);
-      if (m < H)
-        for (int k = 0; k < 8; k++) if (v[k] != 0.f) atomicAdd(&grad[OFF_W4 + m * 8 + k], v[k]);
+    float v[16];
+    tcLoad16(tmem + lane0 + TT_DW4, v);
+    if (m < H) {
+      addGlobal4(grad + OFF_W4 + m * 8, v);  // columns 4..7 are padding
     }
     for (int c = 0; c < H; c += 16) {
       float v3[16], v2[16], v1[16];
       tcLoad16(tmem + lane0 + TT_DW3 + c, v3);
       tcLoad16(tmem + lane0 + TT_DW2 + c, v2);
       tcLoad16(tmem + lane0 + TT_DW1 + c, v1);
-      for (int k = 0; k < 16; k++) {
-        if (m < H && v3[k] != 0.f) atomicAdd(&grad[OFF_W3 + m * H + c + k], v3[k]);
-        if (m < H && v2[k] != 0.f) atomicAdd(&grad[OFF_W2 + m * H + c + k], v2[k]);
-        if (m < 16 && v1[k] != 0.f) atomicAdd(&grad[OFF_W1 + m * H + c + k], v1[k]);
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) {
+        if (m < H) addGlobal4(grad + OFF_W3 + m * H + c + k, v3 + k);
+        if (m < H) addGlobal4(grad + OFF_W2 + m * H + c + k, v2 + k);
+        if (m < 16) addGlobal4(grad + OFF_W1 + m * H + c + k, v1 + k);
       }
     }
+    // the warps' bias sums into the CTA's
+    const int lane = t & 31;
+    atomicAdd(&gb[lane], gb1[0]); atomicAdd(&gb[32 + lane], gb1[1]);
+    atomicAdd(&gb[H + lane], gb2[0]); atomicAdd(&gb[H + 32 + lane], gb2[1]);
+    atomicAdd(&gb[2 * H + lane], gb3[0]); atomicAdd(&gb[2 * H + 32 + lane], gb3[1]);
+    if (lane == 0)
+      for (int k = 0; k < ELL_TARGETS; k++) atomicAdd(&gb[3 * H + k], gb4[k]);
   }
   for (int o = 16; o > 0; o >>= 1) myLoss += __shfl_xor_sync(0xffffffffu, myLoss, o);
   if ((t & 31) == 0) atomicAdd(reinterpret_cast<float*>(sm + TT_LOSS), myLoss);

@@ -218,6 +218,8 @@ struct wdem_handle {
   // learned warm start: FP32 master weights (padded layout), BF16 copy, Adam moments, gradient
   float *mlpW = nullptr, *mlpM = nullptr, *mlpV = nullptr, *mlpGrad = nullptr, *mlpLoss = nullptr;
   uint16_t* mlpWbf = nullptr;
+  float* warmIO = nullptr;      // inputs and outputs of wdem_warm_predict / wdem_warm_grad
+  long long warmIOCap = 0;
   bool mlpReady = false;
   long long mlpT = 0;
   double* dStress = nullptr;    // 9 stress components + scratch for the terms
@@ -734,7 +736,7 @@ int wdem_destroy(wdem_handle* h) {
   cudaFree(d.fv1); cudaFree(d.fv2);
   cudaFree(h->ellLog); cudaFree(h->ellLogCount);
   cudaFree(h->dMatDt); cudaFree(h->cs.sceneWall);
-  cudaFree(h->mlpW); cudaFree(h->mlpM); cudaFree(h->mlpV); cudaFree(h->mlpGrad); cudaFree(h->mlpLoss); cudaFree(h->mlpWbf);
+  cudaFree(h->mlpW); cudaFree(h->mlpM); cudaFree(h->mlpV); cudaFree(h->mlpGrad); cudaFree(h->mlpLoss); cudaFree(h->mlpWbf); cudaFree(h->warmIO);
   cudaFree(d.posr); cudaFree(d.velm); cudaFree(d.angw); cudaFree(d.inert); cudaFree(d.ori);
   cudaFree(d.lastPos); cudaFree(d.bbmin); cudaFree(d.bbmax); cudaFree(d.force); cudaFree(d.torque); cudaFree(d.meta); cudaFree(d.posf); cudaFree(d.lastPosf); cudaFree(d.touched); cudaFree(d.rowMask); cudaFree(d.rotList); cudaFree(d.touchList);
   for (int k = 0; k < 3; k++) cudaFree(d.energy[k]);
@@ -2161,6 +2163,19 @@ int mlpEnsure(wdem_handle* h) {
   CK(cudaMemsetAsync(h->mlpGrad, 0, n * sizeof(float), h->stream));
   return WDEM_OK;
 }
+// device buffer of the network's inputs and outputs, kept from call to call up to WARM_IO_KEEP bytes (allocating and
+// freeing it took a third of a gradient call on 64k records); a larger call's buffer is given back by the next
+// smaller one
+const long long WARM_IO_KEEP = 256ll << 20;
+int ensureWarmIO(wdem_handle* h, long long floats) {
+  const bool tooLarge = h->warmIOCap * (long long)sizeof(float) > WARM_IO_KEEP && 2 * floats < h->warmIOCap;
+  if (floats > h->warmIOCap || tooLarge) {
+    h->warmIOCap = 0;
+    CK(dalloc(h->warmIO, (size_t)floats));
+    h->warmIOCap = floats;
+  }
+  return WDEM_OK;
+}
 int mlpUpload(wdem_handle* h, const std::vector<float>& pad) {
   const int n = mlp_npad();
   CK(cudaMemcpyAsync(h->mlpW, pad.data(), n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
@@ -2226,17 +2241,15 @@ int wdem_warm_predict(wdem_handle* h, const float* x, int64_t n, float* y) {
   if (!h->mlpReady) return fail(h, WDEM_ERR_STATE, "no warm-start network");
   if (n == 0) return WDEM_OK;
   CK(cudaSetDevice(h->device));
-  float *dx = nullptr, *dy = nullptr;
-  CK(dalloc(dx, (size_t)n * WDEM_WARM_INPUTS));
-  if (dalloc(dy, (size_t)n * WDEM_WARM_OUTPUTS) != cudaSuccess) { cudaFree(dx); return fail(h, WDEM_ERR_CUDA, "out of memory"); }
+  int rc;
+  if ((rc = ensureWarmIO(h, n * (WDEM_WARM_INPUTS + WDEM_WARM_OUTPUTS)))) return rc;
+  float *dx = h->warmIO, *dy = h->warmIO + (size_t)n * WDEM_WARM_INPUTS;
   cudaMemcpyAsync(dx, x, (size_t)n * WDEM_WARM_INPUTS * sizeof(float), cudaMemcpyHostToDevice, h->stream);
   mlp_launch_predict(h->stream, dx, n, dy, h->mlpWbf, h->mlpW, h->dst);
   cudaMemcpyAsync(y, dy, (size_t)n * WDEM_WARM_OUTPUTS * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
   cudaMemcpyAsync(h->hst, h->dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  cudaFree(dx); cudaFree(dy);
   if (e != cudaSuccess) return fail(h, WDEM_ERR_CUDA, cudaGetErrorString(e));
-  int rc;
   if ((rc = checkDeviceStatus(h))) return rc;
   return WDEM_OK;
 }
@@ -2245,8 +2258,9 @@ int wdem_warm_grad(wdem_handle* h, const float* records, int64_t n, float* grad,
   if (!h || !records || !grad || !loss || n <= 0) return WDEM_ERR_ARG;
   if (!h->mlpReady) return fail(h, WDEM_ERR_STATE, "no warm-start network");
   CK(cudaSetDevice(h->device));
-  float* dr = nullptr;
-  CK(dalloc(dr, (size_t)n * WDEM_WARM_RECORD));
+  int rc;
+  if ((rc = ensureWarmIO(h, n * WDEM_WARM_RECORD))) return rc;
+  float* dr = h->warmIO;
   cudaMemcpyAsync(dr, records, (size_t)n * WDEM_WARM_RECORD * sizeof(float), cudaMemcpyHostToDevice, h->stream);
   cudaMemsetAsync(h->mlpGrad, 0, mlp_npad() * sizeof(float), h->stream);
   cudaMemsetAsync(h->mlpLoss, 0, sizeof(float), h->stream);
@@ -2257,9 +2271,7 @@ int wdem_warm_grad(wdem_handle* h, const float* records, int64_t n, float* grad,
   cudaMemsetAsync(h->mlpGrad, 0, mlp_npad() * sizeof(float), h->stream);
   cudaMemcpyAsync(h->hst, h->dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
-  cudaFree(dr);
   if (e != cudaSuccess) return fail(h, WDEM_ERR_CUDA, cudaGetErrorString(e));
-  int rc;
   if ((rc = checkDeviceStatus(h))) return rc;
   mlp_pack(pad.data(), grad);
   return WDEM_OK;
