@@ -981,62 +981,76 @@ void launch_dyndt(cudaStream_t s, const StepParams& P, Particles p, int n, Conta
 // Rows up to REDUCE_ROW entries are summed by one thread.  A wall's row has an entry for every body near it, and
 // one thread walking it was the whole kernel (1167 us for the beds of 120k spheres, whose walls have 2,500
 // entries): such a row is taken by a warp, which loads 32 records at a time, packs the stamped ones into shared
-// memory in row order, and adds them with one lane per component, so the six sums keep the row's order.
+// memory in row order, and adds them with one lane per component, so the six sums keep the row's order.  A wall or
+// facet has a block of its own (the chain of additions of each wall is what remains; six of them after one another
+// in the block of their ids took 157 us), the long row of another body a warp of its block.
 static const int REDUCE_T = 128, REDUCE_ROW = 64;
-__global__ void __launch_bounds__(REDUCE_T) k_reduce_forces(StepParams P, Particles p, int n, Contacts c, Csr csr) {
+__device__ __forceinline__ void reduceRowWarp(const StepParams& P, const Particles& p, const Contacts& c, const Csr& csr, int r,
+                                              long long want, double (*packed)[6]) {
+  const int lane = threadIdx.x & 31;
+  const int e0 = csr.rowptr[r], e1 = csr.rowptr[r + 1];
+  double acc = 0.;  // lanes 0-2: force, 3-5: torque
+  const d3 g = gravityForce(P, p.velm[r].w, (unsigned)p.meta[r].w);
+  if (lane < 3) acc = comp(g, lane);
+  double4_32a f, t;
+  auto load = [&](int e) {
+    f.w = 0.;
+    if (e < e1) { f = c.out[OUT_RECORDS * (long long)e + OUT_F]; t = c.out[OUT_RECORDS * (long long)e + OUT_T]; }
+  };
+  load(e0 + lane);
+  for (int e = e0; e < e1; e += 32) {
+    const bool on = e + lane < e1 && __double_as_longlong(f.w) == want;
+    const unsigned b = __ballot_sync(0xffffffffu, on);
+    if (on) {
+      double* o = packed[__popc(b & ((1u << lane) - 1u))];
+      o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = t.x; o[4] = t.y; o[5] = t.z;
+    }
+    load(e + 32 + lane);  // the next 32 records arrive during the additions
+    __syncwarp();
+    const int m = __popc(b);
+    if (lane < 6)
+      for (int k = 0; k < m; k++) acc = acc + packed[k][lane];
+    __syncwarp();
+  }
+  if (lane < 6) (lane < 3 ? reinterpret_cast<double*>(&p.force[r]) : reinterpret_cast<double*>(&p.torque[r]) - 3)[lane] = acc;
+  if (lane == 6) p.force[r].w = 0.;
+  if (lane == 7) p.torque[r].w = 0.;
+}
+__global__ void __launch_bounds__(REDUCE_T) k_reduce_forces(StepParams P, Particles p, int n, Contacts c, Csr csr,
+                                                            const int* large, int nLarge) {
   __shared__ int longRow[REDUCE_T];
   __shared__ int nLong;
   __shared__ double packed[REDUCE_T / 32][32][6];
-  const int i = blockIdx.x * REDUCE_T + threadIdx.x;
+  const long long want = P.seq - 1;
+  const int w = threadIdx.x >> 5;
+  if (blockIdx.x < (unsigned)nLarge) {  // the long chains start first
+    if (w == 0) reduceRowWarp(P, p, c, csr, large[blockIdx.x], want, packed[0]);
+    return;
+  }
+  const int i = (blockIdx.x - nLarge) * REDUCE_T + threadIdx.x;
   if (threadIdx.x == 0) nLong = 0;
   __syncthreads();
-  const long long want = P.seq - 1;
   if (i < n) {
-    if (csr.rowptr[i + 1] - csr.rowptr[i] > REDUCE_ROW) longRow[atomicAdd(&nLong, 1)] = i;
+    const int4 meta = p.meta[i];
+    const int shape = meta.x & 15;
+    if (shape == WDEM_SHAPE_WALL || shape == WDEM_SHAPE_FACET) {
+      // in the large list
+    } else if (csr.rowptr[i + 1] - csr.rowptr[i] > REDUCE_ROW) longRow[atomicAdd(&nLong, 1)] = i;
     else {
-      d3 F = gravityForce(P, p.velm[i].w, (unsigned)p.meta[i].w), T = mk(0, 0, 0);
+      d3 F = gravityForce(P, p.velm[i].w, (unsigned)meta.w), T = mk(0, 0, 0);
       gatherRow(want, i, c, csr, F, T);
       p.force[i] = make_double4_32a(F.x, F.y, F.z, 0);
       p.torque[i] = make_double4_32a(T.x, T.y, T.z, 0);
     }
   }
   __syncthreads();
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int q = w; q < nLong; q += REDUCE_T / 32) {
-    const int r = longRow[q];
-    const int e0 = csr.rowptr[r], e1 = csr.rowptr[r + 1];
-    double acc = 0.;  // lanes 0-2: force, 3-5: torque
-    const d3 g = gravityForce(P, p.velm[r].w, (unsigned)p.meta[r].w);
-    if (lane < 3) acc = comp(g, lane);
-    double4_32a f, t;
-    auto load = [&](int e) {
-      f.w = 0.;  // stamp 0: no pass
-      if (e < e1) { f = c.out[OUT_RECORDS * (long long)e + OUT_F]; t = c.out[OUT_RECORDS * (long long)e + OUT_T]; }
-    };
-    load(e0 + lane);
-    for (int e = e0; e < e1; e += 32) {
-      const bool on = e + lane < e1 && __double_as_longlong(f.w) == want;
-      const unsigned b = __ballot_sync(0xffffffffu, on);
-      if (on) {
-        double* o = packed[w][__popc(b & ((1u << lane) - 1u))];
-        o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = t.x; o[4] = t.y; o[5] = t.z;
-      }
-      load(e + 32 + lane);  // the next 32 records arrive during the additions
-      __syncwarp();
-      const int m = __popc(b);
-      if (lane < 6)
-        for (int k = 0; k < m; k++) acc = acc + packed[w][k][lane];
-      __syncwarp();
-    }
-    if (lane < 6) (lane < 3 ? reinterpret_cast<double*>(&p.force[r]) : reinterpret_cast<double*>(&p.torque[r]) - 3)[lane] = acc;
-    if (lane == 6) p.force[r].w = 0.;
-    if (lane == 7) p.torque[r].w = 0.;
-  }
+  for (int q = w; q < nLong; q += REDUCE_T / 32) reduceRowWarp(P, p, c, csr, longRow[q], want, packed[w]);
 }
 
-void launch_reduce_forces(cudaStream_t s, const StepParams& P, Particles p, int n, Contacts c, Csr csr) {
+void launch_reduce_forces(cudaStream_t s, const StepParams& P, Particles p, int n, Contacts c, Csr csr, const int* large,
+                          int nLarge) {
   if (n <= 0) return;
-  (k_reduce_forces<<<(n + REDUCE_T - 1) / REDUCE_T, REDUCE_T, 0, s>>>(P, p, n, c, csr), ++::wdem::g_kernel_launches);
+  (k_reduce_forces<<<nLarge + (n + REDUCE_T - 1) / REDUCE_T, REDUCE_T, 0, s>>>(P, p, n, c, csr, large, nLarge), ++::wdem::g_kernel_launches);
 }
 
 WDEM_VARIANT_END

@@ -1493,7 +1493,7 @@ int wdem_download_particles(wdem_handle* h, wdem_particles* p) {
   if (!h->forcesInArrays) {
     StepParams P = h->P;
     P.seq = h->seq + 1;  // the records of the last contact pass
-    launch_reduce_forces(s, P, h->d, h->n, h->buf[h->cur].c, h->csr);
+    launch_reduce_forces(s, P, h->d, h->n, h->buf[h->cur].c, h->csr, h->cs.large, h->cs.nLarge);
   }
   std::vector<double4_32a> posr(n), velm(n), angw(n), ori(n), force(n), torque(n);
   if (n > 0) {
@@ -1811,7 +1811,7 @@ void materialiseForces(wdem_handle* h) {
   if (!h->forcesInArrays) {
     StepParams P = h->P;
     P.seq = h->seq + 1;  // the records of the last contact pass
-    launch_reduce_forces(h->stream, P, h->d, h->n, h->buf[h->cur].c, h->csr);
+    launch_reduce_forces(h->stream, P, h->d, h->n, h->buf[h->cur].c, h->csr, h->cs.large, h->cs.nLarge);
     h->forcesInArrays = true;
   }
 }

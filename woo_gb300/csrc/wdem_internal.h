@@ -288,7 +288,9 @@ __device__ __forceinline__ bool haltedContacts(const DeviceStatus* st, long long
 // ---- launchers (k_leapfrog.cu) ----
 void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, int fromArrays,
                      Contacts c, Csr csr, DeviceStatus* st);
-void launch_reduce_forces(cudaStream_t s, const StepParams& P, Particles p, int n, Contacts c, Csr csr);
+// large, nLarge: the walls and facets
+void launch_reduce_forces(cudaStream_t s, const StepParams& P, Particles p, int n, Contacts c, Csr csr, const int* large,
+                          int nLarge);
 // DynDt: the smallest nodal critical step^2 into st->dynNotMin (as ~bits; cleared by the caller)
 void launch_dyndt(cudaStream_t s, const StepParams& P, Particles p, int n, Contacts c, Csr csr, DeviceStatus* st);
 void launch_state_in(cudaStream_t s, Particles p, int n, const double* pos, const double* vel, const double* angVel,
