@@ -1248,37 +1248,49 @@ __device__ __forceinline__ bool cullOne(const StepParams& P, const Particles& p,
   return (s1 & CS_MASK) != CS_DEAD && (s1 & CS_SHAPES) != (CS_WALL_A | CS_WALL_B) && !(s1 & CS_FAR);
 }
 
-// warp-aggregated appends: the work list (real contacts from the front, potential pairs from the back)
-// and, in the full pass, the active list
-__device__ __forceinline__ void cullAppend(unsigned* work, unsigned* count, long long nc, long long i, bool need,
-                                           bool realNow, unsigned* act, unsigned* actCount, bool active) {
-  const int lane = threadIdx.x & 31;
+// Block-aggregated appends: the work list (real contacts from the front, potential pairs from the back) and, in the
+// full pass, the active list.  One atomic per list and block: with one per warp, the tens of thousands on one counter
+// were half of the pass over the 1.4 M pairs of 1M falling spheres.  Two barriers an append; the shared words
+// alternate, so the next append needs no third.
+template <int BS, bool FULL>
+struct CullAppend {
+  static const int NW = BS / 32, LISTS = FULL ? 3 : 2;
+  unsigned cnt[2][LISTS][NW], base[2][LISTS];
+};
+template <int BS, bool FULL>
+__device__ __forceinline__ void cullAppend(CullAppend<BS, FULL>& sh, int turn, unsigned* work, unsigned* count, long long nc,
+                                           long long i, bool need, bool realNow, unsigned* act, unsigned* actCount,
+                                           bool active) {
+  typedef CullAppend<BS, FULL> S;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1;
-  const unsigned bReal = __ballot_sync(0xffffffffu, need && realNow);
-  const unsigned bPot = __ballot_sync(0xffffffffu, need && !realNow);
-  if (bReal) {
-    const int leader = __ffs(bReal) - 1;
-    unsigned base = 0;
-    if (lane == leader) base = atomicAdd(&count[0], (unsigned)__popc(bReal));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (need && realNow) work[base + __popc(bReal & below)] = (unsigned)i;
+  const bool in[3] = {need && realNow, need && !realNow, active};
+  unsigned b[S::LISTS];
+#pragma unroll
+  for (int k = 0; k < S::LISTS; k++) {
+    b[k] = __ballot_sync(0xffffffffu, in[k]);
+    if (lane == 0) sh.cnt[turn][k][w] = (unsigned)__popc(b[k]);
   }
-  if (bPot) {
-    const int leader = __ffs(bPot) - 1;
-    unsigned base = 0;
-    if (lane == leader) base = atomicAdd(&count[1], (unsigned)__popc(bPot));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (need && !realNow) work[nc - 1 - (base + __popc(bPot & below))] = (unsigned)i;
-  }
-  if (act) {
-    const unsigned bAct = __ballot_sync(0xffffffffu, active);
-    if (bAct) {
-      const int leader = __ffs(bAct) - 1;
-      unsigned base = 0;
-      if (lane == leader) base = atomicAdd(actCount, (unsigned)__popc(bAct));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (active) act[base + __popc(bAct & below)] = (unsigned)i;
+  __syncthreads();
+  if (threadIdx.x < S::LISTS) {
+    unsigned sum = 0;
+#pragma unroll
+    for (int q = 0; q < S::NW; q++) {
+      const unsigned c = sh.cnt[turn][threadIdx.x][q];
+      sh.cnt[turn][threadIdx.x][q] = sum;
+      sum += c;
     }
+    unsigned* to = threadIdx.x < 2 ? &count[threadIdx.x] : actCount;
+    sh.base[turn][threadIdx.x] = sum ? atomicAdd(to, sum) : 0u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < S::LISTS; k++) {
+    if (!in[k]) continue;
+    const unsigned at = sh.base[turn][k] + sh.cnt[turn][k][w] + (unsigned)__popc(b[k] & below);
+    if (k == 0) work[at] = (unsigned)i;
+    else if (k == 1) work[nc - 1 - at] = (unsigned)i;
+    else act[at] = (unsigned)i;
   }
 }
 
@@ -1299,13 +1311,15 @@ __global__ void __launch_bounds__(BS) k_contacts_cull(StepParams P, Particles p,
   if (haltedContacts(st, stepOf(P, st))) return;
   // the integrator's lists of this step have been consumed: their counters start the next step at 0
   if (first + threadIdx.x == 0) { st->rotCount = 0; st->touchCount = 0; }
+  __shared__ CullAppend<BS, FULL> sh;
   const long long stride = FULL ? m + 1 : (long long)gridDim.x * blockDim.x;
-  for (long long base = first; base < m; base += stride) {
+  int turn = 0;
+  for (long long base = first; base < m; base += stride, turn ^= 1) {  // the same rounds for the whole block
     const long long k = base + threadIdx.x;
     const long long i = k < m ? (FULL ? k : (long long)c.act[k]) : -1;
     bool need = false, realNow = false, active = false;
     if (i >= 0) active = cullOne<PERI, ELL>(P, p, c, nc, i, c.state[i], st, need, realNow);
-    cullAppend(work, count, nc, i, need, realNow, FULL ? c.act : nullptr, &st->actCount, active && FULL);
+    cullAppend<BS, FULL>(sh, turn, work, count, nc, i, need, realNow, c.act, &st->actCount, active && FULL);
   }
 }
 

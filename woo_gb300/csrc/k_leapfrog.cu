@@ -657,8 +657,11 @@ __device__ __forceinline__ bool spinFast(const StepParams& P, const Particles& p
   return rotate;
 }
 
-// A node without contact forces, in the first pass: untouched spinning spheres go to the rotation list of the
-// second pass (they are scattered over most warps, whose FP64 pipe would wait for their few spinning lanes).
+// A node without contact forces, in the first pass.  Spinning spheres of a warp that has ROTATE_HERE of them or more
+// are turned here, while the pass waits for memory; fewer go to the rotation list of the second pass (scattered over
+// most warps they would each cost their warp the FP64 time of 32).  1M falling, spinning spheres: first and second
+// pass 47 + 141 us a step with all of them listed (one atomic a warp on one counter), see k_leapfrog_lists for now.
+static const int ROTATE_HERE = 16;
 template <bool PERI>
 __device__ __forceinline__ void integrateFast(const StepParams& P, const Particles& p, const int i, const int n,
                                               DeviceStatus* st, const FastRec& rec) {
@@ -666,7 +669,8 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
   const bool rotate = spinFast<PERI>(P, p, i, rec.meta, rec.w4, mk(0, 0, 0), nullptr, angVel);
   const unsigned am = __activemask();
   const unsigned b = __ballot_sync(am, rotate);
-  if (b) {
+  const bool here = __popc(b) >= ROTATE_HERE;
+  if (b != 0 && !here) {
     const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
     unsigned base = 0;
     if (lane == leader) base = atomicAdd(&st->rotCount, (unsigned)__popc(b));
@@ -674,7 +678,10 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
     const unsigned slot = base + __popc(b & ((1u << lane) - 1));
     if (rotate && slot < (unsigned)n) p.rotList[slot] = (unsigned)i;
   }
+  double4_32a o4;
+  if (here && rotate) o4 = p.ori[i];
   translateFast<PERI>(P, p, i, st, false, rec, mk(0, 0, 0));
+  if (here && rotate) rotateSphere(P, p, (unsigned)i, o4, angVel, rec.meta.y);
 }
 
 // First pass: particles without contact forces this step.  Those that a real contact touched are
