@@ -1215,8 +1215,7 @@ __device__ __forceinline__ bool cullOne(const StepParams& P, const Particles& p,
           // FP32 image shift; its rounding is bounded by 2^-23 x sum |h_ij cellDist_j|, added to the margin
           const int4 cd = c.cdist[i];
           const float c0 = (float)cd.x, c1 = (float)cd.y, c2 = (float)cd.z;
-          const float h[9] = {(float)P.hS[0], (float)P.hS[1], (float)P.hS[2], (float)P.hS[3], (float)P.hS[4],
-                              (float)P.hS[5], (float)P.hS[6], (float)P.hS[7], (float)P.hS[8]};
+          const float* h = P.hSF;
           fb.x += h[0] * c0 + h[1] * c1 + h[2] * c2;
           fb.y += h[3] * c0 + h[4] * c1 + h[5] * c2;
           fb.z += h[6] * c0 + h[7] * c1 + h[8] * c2;
@@ -1314,12 +1313,15 @@ __global__ void __launch_bounds__(BS) k_contacts_cull(StepParams P, Particles p,
   __shared__ CullAppend<BS, FULL> sh;
   const long long stride = FULL ? m + 1 : (long long)gridDim.x * blockDim.x;
   int turn = 0;
-  for (long long base = first; base < m; base += stride, turn ^= 1) {  // the same rounds for the whole block
+  for (long long base = first; base < m; base += stride) {  // the same rounds for the whole block
     const long long k = base + threadIdx.x;
     const long long i = k < m ? (FULL ? k : (long long)c.act[k]) : -1;
     bool need = false, realNow = false, active = false;
     if (i >= 0) active = cullOne<PERI, ELL>(P, p, c, nc, i, c.state[i], st, need, realNow);
-    cullAppend<BS, FULL>(sh, turn, work, count, nc, i, need, realNow, c.act, &st->actCount, active && FULL);
+    if (__syncthreads_or(need || (FULL && active))) {
+      cullAppend<BS, FULL>(sh, turn, work, count, nc, i, need, realNow, c.act, &st->actCount, active && FULL);
+      turn ^= 1;
+    }
   }
 }
 
@@ -1329,8 +1331,9 @@ static void launchCull(cudaStream_t s, const StepParams& P, Particles p, Contact
                        DeviceStatus* st, bool full) {
   const int bs = P.shCullBlock == 128 || P.shCullBlock == 512 ? P.shCullBlock : 256;
   const long long sms = P.numSMs > 0 ? P.numSMs : 152;
-  // full pass: a thread per contact; list pass: a grid-stride walk of the active list (2048 threads an SM)
-  const unsigned cb = full ? (unsigned)((nc + bs - 1) / bs) : (unsigned)std::min<long long>((nc + bs - 1) / bs, sms * (2048 / bs));
+  // full pass: a thread per contact; list pass: a walk of the active list by two waves of 2048 threads an SM (2 M pairs
+  // that need nothing: 63.3 us a step with two, 65.1 with one, 63.9 with four; 508k batched: 3.72, 3.76, 3.75 ms a pass)
+  const unsigned cb = full ? (unsigned)((nc + bs - 1) / bs) : (unsigned)std::min<long long>((nc + bs - 1) / bs, 2 * sms * (2048 / bs));
 #define WDEM_CULL(BS_)                                                                                              \
   (full ? k_contacts_cull<PERI, ELL, true, BS_> : k_contacts_cull<PERI, ELL, false, BS_>)<<<cb, BS_, 0, s>>>(      \
       P, p, c, nc, c.work, count, st)

@@ -678,10 +678,8 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
     const unsigned slot = base + __popc(b & ((1u << lane) - 1));
     if (rotate && slot < (unsigned)n) p.rotList[slot] = (unsigned)i;
   }
-  double4_32a o4;
-  if (here && rotate) o4 = p.ori[i];
+  if (here && rotate) rotateSphere(P, p, (unsigned)i, p.ori[i], angVel, rec.meta.y);
   translateFast<PERI>(P, p, i, st, false, rec, mk(0, 0, 0));
-  if (here && rotate) rotateSphere(P, p, (unsigned)i, o4, angVel, rec.meta.y);
 }
 
 // First pass: particles without contact forces this step.  Those that a real contact touched are

@@ -611,6 +611,7 @@ void fillCellParams(wdem_handle* h) {
   const HostCell& c = h->cell;
   const double dt = P.dt;
   put9(P.hS, c.hSize);
+  for (int k = 0; k < 9; k++) P.hSF[k] = (float)P.hS[k];
   put9(P.shv, mul(c.gradV, c.pprevHsize));
   put9(P.unsh, c.unshearTrsf);
   for (int k = 0; k < 3; k++) { P.csize[k] = c.size[k]; P.sae[k] = 1 / c.cos[k] - 1; P.spinVec[k] = c.spinVec[k]; }

@@ -139,6 +139,7 @@ struct StepParams {
   int periodic;
   int hasShear;
   double hS[9];        // Cell.hSize: Contact shift = hSize * cellDist
+  float hSF[9];        // its FP32 copy (contact cull)
   double shv[9];       // Cell.gradV * Cell.pprevHsize: shift velocity = shv * cellDist
   double unsh[9];      // Cell unshear transformation (box centres)
   double csize[3];     // cell lengths (periodic collider)
