@@ -212,8 +212,9 @@ __device__ __forceinline__ d3 mvec(const double* m, d3 v) {
 struct qd { double w, x, y, z; };
 
 // x * 0.5 and x + x on the integer pipe (the exponent moved by one: exact while the result is normal);
-// subnormal results, overflows, infinities and NaN take the FP64 operation.  An FP64 instruction holds the
-// pipe for 16 cycles a warp on GB300, these few integer ones for about 2.
+// subnormal results, overflows, infinities and NaN take the FP64 operation.  An FP64 instruction holds a
+// scheduler's pipe for 64 cycles on GB300 however many lanes of the warp are active (measured: 64.4 cycles a DFMA
+// with 32, 16, 8, 4, 2 and 1 lanes, and as much latency), an integer one for 1 or 2.
 __device__ __forceinline__ double halfOf(double x) {
   const Halves h = halvesOf(x);
   const unsigned e = h.hi & 0x7ff00000u;
