@@ -764,10 +764,8 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
           if (P.trackEnergy) ePl = (kt != 0. ? (maxFt) * (FtNorm - maxFt) / kt : 0.);
           fy *= ratio; fz *= ratio;
         }
-        // Eigen maxCoeff = maxi(maxi(f0,f1),f2) with maxi(a,b) = a<b ? b : a
-        double m01 = (fx < fy) ? fy : fx;
-        double mm = (m01 < fz) ? fz : m01;
-        if (nanBits(mm)) { if (atomicCAS(&st->code, 0, WDEM_ERR_NAN) == 0) st->detail = a; }
+        // Eigen maxCoeff = maxi(maxi(f0,f1),f2) with maxi(a,b) = a<b ? b : a is NaN exactly when f0 is
+        if (nanBits(fx)) { if (atomicCAS(&st->code, 0, WDEM_ERR_NAN) == 0) st->detail = a; }
       }
       if (P.trackEnergy) {
         const double el = 0.5 * (fx * fx / kn + (kt != 0. ? (fy * fy + fz * fz) / kt : 0.));
@@ -817,7 +815,7 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
       double sc = dt * kt;
       fy = fy + sc * gvel.y;
       fz = fz + sc * gvel.z;
-      double maxFt = fabs(dmin(0., fx) * tanPhi);
+      double maxFt = fabs((negativeBits(fx) ? fx : 0.) * tanPhi);
       double ftSq = fy * fy + fz * fz;
       if (ftSq > maxFt * maxFt) {
 #ifdef WDEM_FMA
@@ -1080,17 +1078,17 @@ __device__ __forceinline__ void contactBodyDW(const StepParams& P, const Particl
       // the normal force in FP64 as in the contracted FP64 body: near equilibrium the elastic and adhesive
       // terms cancel, and the sum must carry no more than the overlap's relative error
       const double velN = dwToD(gvel.x);
-      const double sq = sqrt(dmax(-uN, 0.));
+      const double sq = SQRT(-uN);
       knD = (3 / 2.) * kn0 * sq;
       const double Fne = -kn0 * pown3(sq);
       const double Fna = c.hist[HIST_E3][i];
       const double hz2 = c.hist[HIST_E2][i];
-      const double etaD = positiveBits(hz2) ? hz2 * sqrt(sq) : 0.;
+      const double etaD = positiveBits(hz2) ? hz2 * SQRT(sq) : 0.;
       double Fnv = etaD * velN;
       if (P.noAttraction && hertzAlphaZero(P, p, a, b) && positiveBits(Fne + Fnv)) Fnv = -Fne;
       fx = dwFrom(Fne + Fna + Fnv);
       const dwf eta = dwFrom(etaD);
-      ktD = c.hist[HIST_E1][i] * sq;
+      ktD = c.hist[HIST_E1][i] * (negativeBits(uN) ? sq : 0.);
       const dwf sc = dwFrom(dtC * ktD);
       fy = dwAdd(fy, dwMul(sc, gvel.y));
       fz = dwAdd(fz, dwMul(sc, gvel.z));

@@ -158,6 +158,13 @@ __device__ __forceinline__ bool sameBits(double a, double b) { const Halves x = 
 // |x| < bound, a positive finite constant whose low 32 bits are ignored (a switch between two formulas)
 __device__ __forceinline__ bool belowHi(double x, double bound) { return (halvesOf(x).hi & 0x7fffffffu) < halvesOf(bound).hi; }
 __device__ __forceinline__ bool finiteBits(double x) { return (halvesOf(x).hi & 0x7ff00000u) != 0x7ff00000u; }
+// a > b for numbers that are not NaN (a NaN compares as a value beyond infinity): the bit patterns as signed
+// integers, those of negative numbers reversed, -0 taken as +0
+__device__ __forceinline__ long long orderedBits(double x) {
+  const long long b = (long long)bitsOf(x);
+  return b >= 0 ? b : (long long)(0x8000000000000000ull - (unsigned long long)b);
+}
+__device__ __forceinline__ bool greaterBits(double a, double b) { return orderedBits(a) > orderedBits(b); }
 // a * b for finite a and b == +-0: the zero with the product's sign
 __device__ __forceinline__ double signedZero(double a, double b) {
   return fromHalves(0u, (halvesOf(a).hi ^ halvesOf(b).hi) & 0x80000000u);
@@ -256,10 +263,10 @@ __device__ __forceinline__ qd quatFromCols(d3 c0, d3 c1, d3 c2) {
   const double m01 = c1.x, m11 = c1.y, m21 = c1.z;
   const double m02 = c2.x, m12 = c2.y, m22 = c2.z;
   const double tr = m00 + m11 + m22;
-  const bool pos = tr > 0;
+  const bool pos = positiveBits(tr);
   // largest diagonal element i, j = i+1, k = j+1 (mod 3)
-  const bool b1 = m11 > m00;
-  const bool i2 = m22 > pick(b1, m11, m00);
+  const bool b1 = greaterBits(m11, m00);
+  const bool i2 = greaterBits(m22, pick(b1, m11, m00));
   const bool i1 = b1 && !i2, i0 = !b1 && !i2;
   const double mi = pick(i0, m00, pick(i1, m11, m22)), mj = pick(i0, m11, pick(i1, m22, m00)),
                mk_ = pick(i0, m22, pick(i1, m00, m11));
