@@ -1151,6 +1151,7 @@ template <int LAW, int CP2, bool PERI, bool ELL, int BS, bool DW = false>
 __global__ void __launch_bounds__(BS, 512 / BS) k_contacts(StepParams P, Particles p, Contacts c, const unsigned* work,
                                                         const unsigned* count, long long nc, DeviceStatus* st,
                                                         int part) {
+  chainWait(P.chainEarly);
   // part 0: the whole work list; 1: the real contacts at its front; 2: the potential pairs behind them
   const unsigned k0 = part == 2 ? count[0] : 0u;
   const unsigned m = part == 1 ? count[0] : workLen(count);
@@ -1302,6 +1303,7 @@ __device__ __forceinline__ void cullAppend(CullAppend<BS, FULL>& sh, int turn, u
 template <bool PERI, bool ELL, bool FULL, int BS>
 __global__ void __launch_bounds__(BS) k_contacts_cull(StepParams P, Particles p, Contacts c, long long nc,
                                                        unsigned* work, unsigned* count, DeviceStatus* st) {
+  chainWait(P.chainEarly);
   const long long first = (long long)blockIdx.x * blockDim.x;
   const long long m = FULL ? nc : (long long)st->actCount;
   // a step queued behind a collider trigger: the work list stays empty, so the heavy pass is a no-op too
@@ -1333,13 +1335,12 @@ static void launchCull(cudaStream_t s, const StepParams& P, Particles p, Contact
   // that need nothing: 63.3 us a step with two, 65.1 with one, 63.9 with four; 508k batched: 3.72, 3.76, 3.75 ms a pass)
   const unsigned cb = full ? (unsigned)((nc + bs - 1) / bs) : (unsigned)std::min<long long>((nc + bs - 1) / bs, 2 * sms * (2048 / bs));
 #define WDEM_CULL(BS_)                                                                                              \
-  (full ? k_contacts_cull<PERI, ELL, true, BS_> : k_contacts_cull<PERI, ELL, false, BS_>)<<<cb, BS_, 0, s>>>(      \
-      P, p, c, nc, c.work, count, st)
+  launchChained(full ? k_contacts_cull<PERI, ELL, true, BS_> : k_contacts_cull<PERI, ELL, false, BS_>, cb, BS_, s, P, p, \
+                c, nc, c.work, count, st)
   if (bs == 128) WDEM_CULL(128);
   else if (bs == 512) WDEM_CULL(512);
   else WDEM_CULL(256);
 #undef WDEM_CULL
-  ++::wdem::g_kernel_launches;
 }
 #ifdef WDEM_FMA
 // the double-word law applies to the whole pass: no facets, no energy tracking, no updatePhys, no approxMask,
@@ -1363,17 +1364,15 @@ static void launchHeavy(cudaStream_t s, const StepParams& P, Particles p, Contac
 #ifdef WDEM_FMA
   if (!ELL && dwEligible<LAW>(P)) {
     // the double-word law for the real contacts, then the FP64 kernel for the potential pairs
-    if (bs == 64) k_contacts<LAW, CP2, PERI, false, 64, true><<<hb, 64, 0, s>>>(P, p, c, c.work, count, nc, st, 1);
-    else if (bs == 256) k_contacts<LAW, CP2, PERI, false, 256, true><<<hb, 256, 0, s>>>(P, p, c, c.work, count, nc, st, 1);
-    else k_contacts<LAW, CP2, PERI, false, 128, true><<<hb, 128, 0, s>>>(P, p, c, c.work, count, nc, st, 1);
-    ++::wdem::g_kernel_launches;
+    if (bs == 64) launchChained(k_contacts<LAW, CP2, PERI, false, 64, true>, hb, 64, s, P, p, c, c.work, count, nc, st, 1);
+    else if (bs == 256) launchChained(k_contacts<LAW, CP2, PERI, false, 256, true>, hb, 256, s, P, p, c, c.work, count, nc, st, 1);
+    else launchChained(k_contacts<LAW, CP2, PERI, false, 128, true>, hb, 128, s, P, p, c, c.work, count, nc, st, 1);
     part = 2;
   }
 #endif
-  if (bs == 64) k_contacts<LAW, CP2, PERI, ELL, 64><<<hb, 64, 0, s>>>(P, p, c, c.work, count, nc, st, part);
-  else if (bs == 256) k_contacts<LAW, CP2, PERI, ELL, 256><<<hb, 256, 0, s>>>(P, p, c, c.work, count, nc, st, part);
-  else k_contacts<LAW, CP2, PERI, ELL, 128><<<hb, 128, 0, s>>>(P, p, c, c.work, count, nc, st, part);
-  ++::wdem::g_kernel_launches;
+  if (bs == 64) launchChained(k_contacts<LAW, CP2, PERI, ELL, 64>, hb, 64, s, P, p, c, c.work, count, nc, st, part);
+  else if (bs == 256) launchChained(k_contacts<LAW, CP2, PERI, ELL, 256>, hb, 256, s, P, p, c, c.work, count, nc, st, part);
+  else launchChained(k_contacts<LAW, CP2, PERI, ELL, 128>, hb, 128, s, P, p, c, c.work, count, nc, st, part);
 }
 
 void launch_contacts(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc, DeviceStatus* st,

@@ -233,6 +233,7 @@ __device__ __forceinline__ void rotateSphere(const StepParams& P, const Particle
 template <bool FROM_ARRAYS, bool PERI, bool ELL>
 __global__ void __launch_bounds__(256) k_leapfrog(StepParams P, Particles p, int n, Contacts c, Csr csr, DeviceStatus* st) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  chainWait(true);
   const long long step = stepOf(P, st);
   if (i >= n || haltedIntegrator(st, step)) return;
   if (i == 0) clearWork(st);
@@ -690,6 +691,7 @@ __device__ __forceinline__ void integrateFast(const StepParams& P, const Particl
 template <bool PERI, int BS, bool DENSE>
 __global__ void __launch_bounds__(BS, 1024 / BS) k_leapfrog_fast(StepParams P, Particles p, int n, Contacts c, Csr csr,
                                                                DeviceStatus* st) {
+  chainWait(true);
   if constexpr (!DENSE) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -795,6 +797,7 @@ __device__ __forceinline__ void integrateTouched(const StepParams& P, const Part
 template <bool PERI>
 __global__ void __launch_bounds__(LIST_T) k_leapfrog_lists(StepParams P, Particles p, int n, Contacts c, Csr csr,
                                                             DeviceStatus* st) {
+  chainWait(true);
   if (haltedIntegrator(st, stepOf(P, st))) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) clearWork(st);
   const unsigned nt = st->touchCount < (unsigned)n ? st->touchCount : (unsigned)n;
@@ -838,6 +841,7 @@ __global__ void __launch_bounds__(LIST_T) k_leapfrog_all(StepParams P, Particles
   const bool turns = threadIdx.x >= LIST_ITEMS;
   const int i = blockIdx.x * LIST_ITEMS + (threadIdx.x & (LIST_ITEMS - 1));
   const bool live = i < n;
+  chainWait(true);
   int4 meta = make_int4(0, 0, 0, 63);
   unsigned mask = 0;
   uint8_t tch = 0;
@@ -881,15 +885,14 @@ static void launchFast(cudaStream_t s, const StepParams& P, Particles p, int n, 
   const int bs = P.shLeapBlock == 128 || P.shLeapBlock == 512 ? P.shLeapBlock : 256;
   const unsigned blocks = (unsigned)((n + bs - 1) / bs);
   if (P.denseTouch) {
-    if (bs == 128) k_leapfrog_fast<PERI, 128, true><<<blocks, 128, 0, s>>>(P, p, n, c, csr, st);
-    else if (bs == 512) k_leapfrog_fast<PERI, 512, true><<<blocks, 512, 0, s>>>(P, p, n, c, csr, st);
-    else k_leapfrog_fast<PERI, 256, true><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st);
+    if (bs == 128) launchChained(k_leapfrog_fast<PERI, 128, true>, blocks, 128, s, P, p, n, c, csr, st);
+    else if (bs == 512) launchChained(k_leapfrog_fast<PERI, 512, true>, blocks, 512, s, P, p, n, c, csr, st);
+    else launchChained(k_leapfrog_fast<PERI, 256, true>, blocks, 256, s, P, p, n, c, csr, st);
   } else {
-    if (bs == 128) k_leapfrog_fast<PERI, 128, false><<<blocks, 128, 0, s>>>(P, p, n, c, csr, st);
-    else if (bs == 512) k_leapfrog_fast<PERI, 512, false><<<blocks, 512, 0, s>>>(P, p, n, c, csr, st);
-    else k_leapfrog_fast<PERI, 256, false><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st);
+    if (bs == 128) launchChained(k_leapfrog_fast<PERI, 128, false>, blocks, 128, s, P, p, n, c, csr, st);
+    else if (bs == 512) launchChained(k_leapfrog_fast<PERI, 512, false>, blocks, 512, s, P, p, n, c, csr, st);
+    else launchChained(k_leapfrog_fast<PERI, 256, false>, blocks, 256, s, P, p, n, c, csr, st);
   }
-  ++::wdem::g_kernel_launches;
 }
 
 void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, int fromArrays, Contacts c, Csr csr,
@@ -900,9 +903,8 @@ void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, in
   if (!fromArrays && !P.hasEll && !P.lfEnergy) {
     const int sms = P.numSMs > 0 ? P.numSMs : 152;
     if (n <= ALL_PER_SM * sms) {
-      if (P.periodic) k_leapfrog_all<true><<<listBlocks, LIST_T, 0, s>>>(P, p, n, c, csr, st);
-      else k_leapfrog_all<false><<<listBlocks, LIST_T, 0, s>>>(P, p, n, c, csr, st);
-      ++::wdem::g_kernel_launches;
+      if (P.periodic) launchChained(k_leapfrog_all<true>, listBlocks, LIST_T, s, P, p, n, c, csr, st);
+      else launchChained(k_leapfrog_all<false>, listBlocks, LIST_T, s, P, p, n, c, csr, st);
       return;
     }
     // st->rotCount and st->touchCount are zero here: k_contacts_cull clears them for the next step (and
@@ -910,23 +912,23 @@ void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, in
     if (P.periodic) {
       const unsigned rb = std::min(listBlocks, listGrid<true>(P));
       launchFast<true>(s, P, p, n, c, csr, st);
-      (k_leapfrog_lists<true><<<rb, LIST_T, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+      launchChained(k_leapfrog_lists<true>, rb, LIST_T, s, P, p, n, c, csr, st);
     } else {
       const unsigned rb = std::min(listBlocks, listGrid<false>(P));
       launchFast<false>(s, P, p, n, c, csr, st);
-      (k_leapfrog_lists<false><<<rb, LIST_T, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+      launchChained(k_leapfrog_lists<false>, rb, LIST_T, s, P, p, n, c, csr, st);
     }
     return;
   }
   if (P.hasEll) {
-    if (fromArrays) (k_leapfrog<true, false, true><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
-    else (k_leapfrog<false, false, true><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+    if (fromArrays) launchChained(k_leapfrog<true, false, true>, blocks, 256, s, P, p, n, c, csr, st);
+    else launchChained(k_leapfrog<false, false, true>, blocks, 256, s, P, p, n, c, csr, st);
   } else if (P.periodic) {
-    if (fromArrays) (k_leapfrog<true, true, false><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
-    else (k_leapfrog<false, true, false><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+    if (fromArrays) launchChained(k_leapfrog<true, true, false>, blocks, 256, s, P, p, n, c, csr, st);
+    else launchChained(k_leapfrog<false, true, false>, blocks, 256, s, P, p, n, c, csr, st);
   } else {
-    if (fromArrays) (k_leapfrog<true, false, false><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
-    else (k_leapfrog<false, false, false><<<blocks, 256, 0, s>>>(P, p, n, c, csr, st), ++::wdem::g_kernel_launches);
+    if (fromArrays) launchChained(k_leapfrog<true, false, false>, blocks, 256, s, P, p, n, c, csr, st);
+    else launchChained(k_leapfrog<false, false, false>, blocks, 256, s, P, p, n, c, csr, st);
   }
 }
 
@@ -1189,6 +1191,7 @@ __global__ void __launch_bounds__(ER_T) k_sums(StepParams P, SumSet S, int row0,
   __shared__ double sh[ER_T];
   __shared__ bool last;
   const int y = row0 + blockIdx.y;
+  chainWait(P.chainEarly);
   if (S.guarded && (y < S.contactRow ? haltedIntegrator(st, stepOf(P, st)) : haltedContacts(st, stepOf(P, st)))) return;
   const long long n = S.n[y], nb = (n + ER_SLICE - 1) / ER_SLICE, blocks = nb > 0 ? nb : 1;
   if ((long long)blockIdx.x >= blocks) return;
@@ -1219,7 +1222,7 @@ __global__ void __launch_bounds__(ER_T) k_sums(StepParams P, SumSet S, int row0,
 void launch_sums(cudaStream_t s, const StepParams& P, const SumSet& S, int row0, int rows, double* partials, DeviceStatus* st) {
   long long nb = 1;
   for (int y = row0; y < row0 + rows; y++) nb = std::max(nb, sum_blocks(S.n[y]));
-  (k_sums<<<dim3((unsigned)nb, (unsigned)rows), ER_T, 0, s>>>(P, S, row0, nb, partials, st->sumTickets, st), ++::wdem::g_kernel_launches);
+  launchChained(k_sums, dim3((unsigned)nb, (unsigned)rows), ER_T, s, P, S, row0, nb, partials, st->sumTickets, st);
 }
 
 WDEM_VARIANT_END
