@@ -33,6 +33,7 @@ static const int SWEEP_MAX_COLS = (1 << 20) - 2;
 // Bo1_Sphere_Aabb::go / Bo1_Wall_Aabb::go + AabbCollider::updateAabb: pos +- bboxFactor*r,
 // walls unbounded except along their axis; both enlarged by verletDist; nodeLastPos = pos.
 __global__ void k_bboxes(StepParams P, Particles p, int n) {
+  chainWait(false);
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double4_32a pr = p.posr[i];
@@ -136,7 +137,7 @@ __global__ void k_bboxes(StepParams P, Particles p, int n) {
 
 void launch_bboxes(cudaStream_t s, const StepParams& P, Particles p, int n) {
   if (n <= 0) return;
-  (k_bboxes<<<(n + 255) / 256, 256, 0, s>>>(P, p, n), ++::wdem::g_kernel_launches);
+  launchChained(k_bboxes, (n + 255) / 256, 256, s, P, p, n);
 }
 
 // ------------------------------------------------------------------------------------ grid setup
@@ -260,6 +261,7 @@ struct GridArgs {
 static const int EXT_T = 256;
 __global__ void __launch_bounds__(EXT_T) k_extents(StepParams P, Particles p, const int* small, int nSmall,
                                                    unsigned long long* ext, GridArgs A) {
+  chainWait(false);
   __shared__ unsigned long long sh[EXT_VALUES];
   __shared__ bool last;
   if (threadIdx.x < EXT_VALUES) sh[threadIdx.x] = ~0ull;
@@ -320,6 +322,7 @@ __device__ __forceinline__ void columnOf(const double4_32a& pr, const GridParams
 // sweep key of each small body (column, quantised lower bound) and its place in its bucket
 __global__ void k_make_keys(Particles p, const int* small, int nSmall, const GridParams* g, unsigned* keys, unsigned* place,
                             unsigned* count) {
+  chainWait(false);
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nSmall) return;
   GridParams G = *g;
@@ -345,6 +348,7 @@ static const long long SCAN_SPIN = 1ll << 22;
 
 __global__ void __launch_bounds__(SCAN_T) k_scan(unsigned* a, long long n, unsigned long long* status, unsigned* ticket,
                                                  unsigned ticket0, unsigned epoch, DeviceStatus* st) {
+  chainWait(false);
   __shared__ unsigned tileS, prefixS;
   __shared__ unsigned warpSum[SCAN_T / 32];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -445,9 +449,8 @@ void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratc
     cs.scanTickets = 0;
   }
   const unsigned nt = (unsigned)((n + SCAN_TILE - 1) / SCAN_TILE);
-  (k_scan<<<nt, SCAN_T, 0, s>>>(a, n, reinterpret_cast<unsigned long long*>(cs.scanScratch + 64), cs.scanScratch,
-                                cs.scanTickets, cs.scanEpoch, cs.st),
-   ++::wdem::g_kernel_launches);
+  launchChained(k_scan, nt, SCAN_T, s, a, n, reinterpret_cast<unsigned long long*>(cs.scanScratch + 64), cs.scanScratch,
+                                cs.scanTickets, cs.scanEpoch, cs.st);
   cs.scanTickets += nt;
 }
 
@@ -459,6 +462,7 @@ void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratc
 // dependent launch of 10 us at 15k bodies and 25 us at 500k.
 __global__ void k_bucket_place(const int* small, int nSmall, const unsigned* keys, const unsigned* place,
                                const unsigned* start, const GridParams* g, unsigned long long* tmp) {
+  chainWait(false);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nSmall) return;
   const unsigned key = keys[k];
@@ -476,6 +480,7 @@ __device__ __forceinline__ unsigned rankInBucket(const unsigned long long* tmp, 
 // walks these contiguous records instead of gathering meta, bbmin and bbmax by particle id.
 __global__ void k_bucket_rank(Particles p, int nSmall, const unsigned long long* tmp, const unsigned* start,
                               const GridParams* g, unsigned* keys, unsigned* vals, float4* rec) {
+  chainWait(false);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nSmall) return;
   const unsigned long long v = tmp[e];
@@ -555,6 +560,7 @@ struct SweepArgs {
 template <bool WRITE>
 __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned* counts, int2* out, long long cap,
                         DeviceStatus* st) {
+  chainWait(false);
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= sweepThreads(A.nSmall, A.nLarge)) return;
   unsigned cnt = 0;
@@ -679,6 +685,7 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
 // removes only non-real contacts on separation, InsertionSortCollider.cpp:107-110).
 __global__ void k_retain_flag(StepParams P, Particles p, Contacts old, long long nOld, unsigned* flag,
                               const float4* pci, const float4* phi) {
+  chainWait(false);
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nOld) return;
   unsigned f = 0;
@@ -703,6 +710,7 @@ __global__ void k_retain_flag(StepParams P, Particles p, Contacts old, long long
   flag[c] = f;
 }
 __global__ void k_retain_write_dist(Contacts old, long long nOld, const unsigned* flagScan, int4* out, long long base, long long cap) {
+  chainWait(false);
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nOld) return;
   if (flagScan[c + 1] != flagScan[c]) {
@@ -711,6 +719,7 @@ __global__ void k_retain_write_dist(Contacts old, long long nOld, const unsigned
   }
 }
 __global__ void k_retain_write(Contacts old, long long nOld, const unsigned* flagScan, int2* out, long long base, long long cap) {
+  chainWait(false);
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nOld) return;
   if (flagScan[c + 1] != flagScan[c]) {
@@ -781,6 +790,7 @@ __device__ __forceinline__ bool maybeLarge(uint8_t state) { return (state & (CS_
 // pass 2 writes each contact at its place: real ones at their rank, the others after them in order.
 __global__ void k_part_flag(Contacts neu, long long nNew, Contacts old, Csr oldCsr, unsigned long long* tmpIds,
                             unsigned* tmpJ, unsigned* flag, int4* tmpDist) {
+  chainWait(false);
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nNew) return;
   const int2 id = neu.ids[c];
@@ -798,6 +808,7 @@ __global__ void k_part_flag(Contacts neu, long long nNew, Contacts old, Csr oldC
 __global__ void k_carry_compact(Particles p, Contacts neu, long long nNew, Contacts old, const unsigned long long* tmpIds,
                                 const unsigned* tmpJ, const unsigned* scan, const int4* tmpDist, long long step, int nHist,
                                 RowCount R) {
+  chainWait(false);
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nNew) return;
   const unsigned before = scan[c];
@@ -835,6 +846,7 @@ __global__ void k_carry_compact(Particles p, Contacts neu, long long nNew, Conta
 // ------------------------------------------------------------------------------------ CSR
 // places in the rows of an uploaded container's contacts (a rebuild takes them in k_carry_compact)
 __global__ void k_csr_places(Contacts c, long long nc, RowCount R) {
+  chainWait(false);
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nc) return;
   const int2 id = c.ids[e];
@@ -843,6 +855,7 @@ __global__ void k_csr_places(Contacts c, long long nc, RowCount R) {
 }
 // the ranges of one large body: counts to starts within its row (one block a body); the row's length to cnt
 __global__ void __launch_bounds__(256) k_csr_large(const int* large, RowCount R) {
+  chainWait(false);
   __shared__ unsigned warpSum[8];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   unsigned* sub = R.sub + (long long)blockIdx.x * R.V;
@@ -869,6 +882,7 @@ __global__ void __launch_bounds__(256) k_csr_large(const int* large, RowCount R)
 }
 // the entries at their places: (partner, contact | isB << 31)
 __global__ void k_csr_fill(Contacts c, long long nc, RowCount R, unsigned long long* tmp) {
+  chainWait(false);
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nc) return;
   const int2 id = c.ids[e], place = c.slot[e];
@@ -883,6 +897,7 @@ __global__ void k_csr_fill(Contacts c, long long nc, RowCount R, unsigned long l
 // so the threads of a warp read the same few rows from L1.
 __global__ void k_csr_rank(Contacts c, long long ne, RowCount R, const unsigned long long* tmp, unsigned* ent,
                            unsigned* partner) {
+  chainWait(false);
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   const unsigned long long v = tmp[e];
@@ -916,6 +931,7 @@ __global__ void k_csr_rank(Contacts c, long long ne, RowCount R, const unsigned 
 // the filter (there the exact test may find an ambiguous contact, which is an error to report).
 __global__ void k_keys_peri(StepParams P, Particles p, const int* small, int nSmall, const PeriGrid* g, unsigned* keys,
                             unsigned* place, unsigned* count, float4* pci, float4* phi, int4* wrap) {
+  chainWait(false);
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nSmall) return;
   const PeriGrid G = *g;
@@ -951,6 +967,7 @@ __global__ void k_keys_peri(StepParams P, Particles p, const int* small, int nSm
 // the bodies in cell order: key, and the FP32 copies with the id in the centre's fourth word
 __global__ void k_bucket_rank_peri(int nSmall, const unsigned long long* tmp, const unsigned* start, unsigned* keys,
                                    const float4* pci, const float4* phi, float4* pc, float4* ph) {
+  chainWait(false);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nSmall) return;
   const unsigned long long v = tmp[e];
@@ -983,6 +1000,7 @@ struct CandArgs {
 template <bool WRITE>
 __global__ void __launch_bounds__(128) k_peri_cand(StepParams P, CandArgs A, const PeriGrid* g, unsigned* counts, int2* cand,
                                                    long long cap) {
+  chainWait(false);
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q > A.nSmall) return;
   if (q == A.nSmall) { if (!WRITE) counts[q] = 0; return; }
@@ -1079,6 +1097,7 @@ __global__ void __launch_bounds__(128) k_peri_cand(StepParams P, CandArgs A, con
 // those for every candidate this pass took 486 us for the 1.6 M pairs of 400k bodies.
 __global__ void k_peri_exact(StepParams P, Particles p, const int2* cand, long long nc, const float4* pci, const float4* phi,
                              const int4* wrap, unsigned* flag, int4* per, DeviceStatus* st) {
+  chainWait(false);
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nc) return;
   const int2 ij = cand[k];
@@ -1106,6 +1125,7 @@ __global__ void k_peri_exact(StepParams P, Particles p, const int2* cand, long l
 // the accepted candidates, in candidate order, with their cellDist
 __global__ void k_peri_emit(const int2* cand, const int4* per, const unsigned* flagScan, long long nc, int2* out,
                             int4* outDist, long long cap) {
+  chainWait(false);
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nc || flagScan[k + 1] == flagScan[k]) return;
   const long long o = flagScan[k];
@@ -1116,6 +1136,7 @@ __global__ void k_peri_emit(const int2* cand, const int4* per, const unsigned* f
 // ContactLoop stress (ContactLoop.cpp:218-229): F (global, on pA) x branch (pB image - pA) per real
 // contact; the nine components are summed by the deterministic energy reduction.
 __global__ void k_stress_terms(StepParams P, Particles p, Contacts c, long long nc, double* terms) {
+  chainWait(false);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc) return;
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -1171,7 +1192,7 @@ static void launchExtents(cudaStream_t s, const StepParams& P, Particles p, cons
   unsigned long long* ext = (unsigned long long*)cs.temp;
   cudaMemsetAsync(ext, 0xff, EXT_WORDS * sizeof(unsigned long long), s);
   const unsigned blocks = (unsigned)std::max(1, std::min((nSmall + EXT_T - 1) / EXT_T, 2 * 152));
-  (k_extents<<<blocks, EXT_T, 0, s>>>(P, p, small, nSmall, ext, A), ++::wdem::g_kernel_launches);
+  launchChained(k_extents, blocks, EXT_T, s, P, p, small, nSmall, ext, A);
 }
 
 // The collider sub-steps are called from wdem_api.cu through these thin wrappers.
@@ -1186,10 +1207,10 @@ void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, Collide
   cudaMemsetAsync(a.start, 0, ((size_t)nb + 1) * sizeof(unsigned), s);
   if (nSmall <= 0) return;
   const unsigned blocks = (unsigned)((nSmall + 255) / 256);
-  (k_make_keys<<<blocks, 256, 0, s>>>(p, small, nSmall, cs.grid, a.keyIn, a.place, a.start), ++::wdem::g_kernel_launches);
+  launchChained(k_make_keys, blocks, 256, s, p, small, nSmall, cs.grid, a.keyIn, a.place, a.start);
   exclusive_scan_u32(s, a.start, nb, cs);
-  (k_bucket_place<<<blocks, 256, 0, s>>>(small, nSmall, a.keyIn, a.place, a.start, cs.grid, a.tmp), ++::wdem::g_kernel_launches);
-  (k_bucket_rank<<<blocks, 256, 0, s>>>(p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec), ++::wdem::g_kernel_launches);
+  launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, cs.grid, a.tmp);
+  launchChained(k_bucket_rank, blocks, 256, s, p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec);
 }
 
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out, long long cap,
@@ -1202,21 +1223,21 @@ void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, Colli
   A.sceneWall = cs.nScenes > 1 ? cs.sceneWall : nullptr;
   A.buf = cs.sweepBufCap >= sweepThreads(nSmall, cs.nLarge) ? cs.sweepBuf : nullptr;
   const int threads = sweepThreads(nSmall, cs.nLarge);
-  if (write) (k_sweep<true><<<(threads + 127) / 128, 128, 0, s>>>(p, A, cs.grid, cs.counts, out, cap, st), ++::wdem::g_kernel_launches);
-  else (k_sweep<false><<<(threads + 127) / 128, 128, 0, s>>>(p, A, cs.grid, cs.counts, out, cap, st), ++::wdem::g_kernel_launches);
+  if (write) launchChained(k_sweep<true>, (threads + 127) / 128, 128, s, p, A, cs.grid, cs.counts, out, cap, st);
+  else launchChained(k_sweep<false>, (threads + 127) / 128, 128, s, p, A, cs.grid, cs.counts, out, cap, st);
 }
 
 void col_retain_write_dist(cudaStream_t s, Contacts old, long long nOld, ColliderScratch& cs, int4* out, long long base,
                            long long cap) {
-  if (nOld > 0) (k_retain_write_dist<<<(unsigned)((nOld + 255) / 256), 256, 0, s>>>(old, nOld, cs.retainFlag, out, base, cap), ++::wdem::g_kernel_launches);
+  if (nOld > 0) launchChained(k_retain_write_dist, (unsigned)((nOld + 255) / 256), 256, s, old, nOld, cs.retainFlag, out, base, cap);
 }
 
 void col_retain_flags(cudaStream_t s, const StepParams& P, Particles p, Contacts old, long long nOld, ColliderScratch& cs) {
-  if (nOld > 0) (k_retain_flag<<<(unsigned)((nOld + 255) / 256), 256, 0, s>>>(P, p, old, nOld, cs.retainFlag, cs.periCi, cs.periHi), ++::wdem::g_kernel_launches);
+  if (nOld > 0) launchChained(k_retain_flag, (unsigned)((nOld + 255) / 256), 256, s, P, p, old, nOld, cs.retainFlag, cs.periCi, cs.periHi);
   exclusive_scan_u32(s, cs.retainFlag, nOld, cs);
 }
 void col_retain_write(cudaStream_t s, Contacts old, long long nOld, ColliderScratch& cs, int2* out, long long base, long long cap) {
-  if (nOld > 0) (k_retain_write<<<(unsigned)((nOld + 255) / 256), 256, 0, s>>>(old, nOld, cs.retainFlag, out, base, cap), ++::wdem::g_kernel_launches);
+  if (nOld > 0) launchChained(k_retain_write, (unsigned)((nOld + 255) / 256), 256, s, old, nOld, cs.retainFlag, out, base, cap);
 }
 
 // periodic pair search, part 1: grid, cell sort, FP32 candidates counted (write false; counts
@@ -1234,35 +1255,33 @@ void col_periodic_cand(cudaStream_t s, const StepParams& P, Particles p, const i
     cudaMemsetAsync(a.start, 0, ((size_t)nb + 1) * sizeof(unsigned), s);
     if (nSmall > 0) {
       const unsigned blocks = (unsigned)((nSmall + 255) / 256);
-      (k_keys_peri<<<blocks, 256, 0, s>>>(P, p, small, nSmall, g, a.keyIn, a.place, a.start, cs.periCi, cs.periHi, cs.periWrap),
-       ++::wdem::g_kernel_launches);
+      launchChained(k_keys_peri, blocks, 256, s, P, p, small, nSmall, g, a.keyIn, a.place, a.start, cs.periCi, cs.periHi, cs.periWrap);
       exclusive_scan_u32(s, a.start, nb, cs);
-      (k_bucket_place<<<blocks, 256, 0, s>>>(small, nSmall, a.keyIn, a.place, a.start, nullptr, a.tmp), ++::wdem::g_kernel_launches);
-      (k_bucket_rank_peri<<<blocks, 256, 0, s>>>(nSmall, a.tmp, a.start, a.key, cs.periCi, cs.periHi, cs.periC, cs.periH),
-       ++::wdem::g_kernel_launches);
+      launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, nullptr, a.tmp);
+      launchChained(k_bucket_rank_peri, blocks, 256, s, nSmall, a.tmp, a.start, a.key, cs.periCi, cs.periHi, cs.periC, cs.periH);
     }
-    (k_peri_cand<false><<<(threads + 127) / 128, 128, 0, s>>>(P, A, g, cs.counts, nullptr, 0), ++::wdem::g_kernel_launches);
+    launchChained(k_peri_cand<false>, (threads + 127) / 128, 128, s, P, A, g, cs.counts, nullptr, 0);
     exclusive_scan_u32(s, cs.counts, nSmall + 1, cs);
   } else {
-    (k_peri_cand<true><<<(threads + 127) / 128, 128, 0, s>>>(P, A, g, cs.counts, cs.cand, cs.candCap), ++::wdem::g_kernel_launches);
+    launchChained(k_peri_cand<true>, (threads + 127) / 128, 128, s, P, A, g, cs.counts, cs.cand, cs.candCap);
   }
 }
 
 // part 2: the exact test of nCand candidates; flags scanned, accepted total at candFlag[nCand]
 void col_periodic_exact(cudaStream_t s, const StepParams& P, Particles p, ColliderScratch& cs, long long nCand,
                         DeviceStatus* st) {
-  if (nCand > 0) (k_peri_exact<<<(unsigned)((nCand + 255) / 256), 256, 0, s>>>(P, p, cs.cand, nCand, cs.periCi, cs.periHi, cs.periWrap, cs.candFlag, cs.candPer, st), ++::wdem::g_kernel_launches);
+  if (nCand > 0) launchChained(k_peri_exact, (unsigned)((nCand + 255) / 256), 256, s, P, p, cs.cand, nCand, cs.periCi, cs.periHi, cs.periWrap, cs.candFlag, cs.candPer, st);
   exclusive_scan_u32(s, cs.candFlag, nCand, cs);
 }
 
 // part 3: accepted pairs and their cellDist into the new container
 void col_periodic_emit(cudaStream_t s, ColliderScratch& cs, long long nCand, int2* out, int4* outDist, long long cap) {
-  if (nCand > 0) (k_peri_emit<<<(unsigned)((nCand + 255) / 256), 256, 0, s>>>(cs.cand, cs.candPer, cs.candFlag, nCand, out, outDist, cap), ++::wdem::g_kernel_launches);
+  if (nCand > 0) launchChained(k_peri_emit, (unsigned)((nCand + 255) / 256), 256, s, cs.cand, cs.candPer, cs.candFlag, nCand, out, outDist, cap);
 }
 
 void launch_stress(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc, double* scratch9,
                    double* partials, double* out9, DeviceStatus* st) {
-  if (nc > 0) (k_stress_terms<<<(unsigned)((nc + 255) / 256), 256, 0, s>>>(P, p, c, nc, scratch9), ++::wdem::g_kernel_launches);
+  if (nc > 0) launchChained(k_stress_terms, (unsigned)((nc + 255) / 256), 256, s, P, p, c, nc, scratch9);
   SumSet S{};
   for (int q = 0; q < 9; q++) {
     S.x[q] = scratch9 + (long long)q * nc;
@@ -1300,10 +1319,10 @@ void col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew
   unsigned* flag = cs.valsAlt;
   int4* tmpDist = neu.cdist ? reinterpret_cast<int4*>(cs.keysAlt) : nullptr;
   const unsigned blocks = (unsigned)((nNew + 255) / 256);
-  (k_part_flag<<<blocks, 256, 0, s>>>(neu, nNew, old, oldCsr, tmpIds, tmpJ, flag, tmpDist), ++::wdem::g_kernel_launches);
+  launchChained(k_part_flag, blocks, 256, s, neu, nNew, old, oldCsr, tmpIds, tmpJ, flag, tmpDist);
   exclusive_scan_u32(s, flag, nNew, cs);
   clearRows(s, n, R, cs);  // the old rows have been read
-  (k_carry_compact<<<blocks, 256, 0, s>>>(p, neu, nNew, old, tmpIds, tmpJ, flag, tmpDist, step, nHist, R), ++::wdem::g_kernel_launches);
+  launchChained(k_carry_compact, blocks, 256, s, p, neu, nNew, old, tmpIds, tmpJ, flag, tmpDist, step, nHist, R);
 }
 
 // The CSR of the container.  placed: its contacts have taken their places (k_carry_compact).
@@ -1312,15 +1331,15 @@ void col_csr(cudaStream_t s, Contacts c, long long nc, int n, Csr& csr, Collider
   const unsigned blocks = (unsigned)((nc + 255) / 256);
   if (!placed) {
     clearRows(s, n, R, cs);
-    if (nc > 0) (k_csr_places<<<blocks, 256, 0, s>>>(c, nc, R), ++::wdem::g_kernel_launches);
+    if (nc > 0) launchChained(k_csr_places, blocks, 256, s, c, nc, R);
   }
   csr.n = n;
-  if (cs.nLarge > 0) (k_csr_large<<<(unsigned)cs.nLarge, 256, 0, s>>>(cs.large, R), ++::wdem::g_kernel_launches);
+  if (cs.nLarge > 0) launchChained(k_csr_large, (unsigned)cs.nLarge, 256, s, cs.large, R);
   exclusive_scan_u32(s, R.cnt, n, cs);
   if (nc <= 0) return;
   unsigned long long* tmp = cs.keysAlt;
-  (k_csr_fill<<<blocks, 256, 0, s>>>(c, nc, R, tmp), ++::wdem::g_kernel_launches);
-  (k_csr_rank<<<(unsigned)((2 * nc + 255) / 256), 256, 0, s>>>(c, 2 * nc, R, tmp, csr.ent, csr.partner), ++::wdem::g_kernel_launches);
+  launchChained(k_csr_fill, blocks, 256, s, c, nc, R, tmp);
+  launchChained(k_csr_rank, (unsigned)((2 * nc + 255) / 256), 256, s, c, 2 * nc, R, tmp, csr.ent, csr.partner);
 }
 
 }  // namespace wdem
