@@ -15,7 +15,7 @@
 //   4. writes the pairs in a deterministic order (count pass with each particle's first pairs buffered,
 //      exclusive scan, write pass),
 //   5. carries contact history over, finding each pair's old contact by a binary search in the old
-//      CSR's sorted keys (row of the lower id, keyed by the partner),
+//      CSR's row of the lower id, whose partners are sorted,
 //   6. builds the per-particle contact CSR with rows ordered by the partner id.
 #include "wdem_internal.h"
 #include "wdem_math.cuh"
@@ -749,7 +749,7 @@ __device__ __forceinline__ long long csrFind(const Csr& csr, int a, int b) {
 // counts gives their starts, the entries go to their places, and each entry's rank among its row's partners is its
 // final position.  Rows hold ten or twenty entries, so the ranks are a few loads from L1; the order does not depend
 // on the atomics.  The radix sort of 2 C keys of up to 46 bits this replaces took 6 passes over 12 bytes an entry
-// (9 sorting launches a rebuild with 500k bodies and 2 M pairs, 730 us of 2 rebuilds; this: see k_csr_rank).
+// (9 launches of 41 us a rebuild with 500k bodies and 2 M pairs; k_csr_fill and k_csr_rank now take 28 + 55 us).
 // A wall's or facet's row can hold every body: it is divided into V ranges of S partner ids, counted apart (so the
 // atomics spread as well), and an entry is ranked within its range.
 struct RowCount {
@@ -1270,13 +1270,17 @@ void col_periodic_cand(cudaStream_t s, const StepParams& P, Particles p, const i
 // part 2: the exact test of nCand candidates; flags scanned, accepted total at candFlag[nCand]
 void col_periodic_exact(cudaStream_t s, const StepParams& P, Particles p, ColliderScratch& cs, long long nCand,
                         DeviceStatus* st) {
-  if (nCand > 0) launchChained(k_peri_exact, (unsigned)((nCand + 255) / 256), 256, s, P, p, cs.cand, nCand, cs.periCi, cs.periHi, cs.periWrap, cs.candFlag, cs.candPer, st);
+  if (nCand > 0)
+    launchChained(k_peri_exact, (unsigned)((nCand + 255) / 256), 256, s, P, p, cs.cand, nCand, cs.periCi, cs.periHi,
+                  cs.periWrap, cs.candFlag, cs.candPer, st);
   exclusive_scan_u32(s, cs.candFlag, nCand, cs);
 }
 
 // part 3: accepted pairs and their cellDist into the new container
 void col_periodic_emit(cudaStream_t s, ColliderScratch& cs, long long nCand, int2* out, int4* outDist, long long cap) {
-  if (nCand > 0) launchChained(k_peri_emit, (unsigned)((nCand + 255) / 256), 256, s, cs.cand, cs.candPer, cs.candFlag, nCand, out, outDist, cap);
+  if (nCand > 0)
+    launchChained(k_peri_emit, (unsigned)((nCand + 255) / 256), 256, s, cs.cand, cs.candPer, cs.candFlag, nCand, out,
+                  outDist, cap);
 }
 
 void launch_stress(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc, double* scratch9,

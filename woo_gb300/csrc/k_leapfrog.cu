@@ -661,7 +661,7 @@ __device__ __forceinline__ bool spinFast(const StepParams& P, const Particles& p
 // A node without contact forces, in the first pass.  Spinning spheres of a warp that has ROTATE_HERE of them or more
 // are turned here, while the pass waits for memory; fewer go to the rotation list of the second pass (scattered over
 // most warps they would each cost their warp the FP64 time of 32).  1M falling, spinning spheres: first and second
-// pass 47 + 141 us a step with all of them listed (one atomic a warp on one counter), see k_leapfrog_lists for now.
+// pass 47 + 141 us a step with all of them listed (one atomic a warp on one counter), 80 + 82 us so.
 static const int ROTATE_HERE = 16;
 template <bool PERI>
 __device__ __forceinline__ void integrateFast(const StepParams& P, const Particles& p, const int i, const int n,
