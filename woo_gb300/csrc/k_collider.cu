@@ -343,17 +343,28 @@ __global__ void k_make_keys(Particles p, const int* small, int nSmall, const Gri
 // and the ticket counts on from where the last scan left it.  A rebuild's scans were 3 to 5 launches each before
 // (tile scans, the scan of their sums, the sums added back), of 3 us for 15k bodies.
 static const int SCAN_T = 256, SCAN_I = 16, SCAN_TILE = SCAN_T * SCAN_I;
+//
+// A look-back whose wait runs out says so in scanFailed and takes 0 for what it waited for; so does a block whose ticket
+// is not one of this launch's (a launch that never ran after its tickets were counted).  The scanned values are then
+// not offsets of anything, and every kernel that uses them, or what was made from them, returns at once.
 static const unsigned SCAN_AGG = 1u, SCAN_PRE = 2u, SCAN_EPOCHS = 1u << 30;
-static const long long SCAN_SPIN = 1ll << 22;
+__device__ __forceinline__ void scanGaveUp(DeviceStatus* st) {
+  st->scanFailed = 1;
+  if (atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT) == 0) st->detail = DETAIL_SCAN;
+}
 
 __global__ void __launch_bounds__(SCAN_T) k_scan(unsigned* a, long long n, unsigned long long* status, unsigned* ticket,
-                                                 unsigned ticket0, unsigned epoch, DeviceStatus* st) {
+                                                 unsigned ticket0, unsigned epoch, int looks, int total, DeviceStatus* st) {
   chainWait(false);
   __shared__ unsigned tileS, prefixS;
   __shared__ unsigned warpSum[SCAN_T / 32];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   if (t == 0) tileS = atomicAdd(ticket, 1u) - ticket0;
   __syncthreads();
+  if (tileS >= gridDim.x) {
+    if (t == 0) scanGaveUp(st);
+    return;
+  }
   const long long tile = tileS;
   const long long first = tile * SCAN_TILE + (long long)t * SCAN_I;
   unsigned v[SCAN_I];
@@ -377,31 +388,32 @@ __global__ void __launch_bounds__(SCAN_T) k_scan(unsigned* a, long long n, unsig
   }
   if (lane == 31) warpSum[warp] = inc;
   __syncthreads();
-  unsigned before = 0, total = 0;
+  unsigned before = 0, tileSum = 0;
 #pragma unroll
   for (int w = 0; w < SCAN_T / 32; w++) {
     if (w < warp) before += warpSum[w];
-    total += warpSum[w];
+    tileSum += warpSum[w];
   }
   if (warp == 0) {
     const unsigned long long tag = (unsigned long long)epoch << 34;
     unsigned prefix = 0;
     if (tile > 0) {
-      if (lane == 0) *(volatile unsigned long long*)(status + tile) = tag | ((unsigned long long)SCAN_AGG << 32) | total;
+      if (lane == 0) *(volatile unsigned long long*)(status + tile) = tag | ((unsigned long long)SCAN_AGG << 32) | tileSum;
       for (long long j = tile - 1; j >= 0; j -= 32) {
         const long long q = j - lane;
         unsigned long long w = tag | ((unsigned long long)SCAN_PRE << 32);  // before the first tile: prefix 0
         if (q >= 0) {
-          w = *(volatile unsigned long long*)(status + q);
-          long long it = 0;
-          while ((w >> 34) != epoch || ((w >> 32) & 3u) == 0) {
-            if (++it > SCAN_SPIN) {
-              atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT);
-              w = tag | ((unsigned long long)SCAN_PRE << 32);
+          for (int left = looks;; left--) {
+            if (left <= 0) {
+              scanGaveUp(st);
+              break;  // w: prefix 0
+            }
+            const unsigned long long seen = *(volatile unsigned long long*)(status + q);
+            if ((seen >> 34) == epoch && ((seen >> 32) & 3u) != 0) {
+              w = seen;
               break;
             }
             __nanosleep(20);
-            w = *(volatile unsigned long long*)(status + q);
           }
         }
         const unsigned pre = __ballot_sync(0xffffffffu, ((w >> 32) & 3u) == SCAN_PRE);
@@ -411,7 +423,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan(unsigned* a, long long n, unsig
       }
     }
     if (lane == 0) {
-      *(volatile unsigned long long*)(status + tile) = tag | ((unsigned long long)SCAN_PRE << 32) | (prefix + total);
+      *(volatile unsigned long long*)(status + tile) = tag | ((unsigned long long)SCAN_PRE << 32) | (prefix + tileSum);
       prefixS = prefix;
     }
   }
@@ -432,15 +444,19 @@ __global__ void __launch_bounds__(SCAN_T) k_scan(unsigned* a, long long n, unsig
     }
   }
   // the thread after the last value (of the last tile, also when n fills it) holds the total
-  if ((tile + 1) * SCAN_TILE >= n && t == SCAN_T - 1) a[n] = prefixS + total;
+  if ((tile + 1) * SCAN_TILE >= n && t == SCAN_T - 1) {
+    a[n] = prefixS + tileSum;
+    if (total >= 0) st->totals[total] = prefixS + tileSum;
+  }
 }
 
 // 32-bit words of scan scratch (ticket, then one 64-bit status word per tile) for scans of n values
 long long scan_scratch_words(long long n) { return 64 + 2 * ((n + SCAN_TILE - 1) / SCAN_TILE + 1); }
 
-void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs) {
+void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs, int total) {
   if (n <= 0) {
     cudaMemsetAsync(a, 0, sizeof(unsigned), s);  // empty: total 0
+    if (total >= 0) cudaMemsetAsync(&cs.st->totals[total], 0, sizeof(unsigned), s);
     return;
   }
   if (++cs.scanEpoch >= SCAN_EPOCHS) {  // the numbers start again: no word of the old ones may be left
@@ -450,7 +466,7 @@ void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratc
   }
   const unsigned nt = (unsigned)((n + SCAN_TILE - 1) / SCAN_TILE);
   launchChained(k_scan, nt, SCAN_T, s, a, n, reinterpret_cast<unsigned long long*>(cs.scanScratch + 64), cs.scanScratch,
-                                cs.scanTickets, cs.scanEpoch, cs.st);
+                cs.scanTickets, cs.scanEpoch, cs.scanLooks, total, cs.st);
   cs.scanTickets += nt;
 }
 
@@ -461,10 +477,11 @@ void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratc
 // is then a table lookup for the sweep.  An LSD radix sort of the keys took 4 passes of 8 bits, each a
 // dependent launch of 10 us at 15k bodies and 25 us at 500k.
 __global__ void k_bucket_place(const int* small, int nSmall, const unsigned* keys, const unsigned* place,
-                               const unsigned* start, const GridParams* g, unsigned long long* tmp) {
+                               const unsigned* start, const GridParams* g, unsigned long long* tmp,
+                               const DeviceStatus* st) {
   chainWait(false);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nSmall) return;
+  if (k >= nSmall || st->scanFailed) return;
   const unsigned key = keys[k];
   const unsigned b = g ? key >> (g->qbits - g->kbits) : key;
   tmp[start[b] + place[k]] = ((unsigned long long)key << 32) | (unsigned)small[k];
@@ -479,10 +496,10 @@ __device__ __forceinline__ unsigned rankInBucket(const unsigned long long* tmp, 
 // test rejects needs no FP64 test), the mask (lo.w) and meta.x with shape and scene (hi.w).  The sweep
 // walks these contiguous records instead of gathering meta, bbmin and bbmax by particle id.
 __global__ void k_bucket_rank(Particles p, int nSmall, const unsigned long long* tmp, const unsigned* start,
-                              const GridParams* g, unsigned* keys, unsigned* vals, float4* rec) {
+                              const GridParams* g, unsigned* keys, unsigned* vals, float4* rec, const DeviceStatus* st) {
   chainWait(false);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nSmall) return;
+  if (e >= nSmall || st->scanFailed) return;
   const unsigned long long v = tmp[e];
   const unsigned key = (unsigned)(v >> 32);
   const int i = (int)(unsigned)v;
@@ -559,10 +576,10 @@ struct SweepArgs {
 // copies them, walking again only for threads that found more: the output is the same, in the same order.
 template <bool WRITE>
 __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned* counts, int2* out, long long cap,
-                        DeviceStatus* st) {
+                        const DeviceStatus* st) {
   chainWait(false);
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= sweepThreads(A.nSmall, A.nLarge)) return;
+  if (s >= sweepThreads(A.nSmall, A.nLarge) || st->scanFailed) return;
   unsigned cnt = 0;
   unsigned long long base = WRITE ? counts[s] : 0;
   if (WRITE && A.buf) {
@@ -807,10 +824,10 @@ __global__ void k_part_flag(Contacts neu, long long nNew, Contacts old, Csr oldC
 }
 __global__ void k_carry_compact(Particles p, Contacts neu, long long nNew, Contacts old, const unsigned long long* tmpIds,
                                 const unsigned* tmpJ, const unsigned* scan, const int4* tmpDist, long long step, int nHist,
-                                RowCount R) {
+                                RowCount R, const DeviceStatus* st) {
   chainWait(false);
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nNew) return;
+  if (c >= nNew || st->scanFailed) return;
   const unsigned before = scan[c];
   const bool wasReal = scan[c + 1] != before;
   const long long d = wasReal ? (long long)before : (long long)scan[nNew] + (c - (long long)before);
@@ -881,10 +898,10 @@ __global__ void __launch_bounds__(256) k_csr_large(const int* large, RowCount R)
   if (t == 0) R.cnt[large[blockIdx.x]] = carry;
 }
 // the entries at their places: (partner, contact | isB << 31)
-__global__ void k_csr_fill(Contacts c, long long nc, RowCount R, unsigned long long* tmp) {
+__global__ void k_csr_fill(Contacts c, long long nc, RowCount R, unsigned long long* tmp, const DeviceStatus* st) {
   chainWait(false);
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nc) return;
+  if (e >= nc || st->scanFailed) return;
   const int2 id = c.ids[e], place = c.slot[e];
   const bool big = maybeLarge(c.state[e]);
   const int kA = rangeOf(R, id.x, id.y, big), kB = rangeOf(R, id.y, id.x, big);
@@ -896,10 +913,10 @@ __global__ void k_csr_fill(Contacts c, long long nc, RowCount R, unsigned long l
 // shares) and their positions in the rows (which bit of the row's mask it sets).  Threads follow the entries of tmp,
 // so the threads of a warp read the same few rows from L1.
 __global__ void k_csr_rank(Contacts c, long long ne, RowCount R, const unsigned long long* tmp, unsigned* ent,
-                           unsigned* partner) {
+                           unsigned* partner, const DeviceStatus* st) {
   chainWait(false);
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
+  if (e >= ne || st->scanFailed) return;
   const unsigned long long v = tmp[e];
   const unsigned val = (unsigned)v, ci = val & 0x7fffffffu;
   const bool isB = (val >> 31) != 0;
@@ -966,10 +983,10 @@ __global__ void k_keys_peri(StepParams P, Particles p, const int* small, int nSm
 
 // the bodies in cell order: key, and the FP32 copies with the id in the centre's fourth word
 __global__ void k_bucket_rank_peri(int nSmall, const unsigned long long* tmp, const unsigned* start, unsigned* keys,
-                                   const float4* pci, const float4* phi, float4* pc, float4* ph) {
+                                   const float4* pci, const float4* phi, float4* pc, float4* ph, const DeviceStatus* st) {
   chainWait(false);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nSmall) return;
+  if (e >= nSmall || st->scanFailed) return;
   const unsigned long long v = tmp[e];
   const unsigned key = (unsigned)(v >> 32);
   const int i = (int)(unsigned)v;
@@ -999,10 +1016,10 @@ struct CandArgs {
 };
 template <bool WRITE>
 __global__ void __launch_bounds__(128) k_peri_cand(StepParams P, CandArgs A, const PeriGrid* g, unsigned* counts, int2* cand,
-                                                   long long cap) {
+                                                   long long cap, const DeviceStatus* st) {
   chainWait(false);
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q > A.nSmall) return;
+  if (q > A.nSmall || st->scanFailed) return;
   if (q == A.nSmall) { if (!WRITE) counts[q] = 0; return; }
   const float4 c1 = A.pc[q];
   const int i = __float_as_int(c1.w);
@@ -1209,12 +1226,12 @@ void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, Collide
   const unsigned blocks = (unsigned)((nSmall + 255) / 256);
   launchChained(k_make_keys, blocks, 256, s, p, small, nSmall, cs.grid, a.keyIn, a.place, a.start);
   exclusive_scan_u32(s, a.start, nb, cs);
-  launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, cs.grid, a.tmp);
-  launchChained(k_bucket_rank, blocks, 256, s, p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec);
+  launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, cs.grid, a.tmp, cs.st);
+  launchChained(k_bucket_rank, blocks, 256, s, p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec, cs.st);
 }
 
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out, long long cap,
-               bool write, DeviceStatus* st) {
+               bool write) {
   SweepArgs A;
   A.rec = cs.srec;
   const SortArrays a = sortArrays(cs);
@@ -1223,8 +1240,8 @@ void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, Colli
   A.sceneWall = cs.nScenes > 1 ? cs.sceneWall : nullptr;
   A.buf = cs.sweepBufCap >= sweepThreads(nSmall, cs.nLarge) ? cs.sweepBuf : nullptr;
   const int threads = sweepThreads(nSmall, cs.nLarge);
-  if (write) launchChained(k_sweep<true>, (threads + 127) / 128, 128, s, p, A, cs.grid, cs.counts, out, cap, st);
-  else launchChained(k_sweep<false>, (threads + 127) / 128, 128, s, p, A, cs.grid, cs.counts, out, cap, st);
+  if (write) launchChained(k_sweep<true>, (threads + 127) / 128, 128, s, p, A, cs.grid, cs.counts, out, cap, cs.st);
+  else launchChained(k_sweep<false>, (threads + 127) / 128, 128, s, p, A, cs.grid, cs.counts, out, cap, cs.st);
 }
 
 void col_retain_write_dist(cudaStream_t s, Contacts old, long long nOld, ColliderScratch& cs, int4* out, long long base,
@@ -1234,7 +1251,7 @@ void col_retain_write_dist(cudaStream_t s, Contacts old, long long nOld, Collide
 
 void col_retain_flags(cudaStream_t s, const StepParams& P, Particles p, Contacts old, long long nOld, ColliderScratch& cs) {
   if (nOld > 0) launchChained(k_retain_flag, (unsigned)((nOld + 255) / 256), 256, s, P, p, old, nOld, cs.retainFlag, cs.periCi, cs.periHi);
-  exclusive_scan_u32(s, cs.retainFlag, nOld, cs);
+  exclusive_scan_u32(s, cs.retainFlag, nOld, cs, TOTAL_RETAINED);
 }
 void col_retain_write(cudaStream_t s, Contacts old, long long nOld, ColliderScratch& cs, int2* out, long long base, long long cap) {
   if (nOld > 0) launchChained(k_retain_write, (unsigned)((nOld + 255) / 256), 256, s, old, nOld, cs.retainFlag, out, base, cap);
@@ -1257,13 +1274,13 @@ void col_periodic_cand(cudaStream_t s, const StepParams& P, Particles p, const i
       const unsigned blocks = (unsigned)((nSmall + 255) / 256);
       launchChained(k_keys_peri, blocks, 256, s, P, p, small, nSmall, g, a.keyIn, a.place, a.start, cs.periCi, cs.periHi, cs.periWrap);
       exclusive_scan_u32(s, a.start, nb, cs);
-      launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, nullptr, a.tmp);
-      launchChained(k_bucket_rank_peri, blocks, 256, s, nSmall, a.tmp, a.start, a.key, cs.periCi, cs.periHi, cs.periC, cs.periH);
+      launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, nullptr, a.tmp, cs.st);
+      launchChained(k_bucket_rank_peri, blocks, 256, s, nSmall, a.tmp, a.start, a.key, cs.periCi, cs.periHi, cs.periC, cs.periH, cs.st);
     }
-    launchChained(k_peri_cand<false>, (threads + 127) / 128, 128, s, P, A, g, cs.counts, nullptr, 0);
-    exclusive_scan_u32(s, cs.counts, nSmall + 1, cs);
+    launchChained(k_peri_cand<false>, (threads + 127) / 128, 128, s, P, A, g, cs.counts, nullptr, 0, cs.st);
+    exclusive_scan_u32(s, cs.counts, nSmall + 1, cs, TOTAL_PAIRS);
   } else {
-    launchChained(k_peri_cand<true>, (threads + 127) / 128, 128, s, P, A, g, cs.counts, cs.cand, cs.candCap);
+    launchChained(k_peri_cand<true>, (threads + 127) / 128, 128, s, P, A, g, cs.counts, cs.cand, cs.candCap, cs.st);
   }
 }
 
@@ -1273,7 +1290,7 @@ void col_periodic_exact(cudaStream_t s, const StepParams& P, Particles p, Collid
   if (nCand > 0)
     launchChained(k_peri_exact, (unsigned)((nCand + 255) / 256), 256, s, P, p, cs.cand, nCand, cs.periCi, cs.periHi,
                   cs.periWrap, cs.candFlag, cs.candPer, st);
-  exclusive_scan_u32(s, cs.candFlag, nCand, cs);
+  exclusive_scan_u32(s, cs.candFlag, nCand, cs, TOTAL_PAIRS);
 }
 
 // part 3: accepted pairs and their cellDist into the new container
@@ -1326,7 +1343,7 @@ void col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew
   launchChained(k_part_flag, blocks, 256, s, neu, nNew, old, oldCsr, tmpIds, tmpJ, flag, tmpDist);
   exclusive_scan_u32(s, flag, nNew, cs);
   clearRows(s, n, R, cs);  // the old rows have been read
-  launchChained(k_carry_compact, blocks, 256, s, p, neu, nNew, old, tmpIds, tmpJ, flag, tmpDist, step, nHist, R);
+  launchChained(k_carry_compact, blocks, 256, s, p, neu, nNew, old, tmpIds, tmpJ, flag, tmpDist, step, nHist, R, cs.st);
 }
 
 // The CSR of the container.  placed: its contacts have taken their places (k_carry_compact).
@@ -1342,8 +1359,8 @@ void col_csr(cudaStream_t s, Contacts c, long long nc, int n, Csr& csr, Collider
   exclusive_scan_u32(s, R.cnt, n, cs);
   if (nc <= 0) return;
   unsigned long long* tmp = cs.keysAlt;
-  launchChained(k_csr_fill, blocks, 256, s, c, nc, R, tmp);
-  launchChained(k_csr_rank, (unsigned)((2 * nc + 255) / 256), 256, s, c, 2 * nc, R, tmp, csr.ent, csr.partner);
+  launchChained(k_csr_fill, blocks, 256, s, c, nc, R, tmp, cs.st);
+  launchChained(k_csr_rank, (unsigned)((2 * nc + 255) / 256), 256, s, c, 2 * nc, R, tmp, csr.ent, csr.partner, cs.st);
 }
 
 }  // namespace wdem

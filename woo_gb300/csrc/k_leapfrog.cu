@@ -940,7 +940,7 @@ void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, in
 // doubles order as their bit patterns (kept complemented, so that zero means none).
 __global__ void k_dyndt(StepParams P, Particles p, int n, Contacts c, Csr csr, DeviceStatus* st) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || st->scanFailed) return;
   const unsigned flags = (unsigned)p.meta[i].w;
   if ((flags & 63u) == 63u) return;  // completely blocked: always stable (Inf)
   d3 kt3 = mk(0, 0, 0), kr3 = mk(0, 0, 0);

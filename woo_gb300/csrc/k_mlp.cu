@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_tc(Particles p, Contacts c, cons
   if (!ok) tcWait(bar, phase ^ 1u);
   if (!ok && t == 0) {
     atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT);
-    st->detail = -1;
+    st->detail = DETAIL_NETWORK;
   }
   tcFenceBefore();
   __syncthreads();
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad_tc(const float* rec, const 
   if (!ok) tcWait(bar, phase ^ 1u);  // as in k_mlp_tc: the timed-out round's MMAs, before TMEM is freed
   if (!ok && t == 0) {
     atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT);
-    st->detail = -1;
+    st->detail = DETAIL_NETWORK;
   }
   // the CTA's sums into the global gradient: weight rows are TMEM lanes (inputs), columns the outputs
   if (ok && !first) {

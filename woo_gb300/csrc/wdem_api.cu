@@ -438,6 +438,12 @@ int ensurePartials(wdem_handle* h, long long n) {
 }
 
 int checkDeviceStatus(wdem_handle* h) {
+  if (h->hst->scanFailed) {
+    // what the failed scan's rebuild left of the container and its rows is not to be read again
+    h->nContacts = 0;
+    h->csr.n = 0;
+    CK(cudaMemsetAsync(h->csr.rowptr, 0, ((size_t)h->N + 1) * sizeof(int), h->stream));
+  }
   if (h->hst->code != 0) {
     int code = h->hst->code;
     std::string m;
@@ -449,7 +455,9 @@ int checkDeviceStatus(wdem_handle* h) {
     else if (code == WDEM_ERR_UNSUPPORTED)
       m = "sphere-facet contact with the projected centre outside all three edges of Facet #" +
           std::to_string(h->hst->detail) + " (degenerate facet)";
-    else if (code == WDEM_ERR_TIMEOUT && h->hst->detail == -1)
+    else if (code == WDEM_ERR_TIMEOUT && h->hst->detail == DETAIL_SCAN)
+      m = "a prefix sum of the collider did not complete within its wait limit";
+    else if (code == WDEM_ERR_TIMEOUT && h->hst->detail == DETAIL_NETWORK)
       m = "the tensor-core warm-start network did not complete within its wait limit";
     else if (code == WDEM_ERR_TIMEOUT)
       m = "a bounded device loop hit its iteration limit (contact solver, particle #" + std::to_string(h->hst->detail) + ")";
@@ -457,6 +465,14 @@ int checkDeviceStatus(wdem_handle* h) {
     return fail(h, code, m);
   }
   return WDEM_OK;
+}
+
+// The totals of the scans so far, with the status word: a failed scan ends the rebuild here.  (Other errors of the
+// status word are reported by the call that ends, as before.)
+int readTotals(wdem_handle* h) {
+  CK(cudaMemcpyAsync(h->hst, h->dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return h->hst->scanFailed ? checkDeviceStatus(h) : WDEM_OK;
 }
 
 // Collider rebuild: InsertionSortCollider full run (InsertionSortCollider.cpp:407-612).
@@ -469,32 +485,27 @@ int rebuild(wdem_handle* h) {
   if ((rc = ensureScratch(h, h->nContacts))) return rc;
   launch_bboxes(s, h->P, h->d, n);
   const int nSweep = sweepThreads(nSmall, cs.nLarge);
-  const unsigned* totalSrc = cs.counts + nSweep;
   long long nCand = 0;
   if (h->periodic) {
     col_periodic_cand(s, h->P, h->d, h->dSmall, nSmall, cs, false);
-    CK(cudaMemcpyAsync(&h->hcounts[0], cs.counts + nSmall + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    nCand = h->hcounts[0];
+    if ((rc = readTotals(h))) return rc;
+    nCand = h->hst->totals[TOTAL_PAIRS];
     if ((rc = ensureCand(h, nCand))) return rc;
     col_periodic_cand(s, h->P, h->d, h->dSmall, nSmall, cs, true);
     col_periodic_exact(s, h->P, h->d, cs, nCand, h->dst);
-    totalSrc = cs.candFlag + nCand;
   } else {
     col_extents_and_grid(s, h->d, h->dSmall, nSmall, cs);
     col_sort(s, h->d, h->dSmall, nSmall, cs);
-    col_sweep(s, h->d, nSmall, h->P.loneMask, cs, nullptr, 0, false, h->dst);
-    exclusive_scan_u32(s, cs.counts, nSweep, cs);
+    col_sweep(s, h->d, nSmall, h->P.loneMask, cs, nullptr, 0, false);
+    exclusive_scan_u32(s, cs.counts, nSweep, cs, TOTAL_PAIRS);
   }
   ContactBuf& old = h->buf[h->cur];
   ContactBuf& neu = h->buf[1 - h->cur];
   const long long nOld = h->nContacts;
   col_retain_flags(s, h->P, h->d, old.c, nOld, cs);
-  CK(cudaMemcpyAsync(&h->hcounts[0], totalSrc, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&h->hcounts[1], cs.retainFlag + nOld, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  const long long total = h->hcounts[0];
-  const long long retained = h->hcounts[1];
+  if ((rc = readTotals(h))) return rc;
+  const long long total = h->hst->totals[TOTAL_PAIRS];
+  const long long retained = h->hst->totals[TOTAL_RETAINED];
   const long long nNew = total + retained;
   if (h->contactLimit > 0 && nNew > h->contactLimit)
     return fail(h, WDEM_ERR_OVERFLOW, "collider: " + std::to_string(nNew) + " contacts exceed the limit of " +
@@ -505,7 +516,7 @@ int rebuild(wdem_handle* h) {
     CK(allocContacts(neu, cap, hertz, h->keepGeom, h->periodic, h->hasEll));
   }
   if (h->periodic) col_periodic_emit(s, cs, nCand, neu.c.ids, neu.c.cdist, neu.cap);
-  else col_sweep(s, h->d, nSmall, h->P.loneMask, cs, neu.c.ids, neu.cap, true, h->dst);
+  else col_sweep(s, h->d, nSmall, h->P.loneMask, cs, neu.c.ids, neu.cap, true);
   col_retain_write(s, old.c, nOld, cs, neu.c.ids, total, neu.cap);
   if (h->periodic && old.c.cdist) col_retain_write_dist(s, old.c, nOld, cs, neu.c.cdist, total, neu.cap);
   const int side = 1 - h->cur;
@@ -1082,7 +1093,7 @@ int wdem_upload_contacts(wdem_handle* h, const wdem_contacts* c) {
   if ((rc = ensureScratch(h, nc))) return rc;
   if ((rc = ensureCsr(h, nc))) return rc;
   col_csr(s, b.c, nc, h->n, h->csr, h->cs, false);
-  CK(cudaStreamSynchronize(s));
+  if ((rc = readTotals(h))) return rc;
   h->nContacts = nc;
   h->needRebuild = true;
   return WDEM_OK;
@@ -1763,15 +1774,14 @@ int wdem_collide_boxes(wdem_handle* h, int32_t n, const double* mins, const doub
   ColliderScratch& cs = h->cs;
   col_extents_and_grid(s, h->d, h->dSmall, nSmall, cs);
   col_sort(s, h->d, h->dSmall, nSmall, cs);
-  col_sweep(s, h->d, nSmall, loneMask, cs, nullptr, 0, false, h->dst);
+  col_sweep(s, h->d, nSmall, loneMask, cs, nullptr, 0, false);
   const int nSweep = sweepThreads(nSmall, cs.nLarge);
-  exclusive_scan_u32(s, cs.counts, nSweep, cs);
-  CK(cudaMemcpyAsync(&h->hcounts[0], cs.counts + nSweep, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  long long total = h->hcounts[0];
+  exclusive_scan_u32(s, cs.counts, nSweep, cs, TOTAL_PAIRS);
+  if ((rc = readTotals(h))) return rc;
+  long long total = h->hst->totals[TOTAL_PAIRS];
   int2* dpairs = nullptr;
   CK(dalloc(dpairs, (size_t)total + 1));
-  col_sweep(s, h->d, nSmall, loneMask, cs, dpairs, total, true, h->dst);
+  col_sweep(s, h->d, nSmall, loneMask, cs, dpairs, total, true);
   std::vector<int2> hp(total);
   if (total > 0) CK(cudaMemcpyAsync(hp.data(), dpairs, total * sizeof(int2), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));

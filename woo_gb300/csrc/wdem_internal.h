@@ -234,12 +234,17 @@ struct GridParams {
   int ok;
 };
 
+// DeviceStatus.detail of a WDEM_ERR_TIMEOUT that is not a contact's (otherwise the particle)
+enum { DETAIL_NETWORK = -1, DETAIL_SCAN = -2 };
+
 struct DeviceStatus {
   int code;
   int detail;
   int dirty;          // set by the integrator when a particle left its verlet box
   int overflow;
   long long haltAt;   // 0, or 1 + the step whose integrator raised the collider trigger (see haltedIntegrator)
+  int scanFailed;     // a prefix sum gave up its wait (k_scan): nothing may index by what was computed from it
+  unsigned totals[2];  // totals of the rebuild's scans: box pairs (periodic: candidates, then pairs), retained contacts
   unsigned long long pairTotal;
   unsigned long long ellSolves, ellIters, ellFallbacks;  // ellipsoid solves / Newton iterations (Brent: evaluations) / MLP fallbacks
   unsigned workCount;  // contact work list of this step: real contacts at work[0 .. workCount)
@@ -248,7 +253,6 @@ struct DeviceStatus {
   unsigned touchCount; // length of the touched-particle list of this step
   unsigned long long dynNotMin;  // DynDt: ~bits of the smallest nodal critical step^2 (0: none yet)
   unsigned actCount;   // length of the contact cull's active list
-  double ext[12];     // box extents reduction scratch (as ordered ints)
   long long stepBase;  // graph replays: Scene.step of the replay's first step
   long long seqBase;   //   and the contact-pass number before it
   unsigned sumTickets[9];  // blocks done per row of the running sums (left at 0)
@@ -277,13 +281,14 @@ __device__ __forceinline__ long long stepOf(const StepParams& P, const DeviceSta
 __device__ __forceinline__ long long seqOf(const StepParams& P, const DeviceStatus* st) {
   return P.stepDev ? st->seqBase + P.seq : P.seq;
 }
+// A failed scan (scanFailed) halts them too: the host learns of it with the status word at the end of the queue.
 __device__ __forceinline__ bool haltedIntegrator(const DeviceStatus* st, long long step) {
   const long long h = st->haltAt;
-  return h != 0 && h <= step;
+  return (h != 0 && h <= step) || st->scanFailed != 0;
 }
 __device__ __forceinline__ bool haltedContacts(const DeviceStatus* st, long long step) {
   const long long h = st->haltAt;
-  return h != 0 && h <= step + 1;
+  return (h != 0 && h <= step + 1) || st->scanFailed != 0;
 }
 #endif
 
@@ -359,6 +364,10 @@ void launch_contacts(cudaStream_t s, const StepParams& P, Particles p, Contacts 
                      bool full, const uint16_t* warmBf = nullptr, const float* warmF = nullptr);
 void launch_init_uploaded(cudaStream_t s, const StepParams& P, Particles p, Contacts c, long long nc);
 // ---- collider (k_collider.cu) ----
+// A wait of k_scan looks this often, with 20 ns and a load between two looks: about a second.
+constexpr int SCAN_LOOKS = 1 << 20;
+// where the total of a scan goes in DeviceStatus.totals, besides the end of the array
+enum { TOTAL_NONE = -1, TOTAL_PAIRS = 0, TOTAL_RETAINED = 1 };
 struct ColliderScratch {
   unsigned long long *keys, *keysAlt;   // sorts of the bodies, the history carry and the CSR entries
   unsigned *vals, *valsAlt;
@@ -366,6 +375,7 @@ struct ColliderScratch {
   unsigned* scanScratch;                // ticket and tile status words of the scans (scan_scratch_words)
   long long scanCap;
   unsigned scanEpoch, scanTickets;      // number of the last scan, tickets its predecessors took
+  int scanLooks = SCAN_LOOKS;           // looks of one wait of a scan before it gives up
   int* largeIdx;                        // N: index of a body in `large`, -1 for the others
   unsigned* rowSub;                     // 2N: entry counts of the large bodies' partner ranges (k_csr_large)
   unsigned* cellStart;                  // first sorted body of each bucket (maxCols + 1; 16-byte aligned)
@@ -397,7 +407,7 @@ void launch_bboxes(cudaStream_t s, const StepParams& P, Particles p, int n);
 void col_extents_and_grid(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs);
 void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs);
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out,
-               long long cap, bool write, DeviceStatus* st);
+               long long cap, bool write);
 // periodic collider: 3-D cell grid, FP32 candidates, exact spatialOverlapPeri, emission
 void col_periodic_cand(cudaStream_t s, const StepParams& P, Particles p, const int* small, int nSmall,
                        ColliderScratch& cs, bool write);
@@ -442,8 +452,10 @@ long long scan_scratch_words(long long n);
 // sort scratch (sized for 2 nNew) as temporary storage
 void col_carry_compact(cudaStream_t s, Particles p, Contacts neu, long long nNew, Contacts old, Csr csr, int nRowsOld,
                        int n, long long step, int nHist, ColliderScratch& cs);
-// exclusive scan of a[0..n) in place; a[n] receives the total (the array holds n+1 entries)
-void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs);
+// exclusive scan of a[0..n) in place; a[n] (the array holds n+1 entries) and DeviceStatus.totals[total] receive the
+// total.  A wait that runs out sets DeviceStatus.scanFailed: every kernel that indexes by scanned values returns
+// at once then, and so do the steps queued behind them.
+void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratch& cs, int total = TOTAL_NONE);
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
