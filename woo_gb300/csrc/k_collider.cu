@@ -350,6 +350,7 @@ static const int SCAN_T = 256, SCAN_I = 16, SCAN_TILE = SCAN_T * SCAN_I;
 static const unsigned SCAN_AGG = 1u, SCAN_PRE = 2u, SCAN_EPOCHS = 1u << 30;
 __device__ __forceinline__ void scanGaveUp(DeviceStatus* st) {
   st->scanFailed = 1;
+  st->haltAt = -1;
   if (atomicCAS(&st->code, 0, WDEM_ERR_TIMEOUT) == 0) st->detail = DETAIL_SCAN;
 }
 

@@ -242,7 +242,8 @@ struct DeviceStatus {
   int detail;
   int dirty;          // set by the integrator when a particle left its verlet box
   int overflow;
-  long long haltAt;   // 0, or 1 + the step whose integrator raised the collider trigger (see haltedIntegrator)
+  long long haltAt;   // 0, or 1 + the step whose integrator raised the collider trigger (see haltedIntegrator); -1: a
+                      //   scan failed
   int scanFailed;     // a prefix sum gave up its wait (k_scan): nothing may index by what was computed from it
   unsigned totals[2];  // totals of the rebuild's scans: box pairs (periodic: candidates, then pairs), retained contacts
   unsigned long long pairTotal;
@@ -281,14 +282,14 @@ __device__ __forceinline__ long long stepOf(const StepParams& P, const DeviceSta
 __device__ __forceinline__ long long seqOf(const StepParams& P, const DeviceStatus* st) {
   return P.stepDev ? st->seqBase + P.seq : P.seq;
 }
-// A failed scan (scanFailed) halts them too: the host learns of it with the status word at the end of the queue.
+// A failed scan halts all steps (haltAt -1); the host learns of it with the status word at the end of the queue.
 __device__ __forceinline__ bool haltedIntegrator(const DeviceStatus* st, long long step) {
   const long long h = st->haltAt;
-  return (h != 0 && h <= step) || st->scanFailed != 0;
+  return h != 0 && h <= step;
 }
 __device__ __forceinline__ bool haltedContacts(const DeviceStatus* st, long long step) {
   const long long h = st->haltAt;
-  return (h != 0 && h <= step + 1) || st->scanFailed != 0;
+  return h != 0 && h <= step + 1;
 }
 #endif
 
