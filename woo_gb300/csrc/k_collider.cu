@@ -257,6 +257,7 @@ struct GridArgs {
   int maxCols, maxBuckets, qbits;
   GridParams* grid;  // null: periodic
   PeriGrid* peri;
+  DeviceStatus* st;
 };
 static const int EXT_T = 256;
 __global__ void __launch_bounds__(EXT_T) k_extents(StepParams P, Particles p, const int* small, int nSmall,
@@ -293,6 +294,7 @@ __global__ void __launch_bounds__(EXT_T) k_extents(StepParams P, Particles p, co
   __syncthreads();
   if (!last || threadIdx.x != 0) return;
   __threadfence();
+  A.st->longBucket = 0;
   unsigned long long e[EXT_VALUES];
   for (int q = 0; q < EXT_VALUES; q++) e[q] = *(volatile unsigned long long*)(ext + q);
   if (A.peri) gridSetupPeri(e, P, A.maxBuckets, A.peri);
@@ -477,15 +479,27 @@ void exclusive_scan_u32(cudaStream_t s, unsigned* a, long long n, ColliderScratc
 // within their buckets, which hold a body or two (sweep keys) or a cell's handful (periodic).  The start of any key
 // is then a table lookup for the sweep.  An LSD radix sort of the keys took 4 passes of 8 bits, each a
 // dependent launch of 10 us at 15k bodies and 25 us at 500k.
+//
+// Ranking costs a bucket the square of its length.  A body far from all others stretches the grid (its columns are
+// widened until they are no more than the buckets) and the others share few buckets: 100k spheres with one 100 edge
+// lengths away along each axis have 9,212 in a bucket, 1M with one 10,000 away along two axes 503,892.  The sweep
+// kernel's start in a neighbouring column is bisected for the same reason.  Above BUCKET_RANKED the bodies are sorted
+// by merges instead (col_sort_merge; k_bucket_place tells, the count behind it is void and made again).  Rebuild in
+// ms, ranked and merged, by the longest bucket: 423 0.178 and 0.237, 1175 0.258 and 0.292 (100k bodies); 2500 1.48
+// and 1.31, 12,100 8.9 and 6.9, 503,892 149 and 19.0 (1M; a radix sort with bisection 20.4).  A cell of the periodic
+// grid is no smaller than the widest box, and the walk over its candidates is quadratic too and 14 times as long:
+// always ranked.
+static const unsigned BUCKET_RANKED = 2048;
 __global__ void k_bucket_place(const int* small, int nSmall, const unsigned* keys, const unsigned* place,
-                               const unsigned* start, const GridParams* g, unsigned long long* tmp,
-                               const DeviceStatus* st) {
+                               const unsigned* start, const GridParams* g, unsigned long long* tmp, DeviceStatus* st) {
   chainWait(false);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nSmall || st->scanFailed) return;
   const unsigned key = keys[k];
   const unsigned b = g ? key >> (g->qbits - g->kbits) : key;
-  tmp[start[b] + place[k]] = ((unsigned long long)key << 32) | (unsigned)small[k];
+  const unsigned first = start[b];
+  tmp[first + place[k]] = ((unsigned long long)key << 32) | (unsigned)small[k];
+  if (g && start[b + 1] - first > BUCKET_RANKED) st->longBucket = 1;
 }
 __device__ __forceinline__ unsigned rankInBucket(const unsigned long long* tmp, unsigned long long v, unsigned beg, unsigned end) {
   unsigned pos = beg;
@@ -496,22 +510,64 @@ __device__ __forceinline__ unsigned rankInBucket(const unsigned long long* tmp, 
 // the maximum rounded up (every pair of FP64 boxes that overlap overlaps in FP32 too, so a pair the FP32
 // test rejects needs no FP64 test), the mask (lo.w) and meta.x with shape and scene (hi.w).  The sweep
 // walks these contiguous records instead of gathering meta, bbmin and bbmax by particle id.
+template <bool SORTED>
 __global__ void k_bucket_rank(Particles p, int nSmall, const unsigned long long* tmp, const unsigned* start,
                               const GridParams* g, unsigned* keys, unsigned* vals, float4* rec, const DeviceStatus* st) {
   chainWait(false);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nSmall || st->scanFailed) return;
+  if (e >= nSmall || st->scanFailed || (!SORTED && st->longBucket)) return;
   const unsigned long long v = tmp[e];
   const unsigned key = (unsigned)(v >> 32);
   const int i = (int)(unsigned)v;
   const double4_32a mn = p.bbmin[i], mx = p.bbmax[i];
   const int4 m = p.meta[i];
-  const unsigned b = key >> (g->qbits - g->kbits);
-  const unsigned s = rankInBucket(tmp, v, start[b], start[b + 1]);
+  unsigned s = (unsigned)e;
+  if (!SORTED) {
+    const unsigned b = key >> (g->qbits - g->kbits);
+    s = rankInBucket(tmp, v, start[b], start[b + 1]);
+  }
   keys[s] = key;
   vals[s] = (unsigned)i;
   rec[2 * s] = make_float4(__double2float_rd(mn.x), __double2float_rd(mn.y), __double2float_rd(mn.z), __uint_as_float((unsigned)m.z));
   rec[2 * s + 1] = make_float4(__double2float_ru(mx.x), __double2float_ru(mx.y), __double2float_ru(mx.z), __int_as_float(m.x));
+}
+
+// The bodies sorted by merges: tiles of SORT_TILE by a bitonic network in shared memory, then runs of twice the length
+// a pass, every entry finding its place in the neighbouring run by bisection (entries are all different).
+static const int SORT_T = 256, SORT_TILE = 2048;
+__global__ void __launch_bounds__(SORT_T) k_tile_sort(const unsigned long long* in, unsigned long long* out, int n) {
+  chainWait(false);
+  __shared__ unsigned long long v[SORT_TILE];
+  const int base = blockIdx.x * SORT_TILE;
+  for (int k = threadIdx.x; k < SORT_TILE; k += SORT_T) v[k] = base + k < n ? in[base + k] : ~0ull;
+  for (int size = 2; size <= SORT_TILE; size *= 2)
+    for (int step = size / 2; step > 0; step /= 2) {
+      __syncthreads();
+      for (int q = threadIdx.x; q < SORT_TILE / 2; q += SORT_T) {
+        const int a = 2 * q - (q & (step - 1)), b = a + step;
+        const unsigned long long x = v[a], y = v[b];
+        if ((x > y) == ((a & size) == 0)) { v[a] = y; v[b] = x; }
+      }
+    }
+  __syncthreads();
+  for (int k = threadIdx.x; k < SORT_TILE; k += SORT_T)
+    if (base + k < n) out[base + k] = v[k];
+}
+__global__ void k_merge_runs(const unsigned long long* in, unsigned long long* out, int n, int run) {
+  chainWait(false);
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const unsigned long long v = in[e];
+  const int first = e / run * run;                          // of this entry's run
+  const bool left = (e / run) % 2 == 0;
+  int lo = left ? min(first + run, n) : first - run;        // the other run
+  int hi = left ? min(first + 2 * (long long)run, (long long)n) : first;
+  const int other = lo;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (in[mid] < v) lo = mid + 1; else hi = mid;
+  }
+  out[(left ? e : e - run) + (lo - other)] = v;
 }
 
 // ------------------------------------------------------------------------------------ sweep
@@ -580,7 +636,7 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
                         const DeviceStatus* st) {
   chainWait(false);
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= sweepThreads(A.nSmall, A.nLarge) || st->scanFailed) return;
+  if (s >= sweepThreads(A.nSmall, A.nLarge) || st->scanFailed || st->longBucket) return;
   unsigned cnt = 0;
   unsigned long long base = WRITE ? counts[s] : 0;
   if (WRITE && A.buf) {
@@ -649,13 +705,14 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
       int q;
       if (c2 == col) q = s + 1;
       else {
-        // the first box of the column after (key, id): from its bucket's start
-        const unsigned target = ((unsigned)c2 << G.qbits) | qi;
-        q = (int)A.start[target >> kshift];
-        while (q < end) {
-          const unsigned kq = A.keys[q];
-          if (kq > target || (kq == target && (int)A.vals[q] >= i)) break;
-          q++;
+        // the first box of the column after (key, id): bisected within its bucket
+        const unsigned target = ((unsigned)c2 << G.qbits) | qi, b = target >> kshift;
+        q = (int)A.start[b];
+        int to = (int)A.start[b + 1];
+        while (q < to) {
+          const int mid = (q + to) >> 1;
+          const unsigned km = A.keys[mid];
+          if (km < target || (km == target && (int)A.vals[mid] < i)) q = mid + 1; else to = mid;
         }
       }
       for (; q < end; q++) {
@@ -1215,7 +1272,7 @@ static void launchExtents(cudaStream_t s, const StepParams& P, Particles p, cons
 
 // The collider sub-steps are called from wdem_api.cu through these thin wrappers.
 void col_extents_and_grid(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs) {
-  GridArgs A{sweepCols(cs, nSmall), maxBuckets(cs, nSmall), sweepQbits(cs, nSmall), cs.grid, nullptr};
+  GridArgs A{sweepCols(cs, nSmall), maxBuckets(cs, nSmall), sweepQbits(cs, nSmall), cs.grid, nullptr, cs.st};
   launchExtents(s, StepParams{}, p, small, nSmall, cs, A);
 }
 
@@ -1228,7 +1285,21 @@ void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, Collide
   launchChained(k_make_keys, blocks, 256, s, p, small, nSmall, cs.grid, a.keyIn, a.place, a.start);
   exclusive_scan_u32(s, a.start, nb, cs);
   launchChained(k_bucket_place, blocks, 256, s, small, nSmall, a.keyIn, a.place, a.start, cs.grid, a.tmp, cs.st);
-  launchChained(k_bucket_rank, blocks, 256, s, p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec, cs.st);
+  launchChained(k_bucket_rank<false>, blocks, 256, s, p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec, cs.st);
+}
+
+void col_sort_merge(cudaStream_t s, Particles p, int nSmall, ColliderScratch& cs) {
+  const SortArrays a = sortArrays(cs);
+  const unsigned blocks = (unsigned)((nSmall + 255) / 256);
+  // the runs alternate between tmp and the array that k_bucket_rank writes, and end in tmp
+  unsigned long long* buf[2] = {a.tmp, cs.keys};
+  int passes = 0;
+  while (((long long)SORT_TILE << passes) < nSmall) passes++;
+  int at = passes & 1;
+  launchChained(k_tile_sort, (unsigned)((nSmall + SORT_TILE - 1) / SORT_TILE), SORT_T, s, a.tmp, buf[at], nSmall);
+  for (int k = 0; k < passes; k++, at ^= 1) launchChained(k_merge_runs, blocks, 256, s, buf[at], buf[at ^ 1], nSmall, SORT_TILE << k);
+  cudaMemsetAsync(&cs.st->longBucket, 0, sizeof(int), s);
+  launchChained(k_bucket_rank<true>, blocks, 256, s, p, nSmall, a.tmp, a.start, cs.grid, a.key, a.id, cs.srec, cs.st);
 }
 
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out, long long cap,
@@ -1268,7 +1339,7 @@ void col_periodic_cand(cudaStream_t s, const StepParams& P, Particles p, const i
   CandArgs A{a.key, cs.periC, cs.periH, a.start, cs.sweepBufCap >= nSmall ? cs.sweepBuf : nullptr, nSmall};
   if (!write) {
     const int nb = maxBuckets(cs, nSmall);
-    GridArgs GA{0, nb, 0, nullptr, g};
+    GridArgs GA{0, nb, 0, nullptr, g, cs.st};
     launchExtents(s, P, p, small, nSmall, cs, GA);
     cudaMemsetAsync(a.start, 0, ((size_t)nb + 1) * sizeof(unsigned), s);
     if (nSmall > 0) {

@@ -475,6 +475,23 @@ int readTotals(wdem_handle* h) {
   return h->hst->scanFailed ? checkDeviceStatus(h) : WDEM_OK;
 }
 
+// The aperiodic box pairs counted (totals[TOTAL_PAIRS], with what else was scanned before).  Bodies are sorted by ranking
+// buckets of a few; where one body far from the others stretches the grid until a bucket holds hundreds, the count is
+// void and is made again after a sort by merges.
+void countPairs(wdem_handle* h, unsigned loneMask) {
+  ColliderScratch& cs = h->cs;
+  const int nSmall = (int)h->smallIds.size();
+  col_sweep(h->stream, h->d, nSmall, loneMask, cs, nullptr, 0, false);
+  exclusive_scan_u32(h->stream, cs.counts, sweepThreads(nSmall, cs.nLarge), cs, TOTAL_PAIRS);
+}
+int readPairTotals(wdem_handle* h, unsigned loneMask) {
+  int rc;
+  if ((rc = readTotals(h)) || !h->hst->longBucket) return rc;  // (never set by the periodic collider)
+  col_sort_merge(h->stream, h->d, (int)h->smallIds.size(), h->cs);
+  countPairs(h, loneMask);
+  return readTotals(h);
+}
+
 // Collider rebuild: InsertionSortCollider full run (InsertionSortCollider.cpp:407-612).
 int rebuild(wdem_handle* h) {
   cudaStream_t s = h->stream;
@@ -484,7 +501,6 @@ int rebuild(wdem_handle* h) {
   int rc;
   if ((rc = ensureScratch(h, h->nContacts))) return rc;
   launch_bboxes(s, h->P, h->d, n);
-  const int nSweep = sweepThreads(nSmall, cs.nLarge);
   long long nCand = 0;
   if (h->periodic) {
     col_periodic_cand(s, h->P, h->d, h->dSmall, nSmall, cs, false);
@@ -496,14 +512,13 @@ int rebuild(wdem_handle* h) {
   } else {
     col_extents_and_grid(s, h->d, h->dSmall, nSmall, cs);
     col_sort(s, h->d, h->dSmall, nSmall, cs);
-    col_sweep(s, h->d, nSmall, h->P.loneMask, cs, nullptr, 0, false);
-    exclusive_scan_u32(s, cs.counts, nSweep, cs, TOTAL_PAIRS);
+    countPairs(h, h->P.loneMask);
   }
   ContactBuf& old = h->buf[h->cur];
   ContactBuf& neu = h->buf[1 - h->cur];
   const long long nOld = h->nContacts;
   col_retain_flags(s, h->P, h->d, old.c, nOld, cs);
-  if ((rc = readTotals(h))) return rc;
+  if ((rc = readPairTotals(h, h->P.loneMask))) return rc;
   const long long total = h->hst->totals[TOTAL_PAIRS];
   const long long retained = h->hst->totals[TOTAL_RETAINED];
   const long long nNew = total + retained;
@@ -1774,10 +1789,8 @@ int wdem_collide_boxes(wdem_handle* h, int32_t n, const double* mins, const doub
   ColliderScratch& cs = h->cs;
   col_extents_and_grid(s, h->d, h->dSmall, nSmall, cs);
   col_sort(s, h->d, h->dSmall, nSmall, cs);
-  col_sweep(s, h->d, nSmall, loneMask, cs, nullptr, 0, false);
-  const int nSweep = sweepThreads(nSmall, cs.nLarge);
-  exclusive_scan_u32(s, cs.counts, nSweep, cs, TOTAL_PAIRS);
-  if ((rc = readTotals(h))) return rc;
+  countPairs(h, loneMask);
+  if ((rc = readPairTotals(h, loneMask))) return rc;
   long long total = h->hst->totals[TOTAL_PAIRS];
   int2* dpairs = nullptr;
   CK(dalloc(dpairs, (size_t)total + 1));

@@ -245,6 +245,7 @@ struct DeviceStatus {
   long long haltAt;   // 0, or 1 + the step whose integrator raised the collider trigger (see haltedIntegrator); -1: a
                       //   scan failed
   int scanFailed;     // a prefix sum gave up its wait (k_scan): nothing may index by what was computed from it
+  int longBucket;     // a bucket of the collider's sort is too long to be ranked (k_bucket_place)
   unsigned totals[2];  // totals of the rebuild's scans: box pairs (periodic: candidates, then pairs), retained contacts
   unsigned long long pairTotal;
   unsigned long long ellSolves, ellIters, ellFallbacks;  // ellipsoid solves / Newton iterations (Brent: evaluations) / MLP fallbacks
@@ -407,6 +408,8 @@ struct ColliderScratch {
 void launch_bboxes(cudaStream_t s, const StepParams& P, Particles p, int n);
 void col_extents_and_grid(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs);
 void col_sort(cudaStream_t s, Particles p, const int* small, int nSmall, ColliderScratch& cs);
+// the sort again, by merges, after col_sort met a bucket too long to rank (DeviceStatus.longBucket)
+void col_sort_merge(cudaStream_t s, Particles p, int nSmall, ColliderScratch& cs);
 void col_sweep(cudaStream_t s, Particles p, int nSmall, unsigned loneMask, ColliderScratch& cs, int2* out,
                long long cap, bool write);
 // periodic collider: 3-D cell grid, FP32 candidates, exact spatialOverlapPeri, emission
