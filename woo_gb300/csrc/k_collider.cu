@@ -1026,8 +1026,8 @@ __global__ void k_keys_peri(StepParams P, Particles p, const int* small, int nSm
     const double w = ctr - per * L;
     c[a] = (float)w;
     h[a] = (float)half;
-    // beyond 2^30 periods (also infinite and NaN): the exact test decides
-    wide |= !(half < .25 * L) || !(fabs(per) < 1073741824.0);
+    // far out (also infinite and NaN): the exact test decides
+    wide |= !(half < .25 * L) || !(fabs(per) < WDEM_PERI_PERIODS);
     f[a] = wide ? 0 : (int)per;
     cell[a] = (int)fmin(fmax(floor(w * G.invCw[a]), 0.0), (double)(G.nc[a] - 1));
   }

@@ -50,10 +50,15 @@ __device__ __forceinline__ float periDist(float c1, float c2, float L, float inv
   return fabsf(d - L * rintf(d * invL));
 }
 // Rounding of the copies and of this arithmetic, u = 2^-24: the two centres (wrapped to [0, L)) u L each, their
-// difference and L's own copy u L each, the half-widths (below L / 4) and their sum u L together: about 5 u L = 3e-7 L.
-// The margin is three times that; pairs within it take the FP64 test, which costs a warp as much for one lane as
+// difference and L's own copy u L each, the half-widths (below L / 4) and their sum u L together: about 5 u L.
+// The reference's test rounds too: min + L at the magnitude of min, M periods out, changes the period it divides by
+// by up to M 2^-53 of itself, which N periods between the bodies make N M 2^-53 L.  The screens decide for bodies
+// less than WDEM_PERI_PERIODS periods out only, where that (and the FP64 rounding of centres and half-widths) is at
+// most 2^15 2^14 2^-53 L = u L.  Together 6 u L = 3.6e-7 L.
+// The margin is nearly three times that; pairs within it take the FP64 test, which costs a warp as much for one lane as
 // for 32 (a margin of 1e-5 L sent 15 % of the warps of a dense packing of 400k there, 90 of 121 us of the pass).
 #define WDEM_PERI_MARGIN 1e-6f
+#define WDEM_PERI_PERIODS 16384.0
 // the boxes are disjoint on this axis for every period shift
 __device__ __forceinline__ bool periFar(float c1, float h1, float c2, float h2, float L, float invL) {
   return periDist(c1, c2, L, invL) > h1 + h2 + WDEM_PERI_MARGIN * L;
