@@ -427,7 +427,8 @@ int wdem_add_particles(wdem_handle* h, const wdem_particles* p, const int32_t* i
 /* Launch shape of the step kernels (no counterpart in the reference, which has none): threads per block of
  * the contact pass's FP64 kernel (64, 128, 256), its resident blocks per SM (0 = as many as fit), threads
  * per block of the contact cull (128, 256, 512) and of the integrator's first pass (128, 256, 512), blocks
- * per SM of the integrator's list pass (0 = as many as fit).  Results do not depend on the shape (every
+ * per SM of the integrator's list pass (0 = as many as fit).  With the defaults of the last two (256, 0) a
+ * scene of up to 256 bodies per SM is integrated in one launch; any other pair gives it the two passes.  Results do not depend on the shape (every
  * contact and particle is computed alone; sums run in fixed orders): only the speed does. */
 typedef struct wdem_launch_shape {
   int32_t contactsBlock;

@@ -902,7 +902,8 @@ void launch_leapfrog(cudaStream_t s, const StepParams& P, Particles p, int n, in
   const unsigned listBlocks = (unsigned)((n + LIST_ITEMS - 1) / LIST_ITEMS);
   if (!fromArrays && !P.hasEll && !P.lfEnergy) {
     const int sms = P.numSMs > 0 ? P.numSMs : 152;
-    if (n <= ALL_PER_SM * sms) {
+    const bool shaped = P.shLeapBlock != 256 || P.shListsPerSM != 0;  // a launch shape of the two passes was asked for
+    if (n <= ALL_PER_SM * sms && !shaped) {
       if (P.periodic) launchChained(k_leapfrog_all<true>, listBlocks, LIST_T, s, P, p, n, c, csr, st);
       else launchChained(k_leapfrog_all<false>, listBlocks, LIST_T, s, P, p, n, c, csr, st);
       return;
