@@ -2189,17 +2189,22 @@ int mlpEnsure(wdem_handle* h) {
   return WDEM_OK;
 }
 // device buffer of the network's inputs and outputs, kept from call to call up to WARM_IO_KEEP bytes (allocating and
-// freeing it took a third of a gradient call on 64k records); a larger call's buffer is given back by the next
-// smaller one
-const long long WARM_IO_KEEP = 256ll << 20;
+// freeing it took a third of a gradient call on 64k records, 4.5 MB); a larger call's buffer is given back when the
+// call ends
+const long long WARM_IO_KEEP = 32ll << 20;
 int ensureWarmIO(wdem_handle* h, long long floats) {
-  const bool tooLarge = h->warmIOCap * (long long)sizeof(float) > WARM_IO_KEEP && 2 * floats < h->warmIOCap;
-  if (floats > h->warmIOCap || tooLarge) {
+  if (floats > h->warmIOCap) {
     h->warmIOCap = 0;
     CK(dalloc(h->warmIO, (size_t)floats));
     h->warmIOCap = floats;
   }
   return WDEM_OK;
+}
+void releaseWarmIO(wdem_handle* h) {
+  if (h->warmIOCap * (long long)sizeof(float) <= WARM_IO_KEEP) return;
+  cudaFree(h->warmIO);
+  h->warmIO = nullptr;
+  h->warmIOCap = 0;
 }
 int mlpUpload(wdem_handle* h, const std::vector<float>& pad) {
   const int n = mlp_npad();
@@ -2274,6 +2279,7 @@ int wdem_warm_predict(wdem_handle* h, const float* x, int64_t n, float* y) {
   cudaMemcpyAsync(y, dy, (size_t)n * WDEM_WARM_OUTPUTS * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
   cudaMemcpyAsync(h->hst, h->dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
+  releaseWarmIO(h);
   if (e != cudaSuccess) return fail(h, WDEM_ERR_CUDA, cudaGetErrorString(e));
   if ((rc = checkDeviceStatus(h))) return rc;
   return WDEM_OK;
@@ -2296,6 +2302,7 @@ int wdem_warm_grad(wdem_handle* h, const float* records, int64_t n, float* grad,
   cudaMemsetAsync(h->mlpGrad, 0, mlp_npad() * sizeof(float), h->stream);
   cudaMemcpyAsync(h->hst, h->dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
+  releaseWarmIO(h);
   if (e != cudaSuccess) return fail(h, WDEM_ERR_CUDA, cudaGetErrorString(e));
   if ((rc = checkDeviceStatus(h))) return rc;
   mlp_pack(pad.data(), grad);
