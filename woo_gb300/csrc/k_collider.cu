@@ -596,22 +596,30 @@ __device__ __forceinline__ bool overlapF(const float4& mn1, const float4& mx1, c
 // itself and the difference of two rounds by 2^-24, so a closed FP64 interval test holds when every difference of a
 // maximum and a minimum exceeds 4e-7 of their magnitudes.  An FP64 compare holds a scheduler for 64 cycles whichever
 // lanes need it, and the six of a box pair ran in nearly every round of a warp's walk: 175 of the 217 us of the
-// sweep over 508k bodies.  NaN fails.
-__device__ __forceinline__ bool clearlyAbove(float mx, float mn) { return mx - mn > 4e-7f * (fabsf(mx) + fabsf(mn)); }
+// sweep over 508k bodies.  NaN fails.  The added 1e-37 is for magnitudes near FP32's subnormals, which round to
+// multiples of 2^-149.
+__device__ __forceinline__ bool clearlyAbove(float mx, float mn) { return mx - mn > __fmaf_rn(4e-7f, fabsf(mx) + fabsf(mn), 1e-37f); }
 __device__ __forceinline__ bool overlapSure(const float4& mn1, const float4& mx1, const float4& mn2, const float4& mx2) {
   return clearlyAbove(mx2.x, mn1.x) && clearlyAbove(mx1.x, mn2.x) && clearlyAbove(mx2.y, mn1.y) && clearlyAbove(mx1.y, mn2.y) &&
          clearlyAbove(mx2.z, mn1.z) && clearlyAbove(mx1.z, mn2.z);
 }
-// a bound of a large body in FP32, within 2^-23 of itself, on the integer pipe (infinities and NaN kept)
+// a bound of a large body in FP32, within 2^-23 of itself, on the integer pipe: infinities kept; NaN for NaN and for
+// what only FP64 can hold, so that every test on it fails and the FP64 test decides
 __device__ __forceinline__ float boundF(double x) {
   const Halves h = halvesOf(x);
-  if ((h.hi & 0x7ff00000u) == 0x7ff00000u)
-    return __uint_as_float((h.hi & 0x80000000u) | 0x7f800000u | ((h.hi & 0xfffffu) | h.lo ? 0x400000u : 0u));
+  const unsigned a = h.hi & 0x7fffffffu;
+  if (a >= 0x47f00000u)  // 2^128
+    return __uint_as_float(a == 0x7ff00000u && h.lo == 0 ? (h.hi & 0x80000000u) | 0x7f800000u : 0x7fc00000u);
   return truncF(x);
 }
-// clearlyAbove for bounds that may be infinite (the difference is infinite too, and the margin is not used)
-__device__ __forceinline__ bool aboveOrInf(float mx, float mn) {
-  return mx == __int_as_float(0x7f800000) || mn == -__int_as_float(0x7f800000) || clearlyAbove(mx, mn);
+// clearlyAbove where the large body's bound, the first argument, is infinite: beyond any bound of a small body, whose
+// copy may be infinite too but stands for a finite number (NaN fails)
+__device__ __forceinline__ bool infAbove(float mx, float fmn) { return mx == __int_as_float(0x7f800000) && fmn < mx; }
+__device__ __forceinline__ bool infBelow(float mn, float fmx) { return mn == -__int_as_float(0x7f800000) && fmx > mn; }
+__device__ __forceinline__ bool overlapSureLarge(const float4& fmn, const float4& fmx, const float4& gn, const float4& gx) {
+  return (infAbove(gx.x, fmn.x) || clearlyAbove(gx.x, fmn.x)) && (infBelow(gn.x, fmx.x) || clearlyAbove(fmx.x, gn.x)) &&
+         (infAbove(gx.y, fmn.y) || clearlyAbove(gx.y, fmn.y)) && (infBelow(gn.y, fmx.y) || clearlyAbove(fmx.y, gn.y)) &&
+         (infAbove(gx.z, fmn.z) || clearlyAbove(gx.z, fmn.z)) && (infBelow(gn.z, fmx.z) || clearlyAbove(fmx.z, gn.z));
 }
 
 struct SweepArgs {
@@ -745,8 +753,7 @@ __global__ void k_sweep(Particles p, SweepArgs A, const GridParams* g, unsigned*
     if (clearlyAbove(gn.x, fmx.x) || clearlyAbove(fmn.x, gx.x) || clearlyAbove(gn.y, fmx.y) || clearlyAbove(fmn.y, gx.y) ||
         clearlyAbove(gn.z, fmx.z) || clearlyAbove(fmn.z, gx.z))
       continue;
-    if (!(aboveOrInf(gx.x, fmn.x) && aboveOrInf(fmx.x, gn.x) && aboveOrInf(gx.y, fmn.y) && aboveOrInf(fmx.y, gn.y) &&
-          aboveOrInf(gx.z, fmn.z) && aboveOrInf(fmx.z, gn.z))) {
+    if (!overlapSureLarge(fmn, fmx, gn, gx)) {
       WDEM_REAL_BRANCH();
       if (!overlap3(mn, mx, ln, lx)) continue;
     }
