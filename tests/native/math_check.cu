@@ -34,3 +34,20 @@ extern "C" int math_eval(int what, const double* x, const double* y, double* out
   cudaFree(d);
   return (int)cudaGetLastError();
 }
+__global__ void k_quat(const double* c, double* out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double* m = c + 9 * (size_t)i;
+  const qd q = quatFromCols(mk(m[0], m[1], m[2]), mk(m[3], m[4], m[5]), mk(m[6], m[7], m[8]));
+  out[4 * (size_t)i] = q.w; out[4 * (size_t)i + 1] = q.x; out[4 * (size_t)i + 2] = q.y; out[4 * (size_t)i + 3] = q.z;
+}
+// quaternions (4n) of n frames given by their columns (9n)
+extern "C" int quat_eval(const double* c, double* out, int n) {
+  double* d = nullptr;
+  if (cudaMalloc((void**)&d, 13 * (size_t)n * sizeof(double)) != cudaSuccess) return 1;
+  cudaMemcpy(d, c, 9 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice);
+  k_quat<<<(n + 255) / 256, 256>>>(d, d + 9 * (size_t)n, n);
+  cudaMemcpy(out, d + 9 * (size_t)n, 4 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return (int)cudaGetLastError();
+}
