@@ -753,9 +753,8 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
         double ftSq = fy * fy + fz * fz;
         if (ftSq > maxFt * maxFt && !P.noSlip) {
 #ifdef WDEM_FMA
-          const double rn = rsqrtFast(ftSq);
-          double FtNorm = ftSq * rn;
-          double ratio = maxFt * rn;
+          double ratio = maxFt * rsqrtFast(ftSq);
+          double FtNorm = P.trackEnergy ? sqrtRefined(ftSq) : 0.;  // read by the dissipated energy only
 #else
           double FtNorm = sqrt(ftSq);
           double ratio = maxFt / FtNorm;
@@ -819,8 +818,8 @@ __device__ __forceinline__ void contactBody(const StepParams& P, const Particles
       double ftSq = fy * fy + fz * fz;
       if (ftSq > maxFt * maxFt) {
 #ifdef WDEM_FMA
-        const double rn = rsqrtFast(ftSq);  // ftSq > 0 here
-        const double FtNorm = ftSq * rn, ratio = maxFt * rn;
+        const double ratio = maxFt * rsqrtFast(ftSq);  // ftSq > 0 here
+        const double FtNorm = P.trackEnergy ? sqrtRefined(ftSq) : 0.;
 #else
         double FtNorm = sqrt(ftSq);
         double ratio = maxFt / FtNorm;
