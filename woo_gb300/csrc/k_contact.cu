@@ -1150,7 +1150,7 @@ template <int LAW, int CP2, bool PERI, bool ELL, int BS, bool DW = false>
 __global__ void __launch_bounds__(BS, 512 / BS) k_contacts(StepParams P, Particles p, Contacts c, const unsigned* work,
                                                         const unsigned* count, long long nc, DeviceStatus* st,
                                                         int part) {
-  chainWait(P.chainEarly);
+  chainWait(false);
   // part 0: the whole work list; 1: the real contacts at its front; 2: the potential pairs behind them
   const unsigned k0 = part == 2 ? count[0] : 0u;
   const unsigned m = part == 1 ? count[0] : workLen(count);
@@ -1302,7 +1302,7 @@ __device__ __forceinline__ void cullAppend(CullAppend<BS, FULL>& sh, int turn, u
 template <bool PERI, bool ELL, bool FULL, int BS>
 __global__ void __launch_bounds__(BS) k_contacts_cull(StepParams P, Particles p, Contacts c, long long nc,
                                                        unsigned* work, unsigned* count, DeviceStatus* st) {
-  chainWait(P.chainEarly);
+  chainWait(false);
   const long long first = (long long)blockIdx.x * blockDim.x;
   const long long m = FULL ? nc : (long long)st->actCount;
   // a step queued behind a collider trigger: the work list stays empty, so the heavy pass is a no-op too

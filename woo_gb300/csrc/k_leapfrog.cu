@@ -1192,7 +1192,7 @@ __global__ void __launch_bounds__(ER_T) k_sums(StepParams P, SumSet S, int row0,
   __shared__ double sh[ER_T];
   __shared__ bool last;
   const int y = row0 + blockIdx.y;
-  chainWait(P.chainEarly);
+  chainWait(false);
   if (S.guarded && (y < S.contactRow ? haltedIntegrator(st, stepOf(P, st)) : haltedContacts(st, stepOf(P, st)))) return;
   const long long n = S.n[y], nb = (n + ER_SLICE - 1) / ER_SLICE, blocks = nb > 0 ? nb : 1;
   if ((long long)blockIdx.x >= blocks) return;

@@ -565,7 +565,6 @@ void fillStepParams(wdem_handle* h) {
   P.shContactsBlock = h->launchShape.contactsBlock; P.shContactsPerSM = h->launchShape.contactsPerSM;
   P.shCullBlock = h->launchShape.cullBlock; P.shLeapBlock = h->launchShape.integratorBlock; P.shListsPerSM = h->launchShape.listsPerSM;
   P.numSMs = h->numSMs;
-  P.chainEarly = h->n > 256 * h->numSMs;
   for (int k = 0; k < 3; k++) P.gravity[k] = r.gravity[k];
   P.hasGravity = !(r.gravity[0] == 0 && r.gravity[1] == 0 && r.gravity[2] == 0);
   {

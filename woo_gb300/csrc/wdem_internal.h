@@ -108,7 +108,6 @@ struct StepParams {
   int hasFacets;            // the scene has facets
   int stepDev;              // 1: step and seq are offsets from DeviceStatus.stepBase/seqBase (steps replayed
                             // from a CUDA graph, whose kernel arguments are fixed at capture)
-  int chainEarly;           // the next kernel's blocks may start beside this one's (chainWait)
   int denseTouch;           // 1: real contacts were at least n/8 in the last step the host saw; the
                             // integrator's first pass then compacts each block's untouched particles
   double gravity[3];
@@ -298,10 +297,14 @@ __device__ __forceinline__ bool haltedContacts(const DeviceStatus* st, long long
 // The kernels of a step or a rebuild follow each other at once and some last only a few microseconds.  They are launched as
 // programmatic dependents: the next kernel is set up while this one ends, and each kernel waits for the one before
 // it (complete, its writes visible) before it touches memory.  early: the next kernel's blocks may take their places
-// as soon as this one's are all running.  The FP64 kernels of a small scene do not fill the GPU, and blocks placed
-// while others still run end up two to a scheduler: there the next kernel starts when this one's blocks have ended
-// (10k spheres: 59.1 us a step without any of this, 63.1 with early everywhere, 52.3 so; the collider's kernels never
-// trigger early: 15k spheres with a rebuild every 5 steps 73.3 us a step with plain launches in it, 65.5 so).
+// as soon as this one's are all running; otherwise when this one's blocks have ended.  Blocks placed while others
+// still run end up beside them on a scheduler whose FP64 pipe they share, and wait there: early in the cull, the
+// contact pass and the sums costs beds of every size (us a step, with it, without, and with plain launches; Frict
+// exact: 10k 56.8, 49.0; 38k 99.7, 94.1; 100k 198, 182, 192; 1M 1735, 1728, 1742; Hertz double-word: 100k 141, 138,
+// 149; 1M 895, 891, 900), and falling clouds (Hertz: 100k 75.5, 67.3, 75.7; 1M 394, 392, 402).  The integrators trigger early:
+// the cull behind them is short of FP64 work (falling: 60k 60.3 and 61.0 without; 700k 285.6 and 287.7; beds alike).
+// The collider's kernels never do (15k spheres with a rebuild every 5 steps: 73.3 us a step with plain launches in
+// it, 65.5 so).
 __device__ __forceinline__ void chainWait(bool early) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
