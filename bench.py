@@ -335,6 +335,21 @@ def read_profile_figures(tag):
 PHASE_KERNELS = {"contacts": ("k_contacts_cull", "k_contacts"), "leapfrog": ("k_leapfrog_fast", "k_leapfrog_lists")}
 PHASE_LABEL = {"contacts": "contact pass (k_contacts_cull + k_contacts: Cg2+Cp2+Law2)",
                "leapfrog": "integrator (k_leapfrog_fast + k_leapfrog_lists: CSR force gather + Leapfrog + verlet check)"}
+# the integrator of scenes of up to 256 bodies an SM (with the default launch shape), and of those with ellipsoids
+ONE_LAUNCH = (("k_leapfrog_all",), "integrator (k_leapfrog_all: CSR force gather + Leapfrog + verlet check)")
+GENERAL = (("k_leapfrog",), "integrator (k_leapfrog: CSR force gather + Leapfrog + verlet check)")
+
+
+def phase_kernels(h, spec, sms):
+    """{phase: (kernels, label)} of the scene's route."""
+    from woo_gb300 import abi
+    out = {ph: (PHASE_KERNELS[ph], PHASE_LABEL[ph]) for ph in PHASE_KERNELS}
+    shape = h.launch_shape()
+    if (spec.particles.shape == abi.SHAPE_ELLIPSOID).any():
+        out["leapfrog"] = GENERAL
+    elif spec.particles.n <= 256 * sms and (shape["integratorBlock"], shape["listsPerSM"]) == (256, 0):
+        out["leapfrog"] = ONE_LAUNCH
+    return out
 
 
 def measure_region(h, spec, args, world, local, barrier, region, clocks=None):
@@ -369,17 +384,18 @@ def measure_region(h, spec, args, world, local, barrier, region, clocks=None):
     hbm_peak, peak_kind = load_peaks()
     fp64_peak = h.fp64_peak()
     figs = read_profile_figures(state_tag(args, region, n))
+    kernels = phase_kernels(h, spec, torch.cuda.get_device_properties(local).multi_processor_count)
     rl = {}
     for ph, abytes in (("contacts", cbytes), ("leapfrog", lbytes)):
         k_ms, k_n = kt.get(ph, (0.0, 0))
         avg = k_ms / max(k_n, 1)
         ach = abytes / (avg / 1e3) / 1e9 if avg > 0 else 0.0
-        names = PHASE_KERNELS[ph]
+        names, label = kernels[ph]
         tr = [figs.get(f"{k}.dram_bytes_per_launch") for k in names]
         traffic = sum(tr) if all(t is not None for t in tr) else None
         dp = [figs.get(f"{k}.fp64_ops_per_launch") for k in names]
         dp_ops = sum(dp) if all(t is not None for t in dp) else None
-        rl[ph] = {"kernel": PHASE_LABEL[ph], "bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s",
+        rl[ph] = {"kernel": label, "bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s",
                   "frac": ach / hbm_peak, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                   "algorithmic_bytes_per_launch": abytes, "traffic": traffic,
                   "traffic_source": "ncu capture of this region's launches (same seeded run)" if traffic else None,
@@ -415,7 +431,7 @@ def e2e_measure(h, n, ne, world, local, barrier):
     ptrs = (pin["pos"].data_ptr(), pin["vel"].data_ptr(), pin["angVel"].data_ptr(), pin["ori"].data_ptr())
     h.read_state(n, *ptrs)
     bytes_io = n * (3 + 3 + 3 + 4) * 8
-    status_bytes = 128
+    status_bytes = 160
     barrier()
     torch.cuda.synchronize()
     t0 = time.perf_counter()

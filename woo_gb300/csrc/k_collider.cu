@@ -829,11 +829,15 @@ __device__ __forceinline__ long long csrFind(const Csr& csr, int a, int b) {
 // ------------------------------------------------------------------------------------ CSR rows
 // The CSR is built by counting: every entry takes a place in its row (one atomic per entry), a scan of the rows'
 // counts gives their starts, the entries go to their places, and each entry's rank among its row's partners is its
-// final position.  Rows hold ten or twenty entries, so the ranks are a few loads from L1; the order does not depend
-// on the atomics.  The radix sort of 2 C keys of up to 46 bits this replaces took 6 passes over 12 bytes an entry
+// final position.  Rows of bodies of like size hold ten or twenty entries, so the ranks are a few loads from L1; the
+// order does not depend on the atomics.  The radix sort of 2 C keys of up to 46 bits this replaces took 6 passes over 12 bytes an entry
 // (9 launches of 41 us a rebuild with 500k bodies and 2 M pairs; k_csr_fill and k_csr_rank now take 28 + 55 us).
 // A wall's or facet's row can hold every body: it is divided into V ranges of S partner ids, counted apart (so the
-// atomics spread as well), and an entry is ranked within its range.
+// atomics spread as well), and an entry is ranked within its range.  A large sphere among small ones has a long row
+// too, ranked in the square of its length; but its box also widens the sweep's columns and its thread walks every
+// partner, which takes far longer: of the 67 ms of a rebuild with a sphere that 38,000 others meet, k_sweep's two
+// passes take 33 and 40 at one launch each, k_csr_rank 0.97 (107 ms with the radix sorts; 3,500 partners among 1M
+// spheres 19.1 and 24.4 ms).
 struct RowCount {
   unsigned* cnt;        // rowptr as counts, then starts
   unsigned* sub;        // nLarge x V counts of the large bodies' ranges, then starts within their rows

@@ -478,8 +478,8 @@ __device__ __forceinline__ FastRec loadFast(const Particles& p, int i) {
   return r;
 }
 
-// Translation: force, damping, velocity, position, the FP32 shadow and the verlet trigger.  SPLIT: called by the
-// list pass, where another thread turns the particle.
+// Translation: force, damping, velocity, position, the FP32 shadow and the verlet trigger (spinFast turns the particle,
+// in another thread where the particle is touched).
 template <bool PERI>
 __device__ __forceinline__ void translateFast(const StepParams& P, const Particles& p, const int i, DeviceStatus* st,
                                               const bool touchedNow, const FastRec& rec, const d3& contactF) {
@@ -661,7 +661,9 @@ __device__ __forceinline__ bool spinFast(const StepParams& P, const Particles& p
 // A node without contact forces, in the first pass.  Spinning spheres of a warp that has ROTATE_HERE of them or more
 // are turned here, while the pass waits for memory; fewer go to the rotation list of the second pass (scattered over
 // most warps they would each cost their warp the FP64 time of 32).  1M falling, spinning spheres: first and second
-// pass 47 + 141 us a step with all of them listed (one atomic a warp on one counter), 80 + 82 us so.
+// pass 47 + 141 us a step with all of them listed (one atomic a warp on one counter), 80 + 82 us so.  Whole steps of
+// 500k falling, of which 10, 50, 75 and 100 % spin, turned here from 4 a warp on: 215.4, 219.9, 219.4 and 218.8 us;
+// from 16: 206.7, 217.8, 220.0, 219.3; from 24: 206.1, 216.7, 221.2, 219.4; never: 205.8, 215.6, 221.0, 225.2.
 static const int ROTATE_HERE = 16;
 template <bool PERI>
 __device__ __forceinline__ void integrateFast(const StepParams& P, const Particles& p, const int i, const int n,
@@ -831,9 +833,11 @@ __global__ void __launch_bounds__(LIST_T) k_leapfrog_lists(StepParams P, Particl
 // The whole integration in one launch, two threads a particle as in the list pass, for all particles in id order:
 // no lists, no second launch, and the records are read where the flags are.  Warps mix touched and untouched
 // particles, which costs FP64 issue where few are touched and many warps compete for it: taken up to ALL_PER_SM
-// particles an SM (4 warps per scheduler).  Whole steps with it and with the two passes: 10k spheres 62.2 and 66.7
-// us; 36k in a bed 109.1 and 110.4, falling 48.8 and 52.2, sheared 123.9 and 128.0; 50k 129.4 and 125.5, 57.7 and
-// 55.4, 112.1 and 107.8; 1M falling 555 and 410.
+// particles an SM (4 warps per scheduler).  Whole steps in us, with it and with the two passes, of a Frict bed (exact),
+// a Hertz bed (contracted), a falling cloud and a sheared packing: 10k 49.0 and 53.1, 32.4 and 37.8, 49.9 and 55.9, 117
+// and 127; 38k 94.1 and 96.9, 54.9 and 58.8, 56.8 and 58.5, 129 and 132; 45k 99.7 and 93.4, 61.9 and 63.0, 61.3 and
+// 61.7, 142 and 144; 60k 120 and 113, 78.2 and 72.0, 66.0 and 62.5, 145 and 145; 100k 169 and 154, 108 and 102, 80.4
+// and 72.2, 195 and 186.
 static const int ALL_PER_SM = 256;
 template <bool PERI>
 __global__ void __launch_bounds__(LIST_T) k_leapfrog_all(StepParams P, Particles p, int n, Contacts c, Csr csr,
